@@ -175,7 +175,8 @@ static __global__ void __launch_bounds__(256) boundary_force_kernel(
 
 // Pressure (spiky gradient), viscosity (Laplacian), tension (Poly6), boundary
 // force and gravity; MODE 0 integrates (symplectic Euler) into pos_out/vel_out,
-// MODE 1 writes the acceleration and the boundary neighbour count instead.
+// MODE 1 writes the acceleration and the boundary neighbour count instead,
+// MODE 2 the velocity after dt of it, with 1/rho, into vel_out (for XSPH).
 // Particle i of the sorted array; cells/bcells/bnear are the particle's own
 // grid tables (the batched solver passes per-scene tables and P).  BSEP: the
 // boundary sums were computed by boundary_force_kernel into bacc.  nflag: the
@@ -258,6 +259,8 @@ __device__ __forceinline__ void force_one(
         pos_out[i] = make_float4(fmaf(dt, nvx, xi.x), fmaf(dt, nvy, xi.y), fmaf(dt, nvz, xi.z),
                                  pos[i].w);
         vel_out[i] = make_float4(nvx, nvy, nvz, 0.0f);
+    } else if (MODE == 2) {
+        vel_out[i] = make_float4(fmaf(dt, axx, vi.x), fmaf(dt, ayy, vi.y), fmaf(dt, azz, vi.z), vi.w);
     } else {
         acc_out[3 * i + 0] = axx;
         acc_out[3 * i + 1] = ayy;

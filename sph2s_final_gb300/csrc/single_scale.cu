@@ -28,7 +28,7 @@ int free_solver(sph_solver* s) {
     void* ptrs[] = {s->pos,     s->vel,     s->spos,    s->svel,  s->rho,   s->aux,
                     s->keys[0], s->keys[1], s->vals[0], s->vals[1], s->cells, s->bcells,
                     s->bpos,    s->sort_mem, s->co_mem,  s->err,   s->stage, s->nbr, s->nbr_count,
-                    s->bnear,   s->pos0, s->xacc, s->xall, s->xnb, s->xa, s->bacc, s->blist, s->bflag, s->bcount, s->bstart, s->bcand};
+                    s->bnear,   s->pos0, s->xvel, s->xall, s->xa, s->bacc, s->blist, s->bflag, s->bcount, s->bstart, s->bcand};
     for (void* p : ptrs)
         if (p) cudaFree(p);
     if (s->side) cudaStreamSynchronize(s->side);
@@ -97,7 +97,8 @@ int enqueue_neighborhood(sph_solver* s) {
 // The density pass, and beside it on the second branch (fork/join events,
 // captured into the step graph as a parallel branch) the boundary force sums
 // of the near-boundary particles, which need only the sorted positions.
-void enqueue_density(sph_solver* s) {
+// With xall, also counts every particle's neighbours at any distance (XSPH).
+void enqueue_density(sph_solver* s, uint32_t* xall) {
     cudaEventRecord(s->fork, s->stream);
     cudaStreamWaitEvent(s->side, s->fork, 0);
     const uint32_t bgrid = std::min(blocks_for(s->n), (uint32_t)(2 * (s->sms > 0 ? s->sms : 1)));
@@ -105,9 +106,9 @@ void enqueue_density(sph_solver* s) {
                                                       s->bcand, s->blist, s->bcount, s->n, s->nb,
                                                       s->P, s->bacc);
     cudaEventRecord(s->join, s->side);
-    density_kernel<false><<<blocks_for(s->n, kDensityThreads), kDensityThreads, 0, s->stream>>>(
-        s->spos, s->cells, s->n, s->P, s->rho, s->aux, s->nbr, s->nbr_count, nullptr, s->xa,
-        s->svel);
+    const auto kernel = xall ? density_kernel<true> : density_kernel<false>;
+    kernel<<<blocks_for(s->n, kDensityThreads), kDensityThreads, 0, s->stream>>>(
+        s->spos, s->cells, s->n, s->P, s->rho, s->aux, s->nbr, s->nbr_count, xall, s->xa, s->svel);
 }
 
 void enqueue_force(sph_solver* s, float dt) {
@@ -123,16 +124,16 @@ void enqueue_step(sph_solver* s, float dt) {
     if (s->n == 0) return;
     enqueue_neighborhood(s);
     if (s->integrator == SPH_INTEGRATOR_XSPH) {
-        // density (+ full neighbour counts), accelerations, XSPH integrate
-        density_kernel<true><<<blocks_for(s->n, kDensityThreads), kDensityThreads, 0, s->stream>>>(
-            s->spos, s->cells, s->n, s->P, s->rho, s->aux, s->nbr, s->nbr_count, s->xall, s->xa,
-            s->svel);
-        force_kernel<1><<<blocks_for(s->n), 256, 0, s->stream>>>(
+        // density (+ full neighbour counts) beside the boundary force, velocities
+        // after the accelerations, XSPH integrate
+        enqueue_density(s, s->xall);
+        cudaStreamWaitEvent(s->stream, s->join, 0);
+        force_kernel<2, true><<<blocks_for(s->n), 256, 0, s->stream>>>(
             s->spos, s->xa, s->svel, s->cells, s->nbr, s->nbr_count, s->bpos, s->bcells, s->bnear,
-            s->n, s->nb, s->P, dt, nullptr, nullptr, s->xacc, s->xnb);
+            s->n, s->nb, s->P, dt, nullptr, s->xvel, nullptr, nullptr, s->bacc, s->bflag);
         xsph_integrate_kernel<<<blocks_for(s->n), 256, 0, s->stream>>>(
-            s->spos, s->svel, s->xacc, s->aux, s->cells, s->nbr, s->nbr_count, s->xall, s->n, s->P,
-            dt, s->cfg.xsph_coeff, s->pos, s->vel);
+            s->spos, s->xvel, s->cells, s->nbr, s->nbr_count, s->xall, s->n, s->P, dt,
+            s->cfg.xsph_coeff, s->pos, s->vel);
         return;
     }
     enqueue_density(s);
@@ -143,11 +144,10 @@ int set_integrator(sph_solver* s, int32_t integrator) {
     if (integrator != SPH_INTEGRATOR_SYMPLECTIC_EULER && integrator != SPH_INTEGRATOR_XSPH)
         return fail(SPH_E_INVALID, "sph_set_integrator: unknown integrator");
     SPH_CUDA(cudaStreamSynchronize(s->stream));
-    if (integrator == SPH_INTEGRATOR_XSPH && !s->xacc) {
+    if (integrator == SPH_INTEGRATOR_XSPH && !s->xvel) {
         const size_t n = s->n ? s->n : 1;
-        SPH_CUDA(cudaMalloc(&s->xacc, 12 * n));
+        SPH_CUDA(cudaMalloc(&s->xvel, 16 * n));
         SPH_CUDA(cudaMalloc(&s->xall, 4 * n));
-        SPH_CUDA(cudaMalloc(&s->xnb, 4 * n));
     }
     if (s->graph) {
         cudaGraphExecDestroy(s->graph);

@@ -55,9 +55,8 @@ struct sph_solver {
     float graph_dt = 0.0f;
     uint64_t step = 0;  // steps advanced since creation (carried by saved states)
     int32_t integrator = SPH_INTEGRATOR_SYMPLECTIC_EULER;
-    float* xacc = nullptr;     // XSPH integrator: accelerations of the step (3 per particle)
+    float4* xvel = nullptr;    // XSPH integrator: (v + dt a, 1/rho) of the step
     uint32_t* xall = nullptr;  // XSPH integrator: neighbours incl. distance 0, per particle
-    uint32_t* xnb = nullptr;   // XSPH integrator: boundary neighbour counts (unused output)
     // asynchronous position readback: two device staging buffers drained by a copy stream
     float* astage[2] = {nullptr, nullptr};
     cudaStream_t copy_stream = nullptr;
@@ -75,7 +74,7 @@ constexpr uint32_t kCoherentMinParticles = 131072;
 // returns the index of the key/value buffers that hold the sorted keys and
 // the permutation.
 int enqueue_neighborhood(sph_solver* s);
-void enqueue_density(sph_solver* s);
+void enqueue_density(sph_solver* s, uint32_t* xall = nullptr);
 void enqueue_force(sph_solver* s, float dt);
 int check_device_error(sph_solver* s);
 // Selects the integrator (allocating the XSPH buffers on first use) and drops

@@ -10,7 +10,12 @@
 //   x'_i  = x_i + dt v''_i
 // v'' is stored as the new velocity.  The self term vanishes (v'_i - v'_i is
 // exactly 0); neighbours come from the density pass's list (0 < r < h), the
-// force pass having written a_i; partners at distance 0 other than i itself
+// force pass having written (v'_i, 1/rho_i), so that a neighbour costs two
+// 16-byte gathers (what bounds the pass is their latency; with position, 1/rho,
+// velocity and three accelerations it was six, and the whole step of 65,536
+// particles took 78 us with three solvers side by side against 54 now, of which
+// the boundary scan inside the force pass was most: it now has its own pass
+// beside density, as in the Euler step); partners at distance 0 other than i itself
 // (flagged by the density pass's full count) are picked up from the home
 // cell, and particles whose list overflowed rescan the stencil.
 #pragma once
@@ -22,28 +27,25 @@ struct XsphAcc {
     float x = 0.f, y = 0.f, z = 0.f;
 };
 
-__device__ __forceinline__ void xsph_pair(XsphAcc& S, const SimParams& P, float r2, float inv_rho_j,
-                                          float vix, float viy, float viz, const float4& vj,
-                                          const float* __restrict__ acc, uint32_t j, float dt) {
+// vj: (v'_j, 1 / rho_j)
+__device__ __forceinline__ void xsph_pair(XsphAcc& S, const SimParams& P, float r2,
+                                          const float4& vi, const float4& vj) {
     const float a = P.h2 - r2;
-    const float w = a * a * a * inv_rho_j;
-    S.x = fmaf(fmaf(dt, acc[3 * j + 0], vj.x) - vix, w, S.x);
-    S.y = fmaf(fmaf(dt, acc[3 * j + 1], vj.y) - viy, w, S.y);
-    S.z = fmaf(fmaf(dt, acc[3 * j + 2], vj.z) - viz, w, S.z);
+    const float w = a * a * a * vj.w;
+    S.x = fmaf(vj.x - vi.x, w, S.x);
+    S.y = fmaf(vj.y - vi.y, w, S.y);
+    S.z = fmaf(vj.z - vi.z, w, S.z);
 }
 
 static __global__ void __launch_bounds__(256) xsph_integrate_kernel(
-    const float4* __restrict__ pos, const float4* __restrict__ vel, const float* __restrict__ acc,
-    const float2* __restrict__ aux, const uint2* __restrict__ cells, const uint4* __restrict__ nbr4,
+    const float4* __restrict__ pos, const float4* __restrict__ vel1,
+    const uint2* __restrict__ cells, const uint4* __restrict__ nbr4,
     const uint32_t* __restrict__ nbr_count, const uint32_t* __restrict__ nbr_all, uint32_t n,
     SimParams P, float dt, float eps, float4* __restrict__ pos_out, float4* __restrict__ vel_out) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const float4 xi = pos[i];
-    const float4 vi = vel[i];
-    const float vix = fmaf(dt, acc[3 * i + 0], vi.x);
-    const float viy = fmaf(dt, acc[3 * i + 1], vi.y);
-    const float viz = fmaf(dt, acc[3 * i + 2], vi.z);
+    const float4 vi = vel1[i];  // (v', 1 / rho)
     XsphAcc S;
     const uint32_t kc = nbr_count[i];
     if (kc <= (uint32_t)kMaxNbr) {
@@ -57,7 +59,7 @@ static __global__ void __launch_bounds__(256) xsph_integrate_kernel(
                     const float4 xj = __ldg(&pos[j]);
                     float dx, dy, dz;
                     const float r2 = dist2(xi.x, xi.y, xi.z, xj.x, xj.y, xj.z, dx, dy, dz);
-                    xsph_pair(S, P, r2, __ldg(&aux[j]).y, vix, viy, viz, __ldg(&vel[j]), acc, j, dt);
+                    xsph_pair(S, P, r2, vi, __ldg(&vel1[j]));
                 }
             }
         }
@@ -72,7 +74,7 @@ static __global__ void __launch_bounds__(256) xsph_integrate_kernel(
                 float dx, dy, dz;
                 const float r2 = dist2(xi.x, xi.y, xi.z, xj.x, xj.y, xj.z, dx, dy, dz);
                 if (j != i && r2 == 0.0f)
-                    xsph_pair(S, P, r2, __ldg(&aux[j]).y, vix, viy, viz, __ldg(&vel[j]), acc, j, dt);
+                    xsph_pair(S, P, r2, vi, __ldg(&vel1[j]));
             }
         }
     } else {
@@ -88,14 +90,13 @@ static __global__ void __launch_bounds__(256) xsph_integrate_kernel(
                         float dx, dy, dz;
                         const float r2 = dist2(xi.x, xi.y, xi.z, xj.x, xj.y, xj.z, dx, dy, dz);
                         if (r2 < P.T && j != i)
-                            xsph_pair(S, P, r2, __ldg(&aux[j]).y, vix, viy, viz, __ldg(&vel[j]),
-                                      acc, j, dt);
+                            xsph_pair(S, P, r2, vi, __ldg(&vel1[j]));
                     }
                 }
             }
     }
     const float c = eps * P.dens_coef;  // dens_coef = m * 315 / (64 pi h^9)
-    const float nvx = fmaf(c, S.x, vix), nvy = fmaf(c, S.y, viy), nvz = fmaf(c, S.z, viz);
+    const float nvx = fmaf(c, S.x, vi.x), nvy = fmaf(c, S.y, vi.y), nvz = fmaf(c, S.z, vi.z);
     pos_out[i] = make_float4(fmaf(dt, nvx, xi.x), fmaf(dt, nvy, xi.y), fmaf(dt, nvz, xi.z), xi.w);
     vel_out[i] = make_float4(nvx, nvy, nvz, 0.0f);
 }
