@@ -58,6 +58,17 @@ inline uint32_t blocks_for(uint32_t n, uint32_t t = 256) { return (n + t - 1) / 
 
 }  // namespace
 
+// What a captured step depends on besides the handle's buffers.
+struct TSGraphKey {
+    uint32_t n_low = 0, n_high = 0, groups = 0;
+    float dt = 0.0f;
+    bool colour = false;
+    bool operator==(const TSGraphKey& o) const {
+        return n_low == o.n_low && n_high == o.n_high && groups == o.groups && dt == o.dt &&
+               colour == o.colour;
+    }
+};
+
 struct sph_solver2 {
     sph_config2 cfg;
     TSParams P;
@@ -74,6 +85,16 @@ struct sph_solver2 {
     cudaEvent_t fork = nullptr, join = nullptr;
     cudaStream_t lowst = nullptr;  // the LOW density and force passes, beside the HIGH ones
     cudaEvent_t pfork = nullptr, pjoin = nullptr;
+    cudaStream_t nearst = nullptr;  // those of the LOW particles beside HIGH ones
+    cudaEvent_t njoin = nullptr;
+    uint8_t* occ = nullptr;         // per LOW cell: holds HIGH particles (this step) ...
+    uint32_t occ_low = 0;           // ... and from here on, per block of LOW cells: LOW particles
+    size_t occ_bytes = 0;
+    uint8_t* near_flag = nullptr;   // per LOW particle: HIGH particles in its stencil's cells
+    uint32_t *near_list = nullptr, *near_count = nullptr;
+    cudaGraphExec_t graph = nullptr;  // one step (ts_launch)
+    TSGraphKey graph_key;
+    int graph_seen = 0;               // steps launched before there was one
     uint32_t* keys[2] = {nullptr, nullptr};
     uint32_t* vals[2] = {nullptr, nullptr};
     void* sort_mem = nullptr;
@@ -106,6 +127,10 @@ int free_solver2(sph_solver2* s) {
     if (s->stream) cudaStreamSynchronize(s->stream);
     if (s->side) cudaStreamSynchronize(s->side);
     if (s->lowst) cudaStreamSynchronize(s->lowst);
+    if (s->nearst) cudaStreamSynchronize(s->nearst);
+    if (s->graph) cudaGraphExecDestroy(s->graph);
+    if (s->njoin) cudaEventDestroy(s->njoin);
+    if (s->nearst) cudaStreamDestroy(s->nearst);
     if (s->pfork) cudaEventDestroy(s->pfork);
     if (s->pjoin) cudaEventDestroy(s->pjoin);
     if (s->lowst) cudaStreamDestroy(s->lowst);
@@ -208,17 +233,15 @@ TSOut outputs(Pop& p, float* acc, uint32_t* nbr_bnd, float* colour = nullptr) {
 
 // hash -> sort -> reorder + cell ranges of both populations (Solver.cu:1616-1680):
 // one stable sort of (population bit, cell key) pairs gives each population the
-// order of its own sort with half the sort launches.
+// order of its own sort with half the sort launches.  ts_front has cleared the
+// sort scratch, the cell tables and the occupancy marks.
 void ts_neighborhoods(sph_solver2* s) {
     Pop &L = s->pop[0], &H = s->pop[1];
     cudaStream_t st = s->stream;
-    cudaMemsetAsync(H.cells, 0xFF, sizeof(uint2) * H.ncells, st);
-    cudaMemsetAsync(L.cells, 0xFF, sizeof(uint2) * L.ncells, st);
     const uint32_t n = L.n + H.n;
     if (n == 0) return;
     const int pop_bit = std::max(L.key_bits, H.key_bits);
     const int passes = sort_passes(pop_bit + 1);
-    sort_reset(s->sort, st);
     uint32_t hb = blocks_for(n);
     if (hb > 1216) hb = 1216;
     ts_hash_hist_kernel<<<hb, 256, 0, st>>>(L.pos, L.n, s->P.g[0], H.pos, H.n, s->P.g[1], pop_bit,
@@ -230,11 +253,12 @@ void ts_neighborhoods(sph_solver2* s) {
         ts_gather_kernel<true><<<blocks_for(H.n), 256, 0, st>>>(
             s->keys[o] + L.n, s->vals[o] + L.n, H.n, mask, L.n, s->P.g[1], H.pos, H.vel, H.stt,
             H.grp, H.spos, H.svel, H.sstt, H.sgrp, H.cells, s->err, s->P.axis, s->P.surface,
-            s->group_base, s->gsum, s->gready);
+            s->group_base, s->gsum, s->gready, s->P.g[0], s->occ);
     if (L.n)
         ts_gather_kernel<false><<<blocks_for(L.n), 256, 0, st>>>(
             s->keys[o], s->vals[o], L.n, mask, 0u, s->P.g[0], L.pos, L.vel, L.stt, L.grp, L.spos,
-            L.svel, L.sstt, L.sgrp, L.cells, s->err, -1, 0, 0, nullptr, nullptr);
+            L.svel, L.sstt, L.sgrp, L.cells, s->err, -1, 0, 0, nullptr, nullptr, s->P.g[0],
+            s->occ + s->occ_low);
 }
 
 // Everything up to and including the force/integrate pass; DEBUG variants
@@ -243,12 +267,21 @@ void ts_front(sph_solver2* s, float dt, bool debug, int dbg_pop, uint32_t* dnb_s
               uint32_t* dnb_compl, float* dacc, uint32_t* dnb_bnd) {
     cudaStream_t st = s->stream;
     const uint32_t gb = s->group_base;
-    if (gb) {
-        cudaMemsetAsync(s->gsum, 0, 8 * (size_t)gb, st);
-        cudaMemsetAsync(s->gready, 0, 4 * (size_t)gb, st);
-        cudaMemsetAsync(s->gacc, 0, 48 * (size_t)gb, st);
+    {
+        ClearBatch c;
+        c.add(s->pop[1].cells, sizeof(uint2) * s->pop[1].ncells, 0xFFFFFFFFu);
+        c.add(s->pop[0].cells, sizeof(uint2) * s->pop[0].ncells, 0xFFFFFFFFu);
+        c.add(s->sort.hist, s->sort.zero_bytes, 0u);
+        c.add(s->occ, s->occ_bytes, 0u);
+        c.add(s->near_count, 4, 0u);
+        c.add(s->ctl + kCtlFadedL, 8, 0u);
+        if (gb) {
+            c.add(s->gsum, 8 * (size_t)gb, 0u);
+            c.add(s->gready, 4 * (size_t)gb, 0u);
+            c.add(s->gacc, 48 * (size_t)gb, 0u);
+        }
+        clear_run(c, s->sms, st);
     }
-    cudaMemsetAsync(s->ctl + kCtlFadedL, 0, 8, st);
     ts_neighborhoods(s);
     Pop &L = s->pop[0], &H = s->pop[1];
     // the boundary force sums of both populations on the second branch, beside
@@ -257,11 +290,10 @@ void ts_front(sph_solver2* s, float dt, bool debug, int dbg_pop, uint32_t* dnb_s
     if (bsep) {
         cudaEventRecord(s->fork, st);
         cudaStreamWaitEvent(s->side, s->fork, 0);
-        for (Pop* p : {&H, &L})
-            if (p->n)
-                boundary_force_kernel<<<blocks_for(p->n), 256, 0, s->side>>>(
-                    p->spos, s->bpos, s->bcells, s->btab.start, s->btab.cand, nullptr, nullptr,
-                    p->n, s->nb, s->BP, p->bacc, s->bnear);
+        if (L.n + H.n)
+            ts_boundary_force_kernel<<<blocks_for(L.n + H.n), 256, 0, s->side>>>(
+                H.spos, H.n, H.bacc, L.spos, L.n, L.bacc, s->bpos, s->bcells, s->btab.start,
+                s->btab.cand, s->bnear, s->nb, s->BP);
         cudaEventRecord(s->join, s->side);
     }
     // The HIGH and LOW passes read only the step's sorted copies of both
@@ -271,8 +303,25 @@ void ts_front(sph_solver2* s, float dt, bool debug, int dbg_pop, uint32_t* dnb_s
     // ones and fill the SMs the smaller population's waves leave idle;
     // results are those of running them one after the other.
     cudaStream_t lo = s->lowst;
+    // LOW particles beside HIGH ones have passes of their own, several lanes
+    // each, on a third stream (not in the debug passes)
+    const bool lanes = !debug && L.n && H.n;
+    const uint8_t* skip = lanes ? s->near_flag : nullptr;
+    if (lanes) {
+        ts_near_kernel<<<blocks_for(L.n), 256, 0, st>>>(L.spos, L.n, s->P.g[0], s->P.h[0], s->occ,
+                                                        s->near_flag, s->near_list, s->near_count);
+    }
     cudaEventRecord(s->pfork, st);
     cudaStreamWaitEvent(lo, s->pfork, 0);
+    if (lanes) {
+        cudaStreamWaitEvent(s->nearst, s->pfork, 0);
+        const uint32_t blocks = std::min(blocks_for(L.n, 32 * kTsWarps / kTsLanes),
+                                         (uint32_t)(4 * s->sms));
+        ts_density_lanes_kernel<<<blocks, 32 * kTsWarps, 0, s->nearst>>>(
+            s->near_list, s->near_count, L.spos, L.cells, L.n, H.spos, H.cells, H.n, s->P, L.rho,
+            L.aux, L.list, L.list_count, L.clist, L.clist_count);
+        cudaEventRecord(s->njoin, s->nearst);
+    }
     if (H.n) {
         if (debug && dbg_pop == 1)
             ts_density_kernel<1, true><<<blocks_for(H.n), 256, 0, st>>>(
@@ -281,7 +330,8 @@ void ts_front(sph_solver2* s, float dt, bool debug, int dbg_pop, uint32_t* dnb_s
         else
             ts_density_kernel<1, false><<<blocks_for(H.n), 256, 0, st>>>(
                 H.spos, H.cells, H.n, L.spos, L.cells, L.n, s->P, H.rho, H.aux, nullptr, nullptr,
-                H.sgrp, gb, s->gsum, H.list, H.list_count, H.clist, H.clist_count);
+                H.sgrp, gb, s->gsum, H.list, H.list_count, H.clist, H.clist_count, nullptr,
+                lanes ? s->occ + s->occ_low : nullptr);
     }
     if (L.n) {
         if (debug && dbg_pop == 0)
@@ -291,10 +341,11 @@ void ts_front(sph_solver2* s, float dt, bool debug, int dbg_pop, uint32_t* dnb_s
         else
             ts_density_kernel<0, false><<<blocks_for(L.n), 256, 0, lo>>>(
                 L.spos, L.cells, L.n, H.spos, H.cells, H.n, s->P, L.rho, L.aux, nullptr, nullptr,
-                L.sgrp, gb, s->gsum, L.list, L.list_count, L.clist, L.clist_count);
+                L.sgrp, gb, s->gsum, L.list, L.list_count, L.clist, L.clist_count, skip);
     }
     cudaEventRecord(s->pjoin, lo);
     cudaStreamWaitEvent(st, s->pjoin, 0);
+    if (lanes) cudaStreamWaitEvent(st, s->njoin, 0);
     // merge decisions (slab: start-of-step centroids; surface: this step's densities)
     if (gb && (s->P.axis >= 0 || s->P.surface))
         ts_group_decide_kernel<<<blocks_for(gb), 256, 0, st>>>(s->gsum, s->gready, gb, s->P.lo43,
@@ -305,6 +356,16 @@ void ts_front(sph_solver2* s, float dt, bool debug, int dbg_pop, uint32_t* dnb_s
     if (bsep) cudaStreamWaitEvent(st, s->join, 0);
     cudaEventRecord(s->pfork, st);
     cudaStreamWaitEvent(lo, s->pfork, 0);
+    if (lanes) {
+        cudaStreamWaitEvent(s->nearst, s->pfork, 0);
+        ts_force_kernel<0, false, kTsLanes><<<blocks_for(L.n, 256 / kTsLanes), 256, 0, s->nearst>>>(
+            L.spos, L.svel, L.sstt, L.sgrp, L.aux, L.cells, L.n, H.spos, H.svel, H.aux, H.cells,
+            H.n, s->bpos, s->bcells, s->bnear, s->nb, s->P, dt, gm, gb, s->gacc, s->ctl, L.rho,
+            L.list, L.list_count, L.clist, L.clist_count,
+            outputs(L, nullptr, nullptr, s->colour_on ? s->colour[0] : nullptr), L.bacc, nullptr,
+            s->near_list, s->near_count);
+        cudaEventRecord(s->njoin, s->nearst);
+    }
     if (H.n) {
         TSOut o = outputs(H, dacc, dnb_bnd, (s->colour_on && !debug) ? s->colour[1] : nullptr);
         if (debug && dbg_pop == 1)
@@ -325,10 +386,11 @@ void ts_front(sph_solver2* s, float dt, bool debug, int dbg_pop, uint32_t* dnb_s
         else
             ts_force_kernel<0, false><<<blocks_for(L.n), 256, 0, lo>>>(
                 L.spos, L.svel, L.sstt, L.sgrp, L.aux, L.cells, L.n, H.spos, H.svel, H.aux, H.cells,
-                H.n, s->bpos, s->bcells, s->bnear, s->nb, s->P, dt, gm, gb, s->gacc, s->ctl, L.rho, L.list, L.list_count, L.clist, L.clist_count, o, bsep ? L.bacc : nullptr);
+                H.n, s->bpos, s->bcells, s->bnear, s->nb, s->P, dt, gm, gb, s->gacc, s->ctl, L.rho, L.list, L.list_count, L.clist, L.clist_count, o, bsep ? L.bacc : nullptr, skip);
     }
     cudaEventRecord(s->pjoin, lo);
     cudaStreamWaitEvent(st, s->pjoin, 0);
+    if (lanes) cudaStreamWaitEvent(st, s->njoin, 0);
 }
 
 int check_err2(sph_solver2* s) {
@@ -347,7 +409,8 @@ int check_err2(sph_solver2* s) {
     return SPH_OK;
 }
 
-int ts_step(sph_solver2* s, float dt) {
+// One step on the handle's streams, up to the copy of its control words.
+void ts_enqueue(sph_solver2* s, float dt) {
     cudaStream_t st = s->stream;
     Pop &L = s->pop[0], &H = s->pop[1];
     const uint32_t gb = s->group_base;
@@ -369,9 +432,60 @@ int ts_step(sph_solver2* s, float dt) {
                 L.soff, L.rho, L.n, s->P.mass[0], s->gmerge, s->moff, s->gacc, gb, s->ctl, hs, ls);
     }
     ts_advance_counters_kernel<<<1, 1, 0, st>>>(s->ctl, s->cap_groups, s->err);
-    SPH_CUDA(cudaGetLastError());
-    SPH_CUDA(cudaMemcpyAsync(s->ctl_host, s->ctl, 4 * kCtlWords, cudaMemcpyDeviceToHost, st));
-    SPH_CUDA(cudaStreamSynchronize(st));
+    cudaMemcpyAsync(s->ctl_host, s->ctl, 4 * kCtlWords, cudaMemcpyDeviceToHost, st);
+}
+
+// Steps launched kernel by kernel before the first graph is made.
+constexpr int kGraphAfter = 3;
+
+// Launches one step.  Its ~45 launches, memsets and event calls are host work
+// that the GPU waits for, since each step's counts are read back before the
+// next is launched; so a step whose sizes stay is launched as a graph.  Every
+// size in a launch comes from the populations, dt and the colour output; when
+// they change, the step is captured anew and the instantiated graph updated with
+// it, which costs about as much as launching the step twice but pays when the
+// next step is of the same sizes (while particles split, merge and fade they
+// change every two or three steps).  38,000 particles: 287 -> 163 us per step
+// (of which the launches were about 110), 314-376 -> 206-288 us while sizes
+// change; waiting for two steps of the same sizes before an update was slower.
+int ts_launch(sph_solver2* s, float dt) {
+    const TSGraphKey key = {s->pop[0].n, s->pop[1].n, s->group_base, dt, s->colour_on};
+    if (!s->graph && s->graph_seen < kGraphAfter) {
+        ++s->graph_seen;
+        ts_enqueue(s, dt);
+        SPH_CUDA(cudaGetLastError());
+        return SPH_OK;
+    }
+    if (!s->graph || !(key == s->graph_key)) {
+        cudaGraph_t g = nullptr;
+        SPH_CUDA(cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal));
+        ts_enqueue(s, dt);
+        const cudaError_t le = cudaGetLastError();
+        const cudaError_t ce = cudaStreamEndCapture(s->stream, &g);
+        SPH_CUDA(le);
+        SPH_CUDA(ce);
+        if (s->graph) {
+            cudaGraphExecUpdateResultInfo info;
+            if (cudaGraphExecUpdate(s->graph, g, &info) != cudaSuccess) {
+                cudaGetLastError();  // other nodes (a population or the groups came or went)
+                cudaGraphExecDestroy(s->graph);
+                s->graph = nullptr;
+            }
+        }
+        const cudaError_t ie = s->graph ? cudaSuccess : cudaGraphInstantiate(&s->graph, g, 0);
+        cudaGraphDestroy(g);
+        SPH_CUDA(ie);
+        s->graph_key = key;
+    }
+    SPH_CUDA(cudaGraphLaunch(s->graph, s->stream));
+    return SPH_OK;
+}
+
+int ts_step(sph_solver2* s, float dt) {
+    Pop &L = s->pop[0], &H = s->pop[1];
+    const int rc = ts_launch(s, dt);
+    if (rc != SPH_OK) return rc;
+    SPH_CUDA(cudaStreamSynchronize(s->stream));
     const uint32_t* c = s->ctl_host;
     s->stats[0] = c[kCtlSplits];
     s->stats[1] = c[kCtlMerges];
@@ -461,6 +575,8 @@ int create_solver2(const sph_config2* config, const TSParams& P, uint64_t capL, 
     TRY(check_cuda(cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking), "stream", __FILE__, __LINE__));
     TRY(check_cuda(cudaStreamCreateWithFlags(&s->side, cudaStreamNonBlocking), "stream", __FILE__, __LINE__));
     TRY(check_cuda(cudaStreamCreateWithFlags(&s->lowst, cudaStreamNonBlocking), "stream", __FILE__, __LINE__));
+    TRY(check_cuda(cudaStreamCreateWithFlags(&s->nearst, cudaStreamNonBlocking), "stream", __FILE__, __LINE__));
+    TRY(check_cuda(cudaEventCreateWithFlags(&s->njoin, cudaEventDisableTiming), "event", __FILE__, __LINE__));
     TRY(check_cuda(cudaEventCreateWithFlags(&s->pfork, cudaEventDisableTiming), "event", __FILE__, __LINE__));
     TRY(check_cuda(cudaEventCreateWithFlags(&s->pjoin, cudaEventDisableTiming), "event", __FILE__, __LINE__));
     TRY(check_cuda(cudaEventCreateWithFlags(&s->fork, cudaEventDisableTiming), "event", __FILE__, __LINE__));
@@ -505,6 +621,15 @@ int create_solver2(const sph_config2* config, const TSParams& P, uint64_t capL, 
     TRY(dalloc(&s->bpos, n_boundary, s->owned));
     TRY(dalloc(&s->bcells, s->pop[0].ncells, s->owned));
     TRY(dalloc(&s->bnear, s->pop[0].ncells, s->owned));
+    // one byte per LOW cell (holds HIGH particles), then one per 4 x 4 x 4 of them
+    // (hold LOW particles); both to whole words, which are cleared together
+    const GridParams& lg = P.g[0];
+    s->occ_low = (s->pop[0].ncells + 15u) & ~15u;
+    s->occ_bytes = (s->occ_low + ts_blocks(lg.dx) * ts_blocks(lg.dy) * ts_blocks(lg.dz) + 15u) & ~15u;
+    TRY(dalloc(&s->occ, s->occ_bytes, s->owned));
+    TRY(dalloc(&s->near_flag, capL, s->owned));
+    TRY(dalloc(&s->near_list, capL, s->owned));
+    TRY(dalloc(&s->near_count, 1, s->owned));
     TRY(check_cuda(cudaMallocHost((void**)&s->ctl_host, 4 * kCtlWords), "pinned", __FILE__, __LINE__));
     TRY(check_cuda(cudaMemset(s->err, 0, 4), "memset", __FILE__, __LINE__));
     {

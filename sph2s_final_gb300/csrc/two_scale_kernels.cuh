@@ -12,6 +12,7 @@
 // State arrays between steps: pos (x, y, z, id bits), vel (v, lambda), stt, grp.
 #pragma once
 #include "common.cuh"
+#include "force_kernel.cuh"
 
 namespace sph {
 
@@ -102,10 +103,17 @@ static __global__ void __launch_bounds__(256) ts_hash_hist_kernel(
     }
 }
 
+// Blocks of 4 x 4 x 4 LOW cells.
+__host__ __device__ __forceinline__ uint32_t ts_blocks(int cells) { return (uint32_t)(cells + 3) >> 2; }
+__device__ __forceinline__ uint32_t ts_block(const GridParams& g, int bx, int by, int bz) {
+    return (uint32_t)bx + ts_blocks(g.dx) * ((uint32_t)by + ts_blocks(g.dy) * (uint32_t)bz);
+}
+
 // Reorder + cell ranges for one population's part of the sorted array (keys
 // masked by key_mask, sorted values minus val_base are its indices); for HIGH
 // also accumulates the group centroid (slab axis, fixed point) and the number
-// of members in state 4.
+// of members in state 4.  With occ, also marks the LOW cells that hold HIGH
+// particles (HIGH) or the 4 x 4 x 4 blocks of them that hold LOW ones (LOW).
 template <bool HIGH_POP>
 __global__ void __launch_bounds__(256) ts_gather_kernel(
     const uint32_t* __restrict__ keys_sorted, const uint32_t* __restrict__ perm, uint32_t n,
@@ -114,7 +122,8 @@ __global__ void __launch_bounds__(256) ts_gather_kernel(
     const int32_t* __restrict__ stt, const uint32_t* __restrict__ grp, float4* __restrict__ spos,
     float4* __restrict__ svel, int32_t* __restrict__ sstt, uint32_t* __restrict__ sgrp,
     uint2* __restrict__ cells, uint32_t* __restrict__ err, int axis, int surface,
-    uint32_t group_base, unsigned long long* __restrict__ gsum, uint32_t* __restrict__ gready) {
+    uint32_t group_base, unsigned long long* __restrict__ gsum, uint32_t* __restrict__ gready,
+    GridParams g_low = GridParams{}, uint8_t* __restrict__ occ = nullptr) {
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     uint32_t q = perm[i] - val_base;
@@ -129,6 +138,12 @@ __global__ void __launch_bounds__(256) ts_gather_kernel(
     const uint32_t gid = grp[q];
     sstt[i] = s;
     sgrp[i] = gid;
+    if (occ) {
+        const int cx = cell_coord(p.x, g_low.ox, g_low.spacing, g_low.dx);
+        const int cy = cell_coord(p.y, g_low.oy, g_low.spacing, g_low.dy);
+        const int cz = cell_coord(p.z, g_low.oz, g_low.spacing, g_low.dz);
+        occ[HIGH_POP ? linear_cell(g_low, cx, cy, cz) : ts_block(g_low, cx >> 2, cy >> 2, cz >> 2)] = 1;
+    }
     if (HIGH_POP && (axis >= 0 || surface) && gid != kNoGroup && gid < group_base) {
         if (axis >= 0) {
             const float xa = axis == 0 ? p.x : (axis == 1 ? p.y : p.z);
@@ -168,9 +183,52 @@ static __global__ void __launch_bounds__(256) ts_group_decide_kernel(
     gmerge[gi] = (gready[gi] == 8u && away) ? 1u : 0u;
 }
 
+// rho and (p / rho^2, 1 / rho) from the sums over both populations.
+template <int R>
+__device__ __forceinline__ float ts_density_out(uint32_t i, float s, float sc, const TSParams& P,
+                                                float* __restrict__ rho,
+                                                float2* __restrict__ aux) {
+    const float rh = P.mass[R] * P.poly6[R] * s + P.mass[1 - R] * sc;
+    const float p = P.bulk * (rh - P.rho0);
+    const float inv = 1.0f / rh;
+    rho[i] = rh;
+    aux[i] = make_float2(p * inv * inv, inv);
+    return rh;
+}
+
+// LOW particles with HIGH particles in the cells of their stencil on the LOW
+// grid (occ, marked by ts_gather_kernel): every HIGH particle within h_LOW lies
+// in one of them.  flag[i], and their sorted indices in no particular order.
+static __global__ void __launch_bounds__(256) ts_near_kernel(
+    const float4* __restrict__ spos, uint32_t n, GridParams g, float h,
+    const uint8_t* __restrict__ occ, uint8_t* __restrict__ flag, uint32_t* __restrict__ list,
+    uint32_t* __restrict__ count) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31u;
+    bool near = false;
+    if (i < n) {
+        const float4 x = spos[i];
+        const Stencil s = stencil(g, x.x, x.y, x.z, h);
+        for (int cz = s.z0; cz <= s.z1; ++cz)
+            for (int cy = s.y0; cy <= s.y1; ++cy)
+                for (int cx = s.x0; cx <= s.x1; ++cx)
+                    near |= __ldg(&occ[linear_cell(g, cx, cy, cz)]) != 0;
+        flag[i] = near ? 1 : 0;
+    }
+    const uint32_t m = __ballot_sync(0xFFFFFFFFu, near);
+    if (!m) return;
+    uint32_t base = 0;
+    if (lane == 0) base = atomicAdd(count, (uint32_t)__popc(m));
+    base = __shfl_sync(0xFFFFFFFFu, base, 0);
+    if (near) list[base + (uint32_t)__popc(m & ((1u << lane) - 1u))] = i;
+}
+
 // Density of population r: same population weighted by lambda_j, plus the
 // complementary population on its own grid with the LOW radius and the
 // averaged kernel 0.5 (W_h0 + W_h1) (SPH2S_FINAL_TWO_SCALE/Solver.cu:732-845).
+// skip: particles that ts_density_lanes_kernel takes.  low_blocks (HIGH): the
+// blocks of LOW cells that hold LOW particles (ts_gather_kernel); looking at up
+// to eight of them instead of 27 LOW cells leaves the pass where it was
+// (622,592 HIGH particles: 204 -> 199 us).
 template <int R, bool DEBUG>
 __global__ void __launch_bounds__(256) ts_density_kernel(
     const float4* __restrict__ spos_r, const uint2* __restrict__ cells_r, uint32_t n_r,
@@ -179,10 +237,11 @@ __global__ void __launch_bounds__(256) ts_density_kernel(
     uint32_t* __restrict__ nbr_compl, const uint32_t* __restrict__ sgrp_r, uint32_t group_base,
     unsigned long long* __restrict__ gsurf, uint4* __restrict__ list4,
     uint32_t* __restrict__ list_count, uint4* __restrict__ clist4,
-    uint32_t* __restrict__ clist_count) {
+    uint32_t* __restrict__ clist_count, const uint8_t* __restrict__ skip = nullptr,
+    const uint8_t* __restrict__ low_blocks = nullptr) {
     constexpr int C = 1 - R;
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n_r) return;
+    if (i >= n_r || (skip && skip[i])) return;
     const float4 xi = spos_r[i];
     float s = 0.0f, sc = 0.0f;
     uint32_t ns = 0, nc = 0;
@@ -220,8 +279,17 @@ __global__ void __launch_bounds__(256) ts_density_kernel(
     // complementary force neighbours (0 < r2 < T_0) in stencil order, same layout
     uint32_t kcl = 0;
     uint32_t* cout = reinterpret_cast<uint32_t*>(clist4) + 4 * (size_t)i;
-    if (n_c > 0) {
-        const Stencil st = stencil(P.g[C], xi.x, xi.y, xi.z, P.h[0]);
+    bool any = n_c > 0 && !skip;  // where skip tells who has any, none is left here
+    Stencil st = {0, -1, 0, -1, 0, -1};
+    if (any) st = stencil(P.g[C], xi.x, xi.y, xi.z, P.h[0]);
+    if (R == 1 && low_blocks) {  // most HIGH particles have no LOW ones near
+        any = false;
+        for (int bz = st.z0 >> 2; bz <= st.z1 >> 2; ++bz)
+            for (int by = st.y0 >> 2; by <= st.y1 >> 2; ++by)
+                for (int bx = st.x0 >> 2; bx <= st.x1 >> 2; ++bx)
+                    any |= __ldg(&low_blocks[ts_block(P.g[0], bx, by, bz)]) != 0;
+    }
+    if (any) {
         for (int cz = st.z0; cz <= st.z1; ++cz)
             for (int cy = st.y0; cy <= st.y1; ++cy) {
                 const uint32_t row = linear_cell(P.g[C], 0, cy, cz);
@@ -249,11 +317,7 @@ __global__ void __launch_bounds__(256) ts_density_kernel(
             }
     }
     clist_count[i] = kcl;
-    const float rh = P.mass[R] * P.poly6[R] * s + P.mass[C] * sc;
-    const float p = P.bulk * (rh - P.rho0);
-    const float inv = 1.0f / rh;
-    rho[i] = rh;
-    aux[i] = make_float2(p * inv * inv, inv);
+    const float rh = ts_density_out<R>(i, s, sc, P, rho, aux);
     list_count[i] = k;
     if (DEBUG) {
         nbr_same[i] = ns;
@@ -263,6 +327,147 @@ __global__ void __launch_bounds__(256) ts_density_kernel(
         const uint32_t gid = sgrp_r[i];
         if (gid != kNoGroup && gid < group_base) atomicAdd(&gsurf[gid], 1ull);
     }
+}
+
+// The same for the listed LOW particles (ts_near_kernel), kTsLanes lanes each:
+// a coarse particle beside the fine ones tests ~1,000 of them after its own
+// ~216, and one thread doing so set the pass's duration at every size (180 us
+// with 10,368 coarse particles, 179 with 184,000).  Now this pass takes 45 / 66
+// us beside 39 / 68 us for the other LOW particles.  Each lane scans a
+// contiguous share of the stencil's rows, its hits go through shared memory
+// into the lists in stencil order, and the lanes' sums are added in a fixed
+// order.  A lane that runs out of room leaves the particle's list to the force
+// pass's rescan.
+constexpr uint32_t kTsLanes = 8;
+constexpr uint32_t kTsSame = 32, kTsCompl = 56;  // hits per lane
+constexpr int kTsWarps = 4;
+
+// Appends the lanes' hits (hit[e * 32], e < k) in lane order to particle i's
+// list; returns the particle's count, beyond `cap` if some lane had no room.
+__device__ __forceinline__ uint32_t ts_lanes_list(const uint32_t* hit, uint32_t k, uint32_t room,
+                                                  uint32_t cap, uint32_t i, uint32_t n, bool on,
+                                                  uint4* __restrict__ list4) {
+    constexpr uint32_t kAll = 0xFFFFFFFFu;
+    const uint32_t sub = threadIdx.x & (kTsLanes - 1u), lane = threadIdx.x & 31u;
+    uint32_t at = k;
+#pragma unroll
+    for (uint32_t d = 1; d < kTsLanes; d <<= 1) {
+        const uint32_t y = __shfl_up_sync(kAll, at, d);
+        if (sub >= d) at += y;
+    }
+    const uint32_t total = __shfl_sync(kAll, at, (int)(lane | (kTsLanes - 1u)));
+    const uint32_t full = __ballot_sync(kAll, k > room) >> (lane & ~(kTsLanes - 1u));
+    at -= k;
+    if (on) {
+        uint32_t* out = reinterpret_cast<uint32_t*>(list4) + 4 * ((size_t)(at >> 2) * n + i) + (at & 3u);
+        const uint32_t next_group = 4u * n - 3u;
+        for (uint32_t e = 0; e < min(k, room) && at < cap; ++e, ++at) {
+            __stcs(out, hit[e * 32]);
+            out += (at & 3u) == 3u ? next_group : 1u;
+        }
+    }
+    return full & ((1u << kTsLanes) - 1u) ? max(total, cap + 1u) : total;
+}
+
+static __global__ void __launch_bounds__(32 * kTsWarps) ts_density_lanes_kernel(
+    const uint32_t* __restrict__ near, const uint32_t* __restrict__ near_count,
+    const float4* __restrict__ spos_l, const uint2* __restrict__ cells_l, uint32_t n_l,
+    const float4* __restrict__ spos_h, const uint2* __restrict__ cells_h, uint32_t n_h,
+    TSParams P, float* __restrict__ rho, float2* __restrict__ aux, uint4* __restrict__ list4,
+    uint32_t* __restrict__ list_count, uint4* __restrict__ clist4,
+    uint32_t* __restrict__ clist_count) {
+    __shared__ uint32_t s_hit[kTsWarps][(kTsSame + kTsCompl) * 32];
+    const uint32_t lane = threadIdx.x & 31u, sub = lane & (kTsLanes - 1u);
+    const uint32_t count = min(*near_count, n_l);
+    const uint32_t per = 32 / kTsLanes, warps = gridDim.x * kTsWarps;
+    uint32_t* hs = s_hit[threadIdx.x >> 5] + lane;
+    uint32_t* hc = hs + kTsSame * 32;
+    for (uint32_t t = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * per; t < count;
+         t += warps * per) {
+        const bool on = t + lane / kTsLanes < count;
+        const uint32_t i = on ? min(near[t + lane / kTsLanes], n_l - 1u) : 0u;
+        const float4 xi = spos_l[i];
+        float s = 0.0f, sc = 0.0f;
+        uint32_t k = 0, kc = 0;
+        // f(j, xj, r2) for this lane's share of the stencil's candidates with r2 < T
+        auto scan = [&](const GridParams& g, const uint2* cells, const float4* pos, uint32_t n,
+                        float h, float T, auto&& f) {
+            const Stencil st = stencil(g, xi.x, xi.y, xi.z, h);
+            const uint32_t ny = (uint32_t)(st.y1 - st.y0 + 1);
+            const uint32_t rows = ny * (uint32_t)(st.z1 - st.z0 + 1);
+            const uint32_t last = (sub + 1) * rows / kTsLanes;
+            for (uint32_t r = sub * rows / kTsLanes; r < last; ++r) {
+                const uint32_t row = linear_cell(g, 0, st.y0 + (int)(r % ny), st.z0 + (int)(r / ny));
+                for (int cx = st.x0; cx <= st.x1; ++cx) {
+                    const uint2 c = __ldg(&cells[row + cx]);
+                    const uint32_t e = min(c.y, n);
+                    for (uint32_t j = c.x; j < e; ++j) {
+                        const float4 xj = __ldg(&pos[j]);
+                        float dx, dy, dz;
+                        const float r2 = dist2(xi.x, xi.y, xi.z, xj.x, xj.y, xj.z, dx, dy, dz);
+                        if (r2 < T) f(j, xj, r2);
+                    }
+                }
+            }
+        };
+        if (on) {
+            scan(P.g[0], cells_l, spos_l, n_l, P.h[0], P.T[0], [&](uint32_t j, const float4& xj, float r2) {
+                const float a = P.h2[0] - r2;
+                s = fmaf(P.coupled ? 1.0f : xj.w, a * a * a, s);
+                if (r2 != 0.0f) {
+                    if (k < kTsSame) hs[k * 32] = j;
+                    ++k;
+                }
+            });
+            scan(P.g[1], cells_h, spos_h, n_h, P.h[0], P.T[0], [&](uint32_t j, const float4& xj, float r2) {
+                const float a0 = P.h2[0] - r2, a1 = P.h2[1] - r2;
+                float w = P.poly6[0] * a0 * a0 * a0;
+                if (r2 < P.T[1]) w += P.poly6[1] * a1 * a1 * a1;
+                sc = fmaf(P.coupled ? 1.0f : xj.w, 0.5f * w, sc);
+                if (r2 != 0.0f) {
+                    if (kc < kTsCompl) hc[kc * 32] = j;
+                    ++kc;
+                }
+            });
+        }
+        __syncwarp();
+        const uint32_t same = ts_lanes_list(hs, k, kTsSame, (uint32_t)kMaxNbr, i, n_l, on, list4);
+        const uint32_t compl_ = ts_lanes_list(hc, kc, kTsCompl, ComplCap<0>::value, i, n_l, on, clist4);
+#pragma unroll
+        for (uint32_t d = kTsLanes / 2; d; d >>= 1) {
+            s += __shfl_xor_sync(0xFFFFFFFFu, s, d);
+            sc += __shfl_xor_sync(0xFFFFFFFFu, sc, d);
+        }
+        if (on && sub == 0) {
+            ts_density_out<0>(i, s, sc, P, rho, aux);
+            list_count[i] = same;
+            clist_count[i] = compl_;
+        }
+        __syncwarp();
+    }
+}
+
+// Boundary force sums of both populations in one launch, HIGH first (LOW grid
+// and radius for both): each population's launch alone took as long as one
+// near-wall particle's chain of candidates.
+static __global__ void __launch_bounds__(256) ts_boundary_force_kernel(
+    const float4* __restrict__ pos_h, uint32_t n_h, float4* __restrict__ bacc_h,
+    const float4* __restrict__ pos_l, uint32_t n_l, float4* __restrict__ bacc_l,
+    const float4* __restrict__ bpos, const uint2* __restrict__ bcells,
+    const uint32_t* __restrict__ bstart, const uint32_t* __restrict__ bcand,
+    const uint8_t* __restrict__ near, uint32_t nb, SimParams P) {
+    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    const bool low = i >= n_h;
+    if (low) i -= n_h;
+    if (low && i >= n_l) return;
+    const float4 xi = low ? pos_l[i] : pos_h[i];
+    const int hx = cell_coord(xi.x, P.g.ox, P.g.spacing, P.g.dx);
+    const int hy = cell_coord(xi.y, P.g.oy, P.g.spacing, P.g.dy);
+    const int hz = cell_coord(xi.z, P.g.oz, P.g.spacing, P.g.dz);
+    const uint32_t home = linear_cell(P.g, hx, hy, hz);
+    if (!__ldg(&near[home])) return;
+    boundary_force_one(i, xi, hx, hy, hz, home, bpos, bcells, bstart, bcand, nb, P,
+                       low ? bacc_l : bacc_h);
 }
 
 struct TSOut {
@@ -279,7 +484,13 @@ struct TSOut {
 
 // Accelerations (SPH2S_FINAL_TWO_SCALE/Solver.cu:847-1048) and integration
 // with the blend/state machine (Solver.cu:1163-1289) of population r.
-template <int R, bool DEBUG>
+// LANES > 1: that many lanes to each listed particle (near, ts_near_kernel), each
+// taking every LANES-th group of its lists (a coarse one has ~270 fine
+// neighbours, whose gathers are a chain of latencies), their sums added in a
+// fixed order: the LOW pass 55 / 61 us (10,368 / 184,000 particles) before,
+// 15 / 14 us for the near ones beside 19 / 39 us for the others now;
+// LANES = 1: one thread per particle, those flagged in skip left out.
+template <int R, bool DEBUG, int LANES = 1>
 __global__ void __launch_bounds__(256) ts_force_kernel(
     const float4* __restrict__ spos_r, const float4* __restrict__ svel_r,
     const int32_t* __restrict__ sstt_r, const uint32_t* __restrict__ sgrp_r,
@@ -292,10 +503,21 @@ __global__ void __launch_bounds__(256) ts_force_kernel(
     unsigned long long* __restrict__ gacc, uint32_t* __restrict__ ctl,
     const float* __restrict__ rho_r, const uint4* __restrict__ list4,
     const uint32_t* __restrict__ list_count, const uint4* __restrict__ clist4,
-    const uint32_t* __restrict__ clist_count, TSOut out, const float4* __restrict__ bacc) {
+    const uint32_t* __restrict__ clist_count, TSOut out, const float4* __restrict__ bacc,
+    const uint8_t* __restrict__ skip = nullptr, const uint32_t* __restrict__ near = nullptr,
+    const uint32_t* __restrict__ near_count = nullptr) {
     constexpr int C = 1 - R;
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n_r) return;
+    const uint32_t sub = LANES > 1 ? threadIdx.x % LANES : 0u;
+    uint32_t i = blockIdx.x * (blockDim.x / LANES) + threadIdx.x / LANES;
+    bool on = true;
+    if (LANES > 1) {
+        const uint32_t count = min(*near_count, n_r);
+        if (i - (threadIdx.x & 31u) / LANES >= count) return;  // whole warps: sums are shuffled
+        on = i < count;
+        i = on ? min(near[i], n_r - 1u) : 0u;
+    } else if (i >= n_r || (skip && skip[i])) {
+        return;
+    }
     const float4 xi = spos_r[i];
     const float4 vi = svel_r[i];
     const float2 ai = aux_r[i];
@@ -304,8 +526,10 @@ __global__ void __launch_bounds__(256) ts_force_kernel(
     // wavelet and mass centre over the same population, self included
     const bool colour = out.colour != nullptr;
     const float psi0 = -3.0f * kMexicanHatC;
-    float psum = psi0, cwx = vi.x * psi0, cwy = vi.y * psi0, cwz = vi.z * psi0;
-    float csx = xi.x, csy = xi.y, csz = xi.z, ccnt = 1.0f;
+    const float first = sub == 0 ? 1.0f : 0.0f;
+    float psum = first * psi0, cwx = first * (vi.x * psi0), cwy = first * (vi.y * psi0),
+          cwz = first * (vi.z * psi0);
+    float csx = first * xi.x, csy = first * xi.y, csz = first * xi.z, ccnt = first;
     const float inv_h2 = 1.0f / P.h2[R];
     {
         const float tco = P.sigma * P.mass[R] * P.poly6[R] * ai.y;
@@ -339,11 +563,13 @@ __global__ void __launch_bounds__(256) ts_force_kernel(
                 ccnt += 1.0f;
             }
         };
-        const uint32_t kc = list_count[i];
+        const uint32_t kc = on ? list_count[i] : 0u;
         if (kc <= (uint32_t)kMaxNbr) {  // the density pass's list, in stencil order
-            uint4 g = kc ? __ldcs(&list4[i]) : make_uint4(0u, 0u, 0u, 0u);
-            for (uint32_t t = 0; t < kc; t += 4) {
-                const uint4 gn = (t + 4 < kc) ? __ldcs(&list4[(size_t)((t >> 2) + 1) * n_r + i]) : g;
+            const uint32_t t0 = 4 * sub;
+            uint4 g = t0 < kc ? __ldcs(&list4[(size_t)sub * n_r + i]) : make_uint4(0u, 0u, 0u, 0u);
+            for (uint32_t t = t0; t < kc; t += 4 * LANES) {
+                const uint4 gn = (t + 4 * LANES < kc)
+                                     ? __ldcs(&list4[(size_t)((t >> 2) + LANES) * n_r + i]) : g;
                 const uint32_t js[4] = {g.x, g.y, g.z, g.w};
 #pragma unroll
                 for (int u = 0; u < 4; ++u) {
@@ -357,7 +583,7 @@ __global__ void __launch_bounds__(256) ts_force_kernel(
                 }
                 g = gn;
             }
-        } else {
+        } else if (sub == 0) {
             const Stencil st = stencil(P.g[R], xi.x, xi.y, xi.z, P.h[R]);
             for (int cz = st.z0; cz <= st.z1; ++cz)
                 for (int cy = st.y0; cy <= st.y1; ++cy) {
@@ -409,12 +635,13 @@ __global__ void __launch_bounds__(256) ts_force_kernel(
             wy = fmaf(vc, vj.y - vi.y, wy);
             wz = fmaf(vc, vj.z - vi.z, wz);
         };
-        const uint32_t kc = clist_count[i];
+        const uint32_t kc = on ? clist_count[i] : 0u;
         if (kc <= ComplCap<R>::value) {  // the density pass's list, in stencil order
-            uint4 gc = kc ? __ldcs(&clist4[i]) : make_uint4(0u, 0u, 0u, 0u);
-            for (uint32_t t = 0; t < kc; t += 4) {
+            const uint32_t t0 = 4 * sub;
+            uint4 gc = t0 < kc ? __ldcs(&clist4[(size_t)sub * n_r + i]) : make_uint4(0u, 0u, 0u, 0u);
+            for (uint32_t t = t0; t < kc; t += 4 * LANES) {
                 const uint4 g = gc;  // this group; the next one is fetched meanwhile
-                gc = (t + 4 < kc) ? __ldcs(&clist4[(size_t)((t >> 2) + 1) * n_r + i]) : g;
+                gc = (t + 4 * LANES < kc) ? __ldcs(&clist4[(size_t)((t >> 2) + LANES) * n_r + i]) : g;
                 const uint32_t js[4] = {g.x, g.y, g.z, g.w};
 #pragma unroll
                 for (int u = 0; u < 4; ++u) {
@@ -427,7 +654,7 @@ __global__ void __launch_bounds__(256) ts_force_kernel(
                     }
                 }
             }
-        } else {
+        } else if (sub == 0) {
             const Stencil st = stencil(P.g[C], xi.x, xi.y, xi.z, P.h[0]);
             for (int cz = st.z0; cz <= st.z1; ++cz)
                 for (int cy = st.y0; cy <= st.y1; ++cy) {
@@ -444,6 +671,29 @@ __global__ void __launch_bounds__(256) ts_force_kernel(
                     }
                 }
         }
+    }
+    if (LANES > 1) {
+        auto total = [](float& v) {
+#pragma unroll
+            for (int d = LANES / 2; d; d >>= 1) v += __shfl_xor_sync(0xFFFFFFFFu, v, d);
+        };
+        total(fx);
+        total(fy);
+        total(fz);
+        total(wx);
+        total(wy);
+        total(wz);
+        if (colour) {
+            total(psum);
+            total(cwx);
+            total(cwy);
+            total(cwz);
+            total(csx);
+            total(csy);
+            total(csz);
+            total(ccnt);
+        }
+        if (!on || sub != 0) return;
     }
     float bx = 0.f, by = 0.f, bz = 0.f;
     uint32_t bcnt = 0;
