@@ -10,7 +10,7 @@
 // (sort permutation, sorted positions and velocities, densities, neighbour
 // lists), then the hand-written adjoint kernels run backwards through it,
 // holding the neighbour structure of every step constant.  Memory is one
-// segment of tape (~310 bytes per particle per step) plus T/K checkpoints.
+// segment of tape (~440 bytes per particle per step) plus T/K checkpoints.
 #include <cmath>
 #include <cstring>
 #include <vector>

@@ -200,7 +200,7 @@ __global__ void __launch_bounds__(BS) b_force_kernel(
         if (i >= R.p_off + R.p_n) continue;
         const SimParams P = R.P;
         force_one<0, true>(i, pos, xa, va, cells + R.c_off, nbr4, nbr_count, bpos,
-                           bcells + R.c_off, bnear + R.c_off, n, nb, P, dt, pos_out, vel_out,
+                           bcells + R.c_off, bnear + R.c_off, n, nb, P, &R.P, dt, pos_out, vel_out,
                            nullptr, nullptr, bacc, bflag);
     }
 }

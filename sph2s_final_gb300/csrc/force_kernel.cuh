@@ -173,6 +173,39 @@ static __global__ void __launch_bounds__(256) boundary_force_kernel(
     }
 }
 
+constexpr uint32_t kForceManyParticles = 1u << 17;
+
+// The pair sums of a particle whose list overflowed: from the stencil, in the
+// same order.  Out of line, so that its registers are not the pass's.
+static __device__ __noinline__ ForceAcc force_rescan(float4 xi, float4 vi, float tcoef,
+                                                     const float4* __restrict__ xa,
+                                                     const float4* __restrict__ va,
+                                                     const uint2* __restrict__ cells, uint32_t n,
+                                                     const SimParams* params) {
+    const SimParams& P = *params;
+    ForceAcc A = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    const Stencil s = stencil(P.g, xi.x, xi.y, xi.z, P.h);
+    for (int cz = s.z0; cz <= s.z1; ++cz)
+        for (int cy = s.y0; cy <= s.y1; ++cy) {
+            const uint32_t row = linear_cell(P.g, 0, cy, cz);
+            for (int cx = s.x0; cx <= s.x1; ++cx) {
+                const uint2 r = __ldg(&cells[row + cx]);
+                const uint32_t e = min(r.y, n);
+                for (uint32_t j = r.x; j < e; ++j) {
+                    const float4 xj = __ldg(&xa[j]);
+                    float dx, dy, dz;
+                    const float r2 = dist2(xi.x, xi.y, xi.z, xj.x, xj.y, xj.z, dx, dy, dz);
+                    if (r2 < P.T && r2 != 0.0f) {
+                        const float4 vj = __ldg(&va[j]);
+                        force_pair(A, P, xi.w, tcoef, vi, dx, dy, dz, r2,
+                                   make_float2(xj.w, vj.w), vj);
+                    }
+                }
+            }
+        }
+    return A;
+}
+
 // Pressure (spiky gradient), viscosity (Laplacian), tension (Poly6), boundary
 // force and gravity; MODE 0 integrates (symplectic Euler) into pos_out/vel_out,
 // MODE 1 writes the acceleration and the boundary neighbour count instead,
@@ -183,14 +216,23 @@ static __global__ void __launch_bounds__(256) boundary_force_kernel(
 // per-particle near-boundary flags written with the boundary pass's list
 // (NearList::flag); without it the particle's cell is recomputed and looked
 // up in bnear (the same answer: both test bnear of the particle's cell).
-template <int MODE, bool BSEP = false>
+// params: P where it can be addressed (kernel parameters or a scene's record).
+// AHEAD: neighbours whose gathers are issued together, before their terms.  The
+// pass is bound by the latency of those gathers: four together, at 64 registers
+// and 4 blocks per SM, against one after another at 40 registers and 6 blocks
+// took a step of 32,768 particles from 75.8 to 72.2 us, 32 batched scenes from
+// 705 to 674 us.  From kForceManyParticles on, one at a time at 48 registers and
+// 5 blocks: three solvers of 155,184 side by side 298 us for four steps (four
+// together: 307), a step of 2,097,152 773 us (four together 796, 40 registers
+// 783).  All the same bits.
+template <int MODE, bool BSEP = false, int AHEAD = 4>
 __device__ __forceinline__ void force_one(
     uint32_t i, const float4* __restrict__ pos, const float4* __restrict__ xa,
     const float4* __restrict__ va, const uint2* __restrict__ cells, const uint4* __restrict__ nbr4,
     const uint32_t* __restrict__ nbr_count, const float4* __restrict__ bpos,
     const uint2* __restrict__ bcells, const uint8_t* __restrict__ bnear, uint32_t n, uint32_t nb,
-    const SimParams& P, float dt, float4* __restrict__ pos_out, float4* __restrict__ vel_out,
-    float* __restrict__ acc_out, uint32_t* __restrict__ nbr_b,
+    const SimParams& P, const SimParams* params, float dt, float4* __restrict__ pos_out,
+    float4* __restrict__ vel_out, float* __restrict__ acc_out, uint32_t* __restrict__ nbr_b,
     const float4* __restrict__ bacc = nullptr, const uint8_t* __restrict__ nflag = nullptr) {
     const float4 xi = xa[i];  // (x, y, z, p/rho^2)
     const float4 vi = va[i];  // (v, 1/rho)
@@ -205,38 +247,29 @@ __device__ __forceinline__ void force_one(
             const uint4 gn = (t + 4 < kc) ? __ldcs(&nbr4[(size_t)((t >> 2) + 1) * n + i]) : g;
             const uint32_t js[4] = {g.x, g.y, g.z, g.w};
 #pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                if (t + u < kc) {
-                    const uint32_t j = min(js[u], n - 1);
-                    const float4 xj = __ldg(&xa[j]);
-                    const float4 vj = __ldg(&va[j]);
-                    float dx, dy, dz;
-                    float r2 = dist2(xi.x, xi.y, xi.z, xj.x, xj.y, xj.z, dx, dy, dz);
-                    force_pair(A, P, xi.w, tcoef, vi, dx, dy, dz, r2, make_float2(xj.w, vj.w), vj);
+            for (int v = 0; v < 4; v += AHEAD) {
+                float4 xj[AHEAD], vj[AHEAD];
+#pragma unroll
+                for (int u = 0; u < AHEAD; ++u) {
+                    if (AHEAD == 1 && t + v >= kc) continue;
+                    const uint32_t j = t + v + u < kc ? min(js[v + u], n - 1) : i;
+                    xj[u] = __ldg(&xa[j]);
+                    vj[u] = __ldg(&va[j]);
                 }
+#pragma unroll
+                for (int u = 0; u < AHEAD; ++u)
+                    if (t + v + u < kc) {
+                        float dx, dy, dz;
+                        const float r2 =
+                            dist2(xi.x, xi.y, xi.z, xj[u].x, xj[u].y, xj[u].z, dx, dy, dz);
+                        force_pair(A, P, xi.w, tcoef, vi, dx, dy, dz, r2,
+                                   make_float2(xj[u].w, vj[u].w), vj[u]);
+                    }
             }
             g = gn;
         }
     } else {
-        const Stencil s = stencil(P.g, xi.x, xi.y, xi.z, P.h);
-        for (int cz = s.z0; cz <= s.z1; ++cz)
-            for (int cy = s.y0; cy <= s.y1; ++cy) {
-                const uint32_t row = linear_cell(P.g, 0, cy, cz);
-                for (int cx = s.x0; cx <= s.x1; ++cx) {
-                    const uint2 r = __ldg(&cells[row + cx]);
-                    const uint32_t e = min(r.y, n);
-                    for (uint32_t j = r.x; j < e; ++j) {
-                        const float4 xj = __ldg(&xa[j]);
-                        float dx, dy, dz;
-                        float r2 = dist2(xi.x, xi.y, xi.z, xj.x, xj.y, xj.z, dx, dy, dz);
-                        if (r2 < P.T && r2 != 0.0f) {
-                            const float4 vj = __ldg(&va[j]);
-                            force_pair(A, P, xi.w, tcoef, vi, dx, dy, dz, r2,
-                                       make_float2(xj.w, vj.w), vj);
-                        }
-                    }
-                }
-            }
+        A = force_rescan(xi, vi, tcoef, xa, va, cells, n, params);
     }
     float bx = 0.f, by = 0.f, bz = 0.f;
     uint32_t bcnt = 0;
@@ -269,19 +302,19 @@ __device__ __forceinline__ void force_one(
     }
 }
 
-template <int MODE, bool BSEP = false>
-__global__ void __launch_bounds__(256, 6) force_kernel(
+template <int MODE, bool BSEP = false, int AHEAD = 4>
+__global__ void __launch_bounds__(256, AHEAD > 1 ? 4 : 5) force_kernel(
     const float4* __restrict__ pos, const float4* __restrict__ xa, const float4* __restrict__ va,
     const uint2* __restrict__ cells, const uint4* __restrict__ nbr4,
     const uint32_t* __restrict__ nbr_count, const float4* __restrict__ bpos,
     const uint2* __restrict__ bcells, const uint8_t* __restrict__ bnear, uint32_t n, uint32_t nb,
-    SimParams P, float dt, float4* __restrict__ pos_out, float4* __restrict__ vel_out,
-    float* __restrict__ acc_out, uint32_t* __restrict__ nbr_b,
+    const __grid_constant__ SimParams P, float dt, float4* __restrict__ pos_out,
+    float4* __restrict__ vel_out, float* __restrict__ acc_out, uint32_t* __restrict__ nbr_b,
     const float4* __restrict__ bacc = nullptr, const uint8_t* __restrict__ nflag = nullptr) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    force_one<MODE, BSEP>(i, pos, xa, va, cells, nbr4, nbr_count, bpos, bcells, bnear, n, nb, P,
-                          dt, pos_out, vel_out, acc_out, nbr_b, bacc, nflag);
+    force_one<MODE, BSEP, AHEAD>(i, pos, xa, va, cells, nbr4, nbr_count, bpos, bcells, bnear, n, nb,
+                                 P, &P, dt, pos_out, vel_out, acc_out, nbr_b, bacc, nflag);
 }
 
 }  // namespace sph

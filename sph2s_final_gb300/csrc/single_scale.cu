@@ -113,7 +113,8 @@ void enqueue_density(sph_solver* s, uint32_t* xall) {
 
 void enqueue_force(sph_solver* s, float dt) {
     cudaStreamWaitEvent(s->stream, s->join, 0);
-    force_kernel<0, true><<<blocks_for(s->n), 256, 0, s->stream>>>(
+    const auto kernel = s->n < kForceManyParticles ? force_kernel<0, true, 4> : force_kernel<0, true, 1>;
+    kernel<<<blocks_for(s->n), 256, 0, s->stream>>>(
         s->spos, s->xa, s->svel, s->cells, s->nbr, s->nbr_count, s->bpos, s->bcells, s->bnear,
         s->n, s->nb, s->P, dt, s->pos, s->vel, nullptr, nullptr, s->bacc, s->bflag);
 }
