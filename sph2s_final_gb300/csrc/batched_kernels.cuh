@@ -205,4 +205,34 @@ __global__ void __launch_bounds__(BS) b_force_kernel(
     }
 }
 
+// One scene's positions, velocities and densities (those that are wanted) for
+// the host, 7 floats per particle at most, in sorted order or by the
+// scene-local ids in pos.w; an id beyond the scene sets kErrSceneId.
+constexpr uint32_t kErrSceneId = 16u;
+static __global__ void __launch_bounds__(256) b_pack_scene_kernel(
+    const float4* __restrict__ pos, const float4* __restrict__ vel, const float* __restrict__ rho,
+    uint32_t off, uint32_t n, int by_id, float* __restrict__ xyz, float* __restrict__ v3,
+    float* __restrict__ r1, uint32_t* __restrict__ err) {
+    const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= n) return;
+    const float4 x = pos[off + k];
+    const uint32_t d = by_id ? __float_as_uint(x.w) : k;
+    if (d >= n) {
+        atomicOr(err, kErrSceneId);
+        return;
+    }
+    if (xyz) {
+        xyz[3 * (size_t)d + 0] = x.x;
+        xyz[3 * (size_t)d + 1] = x.y;
+        xyz[3 * (size_t)d + 2] = x.z;
+    }
+    if (v3) {
+        const float4 v = vel[off + k];
+        v3[3 * (size_t)d + 0] = v.x;
+        v3[3 * (size_t)d + 1] = v.y;
+        v3[3 * (size_t)d + 2] = v.z;
+    }
+    if (r1) r1[d] = rho[off + k];
+}
+
 }  // namespace sph

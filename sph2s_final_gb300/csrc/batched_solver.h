@@ -60,6 +60,12 @@ struct sph_batch {
     std::vector<sph_config> cfgs;     // per-scene configuration (viscosity changes in rollouts)
     float4* pos0 = nullptr;           // creation positions, packed by scene (rollout restarts)
     std::vector<uint32_t> tile_first; // first 256-particle tile of each scene in tiles[1]
+    // readback of a scene: packed on the device, copied out through two pinned
+    // buffers (allocated on first use)
+    float* pack = nullptr;
+    size_t pack_floats = 0;
+    char* pinned[2] = {nullptr, nullptr};
+    cudaEvent_t copied[2] = {nullptr, nullptr};
     sph::BRollout* rollout = nullptr; // tape of a batched differentiable rollout
 };
 
