@@ -39,6 +39,7 @@ struct Rollout {
     std::vector<uint32_t*> cnt;
     std::vector<uint2*> cells;
     float4 *gx = nullptr, *gv = nullptr, *gx2 = nullptr, *gv2 = nullptr, *lam = nullptr;
+    float4* gb = nullptr;  // the boundary force's part of gx2
     float4* gxT = nullptr;
     float* grho = nullptr;
     float* gmu_part = nullptr;
@@ -97,6 +98,7 @@ int alloc_rollout(sph_solver* s, int T, int K, Rollout** out) {
     if (rc == SPH_OK &&
         ((rc = ralloc(r, &r->gx, n)) || (rc = ralloc(r, &r->gv, n)) || (rc = ralloc(r, &r->gx2, n)) ||
          (rc = ralloc(r, &r->gv2, n)) || (rc = ralloc(r, &r->lam, n)) || (rc = ralloc(r, &r->gxT, n)) ||
+         (rc = ralloc(r, &r->gb, n)) ||
          (rc = ralloc(r, &r->grho, n)) || (rc = ralloc(r, &r->gmu_part, blocks)) ||
          (rc = ralloc(r, &r->gmu_acc, 1)))) {
     }
@@ -277,15 +279,21 @@ int sph_rollout_backward(sph_solver* s, float* grad_v0, float* grad_x0, double* 
         s->nbr = nbr0;
         s->nbr_count = cnt0;
         for (int k = len - 1; k >= 0; --k) {  // reverse through the segment
-            adj_lambda_kernel<<<blocks, 256, 0, st>>>(r->gx, r->gv, n, r->dt, r->lam);
+            adj_lambda_kernel<<<blocks, 256, 0, st>>>(r->gx, r->gv, r->aux[k], n, r->dt, r->lam);
+            // the boundary force's adjoint beside that of the pair forces
+            SPH_CUDA(cudaEventRecord(s->fork, st));
+            SPH_CUDA(cudaStreamWaitEvent(s->side, s->fork, 0));
+            adj_boundary_kernel<<<blocks_for(n, 256 / 32 * kBndLanes), 256, 0, s->side>>>(
+                r->xh[k], r->lam, s->bpos, s->bcells, s->bnear, s->bstart, s->bcand, n, s->nb, s->P,
+                r->gb);
+            SPH_CUDA(cudaEventRecord(s->join, s->side));
             adj_force_kernel<<<blocks, 256, 0, st>>>(
-                r->xh[k], r->vh[k], r->rho[k], r->aux[k], r->nbr[k], r->cnt[k], r->cells[k], s->bpos,
-                s->bcells, s->bnear, s->bstart, s->bcand, n, s->nb, s->P, r->mu, r->dt, r->lam,
-                r->gx, r->gv, r->gx2,
-                r->gv2, r->grho, r->gmu_part);
+                r->xh[k], r->vh[k], r->rho[k], r->nbr[k], r->cnt[k], r->cells[k], n, s->P, r->mu,
+                r->dt, r->lam, r->gx, r->gv, r->gx2, r->gv2, r->grho, r->gmu_part);
             adj_sum_kernel<<<1, 32, 0, st>>>(r->gmu_part, blocks, r->gmu_acc);
+            SPH_CUDA(cudaStreamWaitEvent(st, s->join, 0));
             adj_density_kernel<<<blocks, 256, 0, st>>>(r->xh[k], r->nbr[k], r->cnt[k], r->cells[k],
-                                                       n, s->P, r->grho, r->gx2);
+                                                       n, s->P, r->grho, r->gb, r->gx2);
             adj_unpermute_kernel<<<blocks, 256, 0, st>>>(r->perm[k], n, r->gx2, r->gv2, r->gx, r->gv);
         }
         SPH_CUDA(cudaGetLastError());

@@ -32,29 +32,45 @@
 
 namespace sph {
 
-// Calls f(j, xj, dx, dy, dz, r2) for every fluid neighbour 0 < r2 < T of
-// particle i, from the list or, on overflow, by rescanning the stencil.
-template <class F>
+// Calls f(payload, dx, dy, dz, r2) for every fluid neighbour 0 < r2 < T of
+// particle i, payload = load(j), from the list or, on overflow, by rescanning the
+// stencil.  The gathers of AHEAD neighbours are issued together, before their
+// terms: their latency is what bounds these passes (65,536 particles: adj_density
+// 16.7 -> 11.5 us with four, adj_force 47.7 -> 19.5 with two, three gathers per
+// neighbour instead of four and the boundary part apart; four spilled there).
+template <int AHEAD, class L, class F>
 __device__ __forceinline__ void visit_force_neighbors(uint32_t i, const float4& xi,
                                                       const float4* __restrict__ pos,
                                                       const uint4* __restrict__ nbr4,
                                                       const uint32_t* __restrict__ nbr_count,
                                                       const uint2* __restrict__ cells, uint32_t n,
-                                                      const SimParams& P, F& f) {
+                                                      const SimParams& P, L&& load, F&& f) {
     const uint32_t kc = nbr_count[i];
     if (kc <= (uint32_t)kMaxNbr) {
+        uint4 g = kc ? __ldg(&nbr4[i]) : make_uint4(0u, 0u, 0u, 0u);
         for (uint32_t t = 0; t < kc; t += 4) {
-            const uint4 g = __ldg(&nbr4[(size_t)(t >> 2) * n + i]);
+            const uint4 gn = t + 4 < kc ? __ldg(&nbr4[(size_t)((t >> 2) + 1) * n + i]) : g;
             const uint32_t js[4] = {g.x, g.y, g.z, g.w};
 #pragma unroll
-            for (int u = 0; u < 4; ++u)
-                if (t + u < kc) {
-                    const uint32_t j = min(js[u], n - 1);
-                    const float4 xj = __ldg(&pos[j]);
-                    float dx, dy, dz;
-                    const float r2 = dist2(xi.x, xi.y, xi.z, xj.x, xj.y, xj.z, dx, dy, dz);
-                    f(j, dx, dy, dz, r2);
+            for (int v = 0; v < 4; v += AHEAD) {
+                float4 xj[AHEAD];
+                decltype(load(0u)) pay[AHEAD];
+#pragma unroll
+                for (int u = 0; u < AHEAD; ++u) {
+                    const uint32_t j = t + v + u < kc ? min(js[v + u], n - 1) : i;
+                    xj[u] = __ldg(&pos[j]);
+                    pay[u] = load(j);
                 }
+#pragma unroll
+                for (int u = 0; u < AHEAD; ++u)
+                    if (t + v + u < kc) {
+                        float dx, dy, dz;
+                        const float r2 =
+                            dist2(xi.x, xi.y, xi.z, xj[u].x, xj[u].y, xj[u].z, dx, dy, dz);
+                        f(pay[u], dx, dy, dz, r2);
+                    }
+            }
+            g = gn;
         }
         return;
     }
@@ -69,32 +85,37 @@ __device__ __forceinline__ void visit_force_neighbors(uint32_t i, const float4& 
                     const float4 xj = __ldg(&pos[j]);
                     float dx, dy, dz;
                     const float r2 = dist2(xi.x, xi.y, xi.z, xj.x, xj.y, xj.z, dx, dy, dz);
-                    if (r2 < P.T && r2 != 0.0f) f(j, dx, dy, dz, r2);
+                    if (r2 < P.T && r2 != 0.0f) f(load(j), dx, dy, dz, r2);
                 }
             }
         }
 }
 
-// lam = dt (gv' + dt gx')
+// lam = dt (gv' + dt gx'), with A = p / rho^2 in w: beside the position and the
+// step's velocity (1 / rho in w) a neighbour's third and last gather.
 static __global__ void __launch_bounds__(256) adj_lambda_kernel(const float4* __restrict__ gx,
                                                                 const float4* __restrict__ gv,
+                                                                const float2* __restrict__ aux,
                                                                 uint32_t n, float dt,
                                                                 float4* __restrict__ lam) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const float4 a = gx[i], b = gv[i];
-    lam[i] = make_float4(dt * fmaf(dt, a.x, b.x), dt * fmaf(dt, a.y, b.y), dt * fmaf(dt, a.z, b.z), 0.f);
+    lam[i] = make_float4(dt * fmaf(dt, a.x, b.x), dt * fmaf(dt, a.y, b.y), dt * fmaf(dt, a.z, b.z),
+                         aux[i].x);
 }
 
+struct AdjNeighbor {
+    float4 v, l;  // (v, 1 / rho), (lam, A)
+};
+
 struct AdjForcePair {
-    const float4* vel;
-    const float2* aux;
-    const float4* lam;
     float h, h2, mu, mCs, sC6;  // mCs = m * 45/(pi h^6) (spiky and viscosity), sC6 = sigma m C6
     float4 vi, li;
     float Ai, dAi, inv_i;
     float gx, gy, gz, gvx, gvy, gvz, grho, gmu;
-    __device__ __forceinline__ void operator()(uint32_t j, float dx, float dy, float dz, float r2) {
+    __device__ __forceinline__ void operator()(const AdjNeighbor& q, float dx, float dy, float dz,
+                                               float r2) {
         const float rs = rsqrtf(r2);
         const float r = r2 * rs;
         const float hr = h - r;
@@ -103,11 +124,9 @@ struct AdjForcePair {
         const float a2 = h2 - r2;
         const float w = a2 * a2 * a2;
         const float wp = -6.0f * r * a2 * a2;
-        const float2 aj = __ldg(&aux[j]);
-        const float inv_j = aj.y;
-        const float4 vj = __ldg(&vel[j]);
-        const float4 lj = __ldg(&lam[j]);
-        const float Asum = Ai + aj.x;
+        const float4 &vj = q.v, &lj = q.l;
+        const float inv_j = vj.w;
+        const float Asum = Ai + lj.w;
         const float phi_i = mCs * Asum * f - sC6 * w * inv_i;
         const float phi_j = mCs * Asum * f - sC6 * w * inv_j;
         const float php_i = mCs * Asum * fp - sC6 * wp * inv_i;
@@ -134,83 +153,130 @@ struct AdjForcePair {
     }
 };
 
-// Adjoint of force + integrate for particle i of the step's sorted order;
-// returns particle i's share of d L / d mu.  cells/bcells/bnear are the
-// particle's own grid tables (the batched rollout passes per-scene tables, P
-// and mu).
+// Adjoint of force + integrate for particle i of the step's sorted order,
+// without the boundary force (adj_boundary_warp); returns particle i's share of
+// d L / d mu.  cells are the particle's own grid's (the batched rollout passes
+// per-scene tables, P and mu).
 __device__ __forceinline__ float adj_force_one(
     uint32_t i, const float4* __restrict__ pos, const float4* __restrict__ vel,
-    const float* __restrict__ rho, const float2* __restrict__ aux, const uint4* __restrict__ nbr4,
-    const uint32_t* __restrict__ nbr_count, const uint2* __restrict__ cells,
+    const float* __restrict__ rho, const uint4* __restrict__ nbr4,
+    const uint32_t* __restrict__ nbr_count, const uint2* __restrict__ cells, uint32_t n,
+    const SimParams& P, float mu, float dt, const float4* __restrict__ lam,
+    const float4* __restrict__ gx_in, const float4* __restrict__ gv_in,
+    float4* __restrict__ gx_out, float4* __restrict__ gv_out, float* __restrict__ grho) {
+    const float4 xi = pos[i];
+    AdjForcePair A;
+    A.h = P.h;
+    A.h2 = P.h2;
+    A.mu = mu;
+    A.mCs = P.pres_coef;
+    A.sC6 = P.tens_coef;
+    A.vi = vel[i];
+    A.li = lam[i];
+    A.Ai = A.li.w;
+    A.inv_i = A.vi.w;
+    A.dAi = P.bulk * (2.0f * P.rho0 - rho[i]) * A.inv_i * A.inv_i * A.inv_i;  // dA/drho
+    A.gx = A.gy = A.gz = A.gvx = A.gvy = A.gvz = A.grho = A.gmu = 0.0f;
+    visit_force_neighbors<2>(
+        i, xi, pos, nbr4, nbr_count, cells, n, P,
+        [&](uint32_t j) { return AdjNeighbor{__ldg(&vel[j]), __ldg(&lam[j])}; }, A);
+    const float4 gxi = gx_in[i], gvi = gv_in[i];
+    gx_out[i] = make_float4(gxi.x + A.gx, gxi.y + A.gy, gxi.z + A.gz, 0.f);
+    gv_out[i] = make_float4(fmaf(dt, gxi.x, gvi.x) + A.gvx, fmaf(dt, gxi.y, gvi.y) + A.gvy,
+                            fmaf(dt, gxi.z, gvi.z) + A.gvz, 0.f);
+    grho[i] = A.grho;
+    return A.gmu;
+}
+
+// Adjoint of the boundary force b_i = sum_k beta(r) x_ik, beta = Bc shape(2r/h) /
+// r^2, of one warp's kBndLanes particles (lane l < kBndLanes holds the l-th's
+// index i, below `end`): gb[i] = its part of gx_i, 0 away from the boundary.
+// It needs the positions and lam alone and runs beside adj_force; inside it, one
+// lane's ~70 candidates in a row held the warp.  Eight lanes take a particle,
+// each every eighth candidate, their sums added in a fixed order: 16 us at 65,536
+// particles, most of it under adj_force's 20.
+constexpr uint32_t kBndLanes = 8;
+
+__device__ __forceinline__ void adj_boundary_warp(
+    uint32_t i, uint32_t end, const float4* __restrict__ pos, const float4* __restrict__ lam,
     const float4* __restrict__ bpos, const uint2* __restrict__ bcells,
     const uint8_t* __restrict__ bnear, const uint32_t* __restrict__ bstart,
-    const uint32_t* __restrict__ bcand, uint32_t n, uint32_t nb, const SimParams& P, float mu,
-    float dt, const float4* __restrict__ lam, const float4* __restrict__ gx_in,
-    const float4* __restrict__ gv_in, float4* __restrict__ gx_out, float4* __restrict__ gv_out,
-    float* __restrict__ grho) {
-    {
-        const float4 xi = pos[i];
-        AdjForcePair A;
-        A.vel = vel;
-        A.aux = aux;
-        A.lam = lam;
-        A.h = P.h;
-        A.h2 = P.h2;
-        A.mu = mu;
-        A.mCs = P.pres_coef;
-        A.sC6 = P.tens_coef;
-        A.vi = vel[i];
-        A.li = lam[i];
-        const float2 ai = aux[i];
-        A.Ai = ai.x;
-        A.inv_i = ai.y;
-        A.dAi = P.bulk * (2.0f * P.rho0 - rho[i]) * ai.y * ai.y * ai.y;  // dA/drho
-        A.gx = A.gy = A.gz = A.gvx = A.gvy = A.gvz = A.grho = A.gmu = 0.0f;
-        visit_force_neighbors(i, xi, pos, nbr4, nbr_count, cells, n, P, A);
-        // boundary: b_i = sum_k beta(r) x_ik, beta = Bc shape(2r/h) / r^2
+    const uint32_t* __restrict__ bcand, uint32_t nb, const SimParams& P,
+    float4* __restrict__ gb) {
+    constexpr uint32_t kAll = 0xFFFFFFFFu;
+    const uint32_t lane = threadIdx.x & 31u, sub = lane & (kBndLanes - 1u);
+    bool near = false;
+    if (lane < kBndLanes && i < end) {
+        near = __ldg(&bnear[home_cell(P.g, pos[i])]) != 0;
+        if (!near) gb[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    uint32_t m = __ballot_sync(kAll, near);
+    while (m) {
+        uint32_t mine = m;
+        for (uint32_t g = 0; g < lane / kBndLanes; ++g) mine &= mine - 1u;  // the earlier groups'
+        const bool work = mine != 0u;
+        const uint32_t p = __shfl_sync(kAll, i, work ? __ffs((int)mine) - 1 : 0);
         float bx = 0.f, by = 0.f, bz = 0.f;
-        const int hx = cell_coord(xi.x, P.g.ox, P.g.spacing, P.g.dx);
-        const int hy = cell_coord(xi.y, P.g.oy, P.g.spacing, P.g.dy);
-        const int hz = cell_coord(xi.z, P.g.oz, P.g.spacing, P.g.dz);
-        const uint32_t home = linear_cell(P.g, hx, hy, hz);
-        if (__ldg(&bnear[home])) {
-            visit_boundary(xi, hx, hy, hz, home, bpos, bcells, bstart, bcand, nb, P,
-                           [&](const float4& xk) {
+        if (work) {
+            const float4 xi = pos[p], li = lam[p];
+            auto pair = [&](const float4& xk) {
                 float dx, dy, dz;
                 const float r2 = dist2(xi.x, xi.y, xi.z, xk.x, xk.y, xk.z, dx, dy, dz);
-                if (r2 < P.T) {
-                    const float rs = rsqrtf(r2);
-                    const float rr = r2 * rs;
-                    const float q = rr * P.two_over_h;
-                    float sh, shp;
-                    if (q < 2.0f / 3.0f) {
-                        sh = 2.0f / 3.0f;
-                        shp = 0.0f;
-                    } else if (q < 1.0f) {
-                        sh = q * (2.0f - 1.5f * q);
-                        shp = 2.0f - 3.0f * q;
-                    } else {
-                        const float t2 = 2.0f - q;
-                        sh = 0.5f * t2 * t2;
-                        shp = -t2;
-                    }
-                    const float beta = P.bnd_coef * sh * rs * rs;
-                    const float betap = P.bnd_coef * (shp * P.two_over_h * rs * rs -
-                                                      2.0f * sh * rs * rs * rs);
-                    const float rad = betap * rs * (A.li.x * dx + A.li.y * dy + A.li.z * dz);
-                    bx += beta * A.li.x + rad * dx;
-                    by += beta * A.li.y + rad * dy;
-                    bz += beta * A.li.z + rad * dz;
+                if (!(r2 < P.T)) return;
+                const float rs = rsqrtf(r2);
+                const float q = r2 * rs * P.two_over_h;
+                float sh, shp;
+                if (q < 2.0f / 3.0f) {
+                    sh = 2.0f / 3.0f;
+                    shp = 0.0f;
+                } else if (q < 1.0f) {
+                    sh = q * (2.0f - 1.5f * q);
+                    shp = 2.0f - 3.0f * q;
+                } else {
+                    const float t2 = 2.0f - q;
+                    sh = 0.5f * t2 * t2;
+                    shp = -t2;
                 }
-            });
+                const float beta = P.bnd_coef * sh * rs * rs;
+                const float betap =
+                    P.bnd_coef * (shp * P.two_over_h * rs * rs - 2.0f * sh * rs * rs * rs);
+                const float rad = betap * rs * (li.x * dx + li.y * dy + li.z * dz);
+                bx += beta * li.x + rad * dx;
+                by += beta * li.y + rad * dy;
+                bz += beta * li.z + rad * dz;
+            };
+            const int hx = cell_coord(xi.x, P.g.ox, P.g.spacing, P.g.dx);
+            const int hy = cell_coord(xi.y, P.g.oy, P.g.spacing, P.g.dy);
+            const int hz = cell_coord(xi.z, P.g.oz, P.g.spacing, P.g.dz);
+            if (boundary_listed(xi, hx, hy, hz, P)) {
+                const uint32_t home = linear_cell(P.g, hx, hy, hz);
+                const uint32_t e = __ldg(&bstart[home + 1]);
+                for (uint32_t k = __ldg(&bstart[home]) + sub; k < e; k += kBndLanes)
+                    pair(__ldg(&bpos[min(__ldg(&bcand[k]), nb - 1)]));
+            } else if (sub == 0) {
+                scan_boundary(xi, bpos, bcells, nb, P, pair);
+            }
         }
-        const float4 gxi = gx_in[i], gvi = gv_in[i];
-        gx_out[i] = make_float4(gxi.x + A.gx + bx, gxi.y + A.gy + by, gxi.z + A.gz + bz, 0.f);
-        gv_out[i] = make_float4(fmaf(dt, gxi.x, gvi.x) + A.gvx, fmaf(dt, gxi.y, gvi.y) + A.gvy,
-                                fmaf(dt, gxi.z, gvi.z) + A.gvz, 0.f);
-        grho[i] = A.grho;
-        return A.gmu;
+#pragma unroll
+        for (uint32_t o = kBndLanes / 2; o; o >>= 1) {
+            bx += __shfl_xor_sync(kAll, bx, o);
+            by += __shfl_xor_sync(kAll, by, o);
+            bz += __shfl_xor_sync(kAll, bz, o);
+        }
+        if (work && sub == 0) gb[p] = make_float4(bx, by, bz, 0.f);
+        for (uint32_t g = 0; g < 32 / kBndLanes; ++g) m &= m - 1u;
     }
+}
+
+static __global__ void __launch_bounds__(256) adj_boundary_kernel(
+    const float4* __restrict__ pos, const float4* __restrict__ lam,
+    const float4* __restrict__ bpos, const uint2* __restrict__ bcells,
+    const uint8_t* __restrict__ bnear, const uint32_t* __restrict__ bstart,
+    const uint32_t* __restrict__ bcand, uint32_t n, uint32_t nb,
+    const __grid_constant__ SimParams P, float4* __restrict__ gb) {
+    const uint32_t w = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    adj_boundary_warp(w * kBndLanes + (threadIdx.x & 31u), n, pos, lam, bpos, bcells, bnear, bstart,
+                      bcand, nb, P, gb);
 }
 
 // Block sum of one value per thread in a fixed order (warp shuffles, then the
@@ -231,54 +297,55 @@ __device__ __forceinline__ float block_sum_fixed(float v) {
 
 static __global__ void __launch_bounds__(256) adj_force_kernel(
     const float4* __restrict__ pos, const float4* __restrict__ vel, const float* __restrict__ rho,
-    const float2* __restrict__ aux, const uint4* __restrict__ nbr4,
-    const uint32_t* __restrict__ nbr_count, const uint2* __restrict__ cells,
-    const float4* __restrict__ bpos, const uint2* __restrict__ bcells,
-    const uint8_t* __restrict__ bnear, const uint32_t* __restrict__ bstart,
-    const uint32_t* __restrict__ bcand, uint32_t n, uint32_t nb, SimParams P, float mu, float dt,
-    const float4* __restrict__ lam, const float4* __restrict__ gx_in,
+    const uint4* __restrict__ nbr4, const uint32_t* __restrict__ nbr_count,
+    const uint2* __restrict__ cells, uint32_t n, const __grid_constant__ SimParams P, float mu,
+    float dt, const float4* __restrict__ lam, const float4* __restrict__ gx_in,
     const float4* __restrict__ gv_in, float4* __restrict__ gx_out, float4* __restrict__ gv_out,
     float* __restrict__ grho, float* __restrict__ gmu_block) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     float gmu_i = 0.0f;
     if (i < n)
-        gmu_i = adj_force_one(i, pos, vel, rho, aux, nbr4, nbr_count, cells, bpos, bcells, bnear,
-                              bstart, bcand, n,
-                              nb, P, mu, dt, lam, gx_in, gv_in, gx_out, gv_out, grho);
+        gmu_i = adj_force_one(i, pos, vel, rho, nbr4, nbr_count, cells, n, P, mu, dt, lam, gx_in,
+                              gv_in, gx_out, gv_out, grho);
     // per-block sum of d L / d mu (reduced in a fixed order afterwards)
     const float t = block_sum_fixed(gmu_i);
     if (threadIdx.x == 0) gmu_block[blockIdx.x] = t;
 }
 
 struct AdjDensityPair {
-    const float* grho;
     float gi, h2, coef;  // coef = -6 m C6
     float gx, gy, gz;
-    __device__ __forceinline__ void operator()(uint32_t j, float dx, float dy, float dz, float r2) {
+    __device__ __forceinline__ void operator()(float grho_j, float dx, float dy, float dz, float r2) {
         const float a = h2 - r2;
-        const float c = coef * a * a * (gi + __ldg(&grho[j]));
+        const float c = coef * a * a * (gi + grho_j);
         gx = fmaf(c, dx, gx);
         gy = fmaf(c, dy, gy);
         gz = fmaf(c, dz, gz);
     }
 };
 
-// Density adjoint: gx_i += -6 m C6 sum_j (h^2 - r^2)^2 (grho_i + grho_j) x_ij.
+// Density adjoint, and the boundary force's part (gb, adj_boundary_warp):
+// gx_i += gb_i - 6 m C6 sum_j (h^2 - r^2)^2 (grho_i + grho_j) x_ij.
 __device__ __forceinline__ void adj_density_one(uint32_t i, const float4* __restrict__ pos,
                                                 const uint4* __restrict__ nbr4,
                                                 const uint32_t* __restrict__ nbr_count,
                                                 const uint2* __restrict__ cells, uint32_t n,
                                                 const SimParams& P, const float* __restrict__ grho,
+                                                const float4* __restrict__ gb,
                                                 float4* __restrict__ gx) {
     const float4 xi = pos[i];
     AdjDensityPair A;
-    A.grho = grho;
     A.gi = grho[i];
     A.h2 = P.h2;
     A.coef = -6.0f * P.dens_coef;
     A.gx = A.gy = A.gz = 0.0f;
-    visit_force_neighbors(i, xi, pos, nbr4, nbr_count, cells, n, P, A);
+    visit_force_neighbors<4>(i, xi, pos, nbr4, nbr_count, cells, n, P,
+                             [&](uint32_t j) { return __ldg(&grho[j]); }, A);
     float4 g = gx[i];
+    const float4 b = gb[i];
+    g.x += b.x;
+    g.y += b.y;
+    g.z += b.z;
     g.x += A.gx;
     g.y += A.gy;
     g.z += A.gz;
@@ -288,10 +355,11 @@ __device__ __forceinline__ void adj_density_one(uint32_t i, const float4* __rest
 static __global__ void __launch_bounds__(256) adj_density_kernel(
     const float4* __restrict__ pos, const uint4* __restrict__ nbr4,
     const uint32_t* __restrict__ nbr_count, const uint2* __restrict__ cells, uint32_t n,
-    SimParams P, const float* __restrict__ grho, float4* __restrict__ gx) {
+    const __grid_constant__ SimParams P, const float* __restrict__ grho,
+    const float4* __restrict__ gb, float4* __restrict__ gx) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    adj_density_one(i, pos, nbr4, nbr_count, cells, n, P, grho, gx);
+    adj_density_one(i, pos, nbr4, nbr_count, cells, n, P, grho, gb, gx);
 }
 
 // Scatter from the step's sorted order back to the order before the sort:
@@ -309,13 +377,22 @@ static __global__ void __launch_bounds__(256) adj_unpermute_kernel(const uint32_
     bo[q] = b[i];
 }
 
-// Deterministic sum of the per-block mu partials into acc (double).
+// Sum of `count` partials by one warp, in double and in a fixed order (each lane
+// every 32nd, then the lanes); valid in every lane.  One thread adding 256 of
+// them took 24 us of each backward step.
+__device__ __forceinline__ double adj_sum_warp(const float* __restrict__ part, uint32_t count) {
+    double s = 0.0;
+    for (uint32_t k = threadIdx.x & 31u; k < count; k += 32) s += (double)part[k];
+#pragma unroll
+    for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xFFFFFFFFu, s, o);
+    return s;
+}
+
+// The per-block mu partials into acc (one warp).
 static __global__ void adj_sum_kernel(const float* __restrict__ part, uint32_t count,
                                       double* __restrict__ acc) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    double s = 0.0;
-    for (uint32_t k = 0; k < count; ++k) s += (double)part[k];
-    *acc += s;
+    const double s = adj_sum_warp(part, count);
+    if (threadIdx.x == 0) *acc += s;
 }
 
 // Poly6 splat of the particles on the cell centres of a node grid:

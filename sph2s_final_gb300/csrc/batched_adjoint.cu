@@ -39,6 +39,7 @@ struct BRollout {
     std::vector<uint32_t*> cnt;
     std::vector<uint2*> cells;
     float4 *gx = nullptr, *gv = nullptr, *gx2 = nullptr, *gv2 = nullptr, *lam = nullptr;
+    float4* gb = nullptr;  // the boundary force's part of gx2
     float4* gxT = nullptr;
     float* grho = nullptr;
     float* gmu_part = nullptr;  // one partial per 256-particle tile
@@ -64,11 +65,8 @@ constexpr int kTile = 256;
 static __global__ void __launch_bounds__(kTile) b_adj_force_kernel(
     const uint2* __restrict__ tiles, uint32_t num_tiles, const SceneRec* __restrict__ recs,
     const float* __restrict__ mu_s, const float4* __restrict__ pos, const float4* __restrict__ vel,
-    const float* __restrict__ rho, const float2* __restrict__ aux, const uint4* __restrict__ nbr4,
-    const uint32_t* __restrict__ cnt, const uint2* __restrict__ cells,
-    const float4* __restrict__ bpos, const uint2* __restrict__ bcells,
-    const uint8_t* __restrict__ bnear, const uint32_t* __restrict__ bstart,
-    const uint32_t* __restrict__ bcand, uint32_t n, uint32_t nb, float dt,
+    const float* __restrict__ rho, const uint4* __restrict__ nbr4,
+    const uint32_t* __restrict__ cnt, const uint2* __restrict__ cells, uint32_t n, float dt,
     const float4* __restrict__ lam, const float4* __restrict__ gx_in,
     const float4* __restrict__ gv_in, float4* __restrict__ gx_out, float4* __restrict__ gv_out,
     float* __restrict__ grho, float* __restrict__ gmu_tile) {
@@ -79,13 +77,28 @@ static __global__ void __launch_bounds__(kTile) b_adj_force_kernel(
         float g = 0.0f;
         if (i < R.p_off + R.p_n) {
             const SimParams P = R.P;
-            g = adj_force_one(i, pos, vel, rho, aux, nbr4, cnt, cells + R.c_off, bpos,
-                              bcells + R.c_off, bnear + R.c_off, bstart + R.c_off, bcand, n, nb,
-                              P, mu_s[tile.x], dt, lam,
-                              gx_in, gv_in, gx_out, gv_out, grho);
+            g = adj_force_one(i, pos, vel, rho, nbr4, cnt, cells + R.c_off, n, P, mu_s[tile.x], dt,
+                              lam, gx_in, gv_in, gx_out, gv_out, grho);
         }
         const float s = block_sum_fixed(g);
         if (threadIdx.x == 0) gmu_tile[t] = s;
+    }
+}
+
+static __global__ void __launch_bounds__(kTile) b_adj_boundary_kernel(
+    const uint2* __restrict__ tiles, uint32_t num_tiles, const SceneRec* __restrict__ recs,
+    const float4* __restrict__ pos, const float4* __restrict__ lam,
+    const float4* __restrict__ bpos, const uint2* __restrict__ bcells,
+    const uint8_t* __restrict__ bnear, const uint32_t* __restrict__ bstart,
+    const uint32_t* __restrict__ bcand, uint32_t nb, float4* __restrict__ gb) {
+    for (uint32_t t = blockIdx.x; t < num_tiles; t += gridDim.x) {
+        const uint2 tile = tiles[t];
+        const SceneRec& R = recs[tile.x];
+        const uint32_t end = min(tile.y + (uint32_t)kTile, R.p_off + R.p_n);
+        const SimParams P = R.P;
+        for (uint32_t k = tile.y + (threadIdx.x >> 5) * kBndLanes; k < end; k += kTile / 32 * kBndLanes)
+            adj_boundary_warp(k + (threadIdx.x & 31u), end, pos, lam, bpos, bcells + R.c_off,
+                              bnear + R.c_off, bstart + R.c_off, bcand, nb, P, gb);
     }
 }
 
@@ -93,28 +106,26 @@ static __global__ void __launch_bounds__(kTile) b_adj_density_kernel(
     const uint2* __restrict__ tiles, uint32_t num_tiles, const SceneRec* __restrict__ recs,
     const float4* __restrict__ pos, const uint4* __restrict__ nbr4, const uint32_t* __restrict__ cnt,
     const uint2* __restrict__ cells, uint32_t n, const float* __restrict__ grho,
-    float4* __restrict__ gx) {
+    const float4* __restrict__ gb, float4* __restrict__ gx) {
     for (uint32_t t = blockIdx.x; t < num_tiles; t += gridDim.x) {
         const uint2 tile = tiles[t];
         const SceneRec& R = recs[tile.x];
         const uint32_t i = tile.y + threadIdx.x;
         if (i >= R.p_off + R.p_n) continue;
         const SimParams P = R.P;
-        adj_density_one(i, pos, nbr4, cnt, cells + R.c_off, n, P, grho, gx);
+        adj_density_one(i, pos, nbr4, cnt, cells + R.c_off, n, P, grho, gb, gx);
     }
 }
 
-// d L_s / d mu_s: the scene's tile partials in tile order (the single-scale
-// adj_sum_kernel's order over its blocks).
-static __global__ void b_adj_sum_kernel(const float* __restrict__ part,
-                                        const uint32_t* __restrict__ first,
-                                        const uint32_t* __restrict__ count, uint32_t S,
-                                        double* __restrict__ acc) {
-    const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
+// d L_s / d mu_s: the scene's tile partials by one warp (adj_sum_warp, the order of
+// the single-scale sum over its blocks).
+static __global__ void __launch_bounds__(128) b_adj_sum_kernel(
+    const float* __restrict__ part, const uint32_t* __restrict__ first,
+    const uint32_t* __restrict__ count, uint32_t S, double* __restrict__ acc) {
+    const uint32_t s = blockIdx.x * 4 + (threadIdx.x >> 5);
     if (s >= S) return;
-    double sum = 0.0;
-    for (uint32_t k = 0; k < count[s]; ++k) sum += (double)part[first[s] + k];
-    acc[s] += sum;
+    const double sum = adj_sum_warp(part + first[s], count[s]);
+    if ((threadIdx.x & 31u) == 0) acc[s] += sum;
 }
 
 // tiles[t] = (scene, first node of the tile within the scene's node grid)
@@ -195,6 +206,7 @@ int alloc_brollout(sph_batch* b, int T, int K, BRollout** out) {
     if (rc == SPH_OK &&
         ((rc = ralloc(r, &r->gx, N)) || (rc = ralloc(r, &r->gv, N)) || (rc = ralloc(r, &r->gx2, N)) ||
          (rc = ralloc(r, &r->gv2, N)) || (rc = ralloc(r, &r->lam, N)) || (rc = ralloc(r, &r->gxT, N)) ||
+         (rc = ralloc(r, &r->gb, N)) ||
          (rc = ralloc(r, &r->grho, N)) || (rc = ralloc(r, &r->gmu_part, b->ntiles[1])) ||
          (rc = ralloc(r, &r->gmu_acc, b->S)) || (rc = ralloc(r, &r->mu, b->S)) ||
          (rc = ralloc(r, &r->tfirst, b->S)) || (rc = ralloc(r, &r->tcount, b->S)))) {
@@ -400,17 +412,24 @@ int sphb_rollout_backward(sph_batch* b, float* grad_v0, float* grad_x0, double* 
         b->nbr = nbr0;
         b->nbr_count = cnt0;
         for (int k = len - 1; k >= 0; --k) {  // reverse through the segment
-            adj_lambda_kernel<<<blocks, kTile, 0, st>>>(r->gx, r->gv, N, r->dt, r->lam);
+            adj_lambda_kernel<<<blocks, kTile, 0, st>>>(r->gx, r->gv, r->aux[k], N, r->dt, r->lam);
+            // the boundary force's adjoint beside that of the pair forces
+            SPH_CUDA(cudaEventRecord(b->fork, st));
+            SPH_CUDA(cudaStreamWaitEvent(b->side, b->fork, 0));
+            b_adj_boundary_kernel<<<grid, kTile, 0, b->side>>>(
+                b->tiles[1], nt, b->recs, r->xh[k], r->lam, b->bpos, b->bcells, b->bnear, b->bstart,
+                b->bcand, b->NB, r->gb);
+            SPH_CUDA(cudaEventRecord(b->join, b->side));
             b_adj_force_kernel<<<grid, kTile, 0, st>>>(
-                b->tiles[1], nt, b->recs, r->mu, r->xh[k], r->vh[k], r->rho[k], r->aux[k],
-                r->nbr[k], r->cnt[k], r->cells[k], b->bpos, b->bcells, b->bnear, b->bstart,
-                b->bcand, N, b->NB, r->dt,
-                r->lam, r->gx, r->gv, r->gx2, r->gv2, r->grho, r->gmu_part);
-            b_adj_sum_kernel<<<(b->S + 127) / 128, 128, 0, st>>>(r->gmu_part, r->tfirst, r->tcount,
-                                                                b->S, r->gmu_acc);
+                b->tiles[1], nt, b->recs, r->mu, r->xh[k], r->vh[k], r->rho[k], r->nbr[k],
+                r->cnt[k], r->cells[k], N, r->dt, r->lam, r->gx, r->gv, r->gx2, r->gv2, r->grho,
+                r->gmu_part);
+            b_adj_sum_kernel<<<(b->S + 3) / 4, 128, 0, st>>>(r->gmu_part, r->tfirst, r->tcount,
+                                                            b->S, r->gmu_acc);
+            SPH_CUDA(cudaStreamWaitEvent(st, b->join, 0));
             b_adj_density_kernel<<<grid, kTile, 0, st>>>(b->tiles[1], nt, b->recs, r->xh[k],
                                                          r->nbr[k], r->cnt[k], r->cells[k], N,
-                                                         r->grho, r->gx2);
+                                                         r->grho, r->gb, r->gx2);
             adj_unpermute_kernel<<<blocks, kTile, 0, st>>>(r->perm[k], N, r->gx2, r->gv2, r->gx, r->gv);
         }
         SPH_CUDA(cudaGetLastError());

@@ -83,30 +83,26 @@ __device__ __forceinline__ void boundary_sum(const float4& xi, const float4* __r
         }
 }
 
-// Calls f(xk) for the boundary particles a particle at xi (home cell
-// (hx, hy, hz), linear `home`) must test, in the full scan's order: from the
-// home cell's static candidate list where it applies (inside the grid's box,
-// stencil = home +-1 clamped; see boundary_force_kernel), else from the
-// stencil scan cut by depth (boundary_reach).  A superset of the boundary
-// particles within h in both cases; f applies the r < h test itself.
-template <class F>
-__device__ __forceinline__ void visit_boundary(const float4& xi, int hx, int hy, int hz,
-                                               uint32_t home, const float4* __restrict__ bpos,
-                                               const uint2* __restrict__ bcells,
-                                               const uint32_t* __restrict__ bstart,
-                                               const uint32_t* __restrict__ bcand, uint32_t nb,
-                                               const SimParams& P, F&& f) {
+// Whether the static candidate list of a particle's home cell (hx, hy, hz)
+// holds all its boundary neighbours: it lies inside the grid's box and its
+// stencil is home +-1 (clamped); see boundary_force_kernel.
+__device__ __forceinline__ bool boundary_listed(const float4& xi, int hx, int hy, int hz,
+                                                const SimParams& P) {
     const Stencil S = stencil(P.g, xi.x, xi.y, xi.z, P.h);
     const bool inside = xi.x >= P.g.ox && xi.x < P.g.ex && xi.y >= P.g.oy && xi.y < P.g.ey &&
                         xi.z >= P.g.oz && xi.z < P.g.ez;
-    if (bstart && inside && S.x0 == max(hx - 1, 0) && S.x1 == min(hx + 1, P.g.dx - 1) &&
-        S.y0 == max(hy - 1, 0) && S.y1 == min(hy + 1, P.g.dy - 1) &&
-        S.z0 == max(hz - 1, 0) && S.z1 == min(hz + 1, P.g.dz - 1)) {
-        const uint32_t e = __ldg(&bstart[home + 1]);
-        for (uint32_t k = __ldg(&bstart[home]); k < e; ++k)
-            f(__ldg(&bpos[min(__ldg(&bcand[k]), nb - 1)]));
-        return;
-    }
+    return inside && S.x0 == max(hx - 1, 0) && S.x1 == min(hx + 1, P.g.dx - 1) &&
+           S.y0 == max(hy - 1, 0) && S.y1 == min(hy + 1, P.g.dy - 1) &&
+           S.z0 == max(hz - 1, 0) && S.z1 == min(hz + 1, P.g.dz - 1);
+}
+
+// Calls f(xk) for the boundary particles of the stencil at xi, each cell's scan
+// cut by depth (boundary_reach); f applies the r < h test itself.
+template <class F>
+__device__ __forceinline__ void scan_boundary(const float4& xi, const float4* __restrict__ bpos,
+                                              const uint2* __restrict__ bcells, uint32_t nb,
+                                              const SimParams& P, F&& f) {
+    const Stencil S = stencil(P.g, xi.x, xi.y, xi.z, P.h);
     const float reach = boundary_reach(P.g, P.h, P.bmargin, xi.x, xi.y, xi.z);
     for (int cz = S.z0; cz <= S.z1; ++cz)
         for (int cy = S.y0; cy <= S.y1; ++cy) {
@@ -121,6 +117,27 @@ __device__ __forceinline__ void visit_boundary(const float4& xi, int hx, int hy,
                 }
             }
         }
+}
+
+// Calls f(xk) for the boundary particles a particle at xi (home cell
+// (hx, hy, hz), linear `home`) must test, in the full scan's order: from the
+// home cell's static candidate list where it applies (boundary_listed), else
+// from the stencil scan.  A superset of the boundary particles within h in both
+// cases; f applies the r < h test itself.
+template <class F>
+__device__ __forceinline__ void visit_boundary(const float4& xi, int hx, int hy, int hz,
+                                               uint32_t home, const float4* __restrict__ bpos,
+                                               const uint2* __restrict__ bcells,
+                                               const uint32_t* __restrict__ bstart,
+                                               const uint32_t* __restrict__ bcand, uint32_t nb,
+                                               const SimParams& P, F&& f) {
+    if (bstart && boundary_listed(xi, hx, hy, hz, P)) {
+        const uint32_t e = __ldg(&bstart[home + 1]);
+        for (uint32_t k = __ldg(&bstart[home]); k < e; ++k)
+            f(__ldg(&bpos[min(__ldg(&bcand[k]), nb - 1)]));
+        return;
+    }
+    scan_boundary(xi, bpos, bcells, nb, P, f);
 }
 
 // The particle's home cell in the linear cell table.
