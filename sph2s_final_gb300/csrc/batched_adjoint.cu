@@ -47,6 +47,11 @@ struct BRollout {
     float* mu = nullptr;        // per scene
     uint32_t *tfirst = nullptr, *tcount = nullptr;
     bool forward_done = false, have_loss = false;
+    // the segment whose steps the tape holds and the scenes' constants they were
+    // computed with, as in the single-scale rollout
+    int taped = -1;
+    std::vector<SceneRec> taped_recs;
+    float4 *end_pos = nullptr, *end_vel = nullptr;
 };
 
 // Node grid of one scene's density loss; off = first node in the packed field.
@@ -209,7 +214,8 @@ int alloc_brollout(sph_batch* b, int T, int K, BRollout** out) {
          (rc = ralloc(r, &r->gb, N)) ||
          (rc = ralloc(r, &r->grho, N)) || (rc = ralloc(r, &r->gmu_part, b->ntiles[1])) ||
          (rc = ralloc(r, &r->gmu_acc, b->S)) || (rc = ralloc(r, &r->mu, b->S)) ||
-         (rc = ralloc(r, &r->tfirst, b->S)) || (rc = ralloc(r, &r->tcount, b->S)))) {
+         (rc = ralloc(r, &r->tfirst, b->S)) || (rc = ralloc(r, &r->tcount, b->S)) ||
+         (nseg == 1 && ((rc = ralloc(r, &r->end_pos, N)) || (rc = ralloc(r, &r->end_vel, N)))))) {
     }
     if (rc == SPH_OK) {
         std::vector<uint32_t> cnt(b->S);
@@ -224,6 +230,57 @@ int alloc_brollout(sph_batch* b, int T, int K, BRollout** out) {
         return fail(rc, m);
     }
     *out = r;
+    return SPH_OK;
+}
+
+// One segment from the batch's state, every step recorded into the tape.
+int record_segment(sph_batch* b, int len) {
+    BRollout* r = b->rollout;
+    float4 *spos0 = b->spos, *svel0 = b->svel;
+    float* rho0 = b->rho;
+    float2* aux0 = b->aux;
+    uint4* nbr0 = b->nbr;
+    uint32_t* cnt0 = b->nbr_count;
+    uint2* cells0 = b->cells;
+    for (int k = 0; k < len; ++k) {
+        b->spos = r->xh[k];
+        b->svel = r->vh[k];
+        b->cells = r->cells[k];
+        b->rho = r->rho[k];
+        b->aux = r->aux[k];
+        b->nbr = r->nbr[k];
+        b->nbr_count = r->cnt[k];
+        const int out = enqueue_neighborhood(b);
+        cudaMemcpyAsync(r->perm[k], b->vals[out], 4 * (size_t)b->N, cudaMemcpyDeviceToDevice,
+                        b->stream);
+        enqueue_density(b);
+        enqueue_force(b, r->dt);
+    }
+    b->spos = spos0;
+    b->svel = svel0;
+    b->cells = cells0;
+    b->rho = rho0;
+    b->aux = aux0;
+    b->nbr = nbr0;
+    b->nbr_count = cnt0;
+    SPH_CUDA(cudaGetLastError());
+    return SPH_OK;
+}
+
+// The forward pass's last segment, recorded: the backward pass need not run it
+// again.  The densities the batch shows are those of the last step, as ever.
+int advance_recorded(sph_batch* b, int seg, int len) {
+    BRollout* r = b->rollout;
+    const size_t N = b->N;
+    int rc = record_segment(b, len);
+    if (rc != SPH_OK) return rc;
+    SPH_CUDA(cudaMemcpyAsync(b->rho, r->rho[len - 1], 4 * N, cudaMemcpyDeviceToDevice, b->stream));
+    if (r->end_pos) {
+        SPH_CUDA(cudaMemcpyAsync(r->end_pos, b->pos, 16 * N, cudaMemcpyDeviceToDevice, b->stream));
+        SPH_CUDA(cudaMemcpyAsync(r->end_vel, b->vel, 16 * N, cudaMemcpyDeviceToDevice, b->stream));
+    }
+    r->taped = seg;
+    r->taped_recs = b->recs_h;
     return SPH_OK;
 }
 
@@ -259,6 +316,7 @@ int sphb_rollout_forward(sph_batch* b, const float* v0_xyz, const float* viscosi
     BRollout* r = b->rollout;
     r->dt = dt;
     r->forward_done = r->have_loss = false;
+    r->taped = -1;
     SPH_CUDA(cudaStreamSynchronize(b->stream));
     if (viscosity)
         for (uint32_t s = 0; s < b->S; ++s) b->cfgs[s].viscosity = viscosity[s];
@@ -280,7 +338,8 @@ int sphb_rollout_forward(sph_batch* b, const float* v0_xyz, const float* viscosi
     for (int c = 0; c < nseg; ++c) {
         SPH_CUDA(cudaMemcpyAsync(r->ck_pos[c], b->pos, 16 * (size_t)N, cudaMemcpyDeviceToDevice, b->stream));
         SPH_CUDA(cudaMemcpyAsync(r->ck_vel[c], b->vel, 16 * (size_t)N, cudaMemcpyDeviceToDevice, b->stream));
-        rc = sphb_advance(b, dt, std::min(K, steps - c * K));
+        const int len = std::min(K, steps - c * K);
+        rc = c == nseg - 1 ? advance_recorded(b, c, len) : sphb_advance(b, dt, len);
         if (rc != SPH_OK) return rc;
     }
     rc = sphb_sync(b);
@@ -377,40 +436,24 @@ int sphb_rollout_backward(sph_batch* b, float* grad_v0, float* grad_x0, double* 
     SPH_CUDA(cudaMemcpyAsync(r->gx, r->gxT, 16 * (size_t)N, cudaMemcpyDeviceToDevice, st));
     SPH_CUDA(cudaMemsetAsync(r->gv, 0, 16 * (size_t)N, st));
     SPH_CUDA(cudaMemsetAsync(r->gmu_acc, 0, 8 * (size_t)b->S, st));
-    // the step's own buffers, redirected into the tape while recording
-    float4 *spos0 = b->spos, *svel0 = b->svel;
-    float* rho0 = b->rho;
-    float2* aux0 = b->aux;
-    uint4* nbr0 = b->nbr;
-    uint32_t* cnt0 = b->nbr_count;
-    uint2* cells0 = b->cells;
+    if (r->taped >= 0)
+        for (uint32_t k = 0; k < b->S; ++k)
+            if (std::memcmp(&r->taped_recs[k].P, &b->recs_h[k].P, sizeof(SimParams))) r->taped = -1;
     const uint32_t blocks = (N + kTile - 1) / kTile;
     const uint32_t nt = b->ntiles[1];
     const uint32_t grid = tile_grid(b, nt);
     for (int c = nseg - 1; c >= 0; --c) {
         const int t0 = c * r->K, len = std::min(r->K, r->T - t0);
-        SPH_CUDA(cudaMemcpyAsync(b->pos, r->ck_pos[c], 16 * (size_t)N, cudaMemcpyDeviceToDevice, st));
-        SPH_CUDA(cudaMemcpyAsync(b->vel, r->ck_vel[c], 16 * (size_t)N, cudaMemcpyDeviceToDevice, st));
-        for (int k = 0; k < len; ++k) {  // recompute the segment, recording the tape
-            b->spos = r->xh[k];
-            b->svel = r->vh[k];
-            b->cells = r->cells[k];
-            b->rho = r->rho[k];
-            b->aux = r->aux[k];
-            b->nbr = r->nbr[k];
-            b->nbr_count = r->cnt[k];
-            const int out = enqueue_neighborhood(b);
-            cudaMemcpyAsync(r->perm[k], b->vals[out], 4 * (size_t)N, cudaMemcpyDeviceToDevice, st);
-            enqueue_density(b);
-            enqueue_force(b, r->dt);
+        const bool taped = c == r->taped;
+        if (!taped || c == 0) {  // the call leaves the batch at the end of its first segment
+            SPH_CUDA(cudaMemcpyAsync(b->pos, taped ? r->end_pos : r->ck_pos[c], 16 * (size_t)N, cudaMemcpyDeviceToDevice, st));
+            SPH_CUDA(cudaMemcpyAsync(b->vel, taped ? r->end_vel : r->ck_vel[c], 16 * (size_t)N, cudaMemcpyDeviceToDevice, st));
         }
-        b->spos = spos0;
-        b->svel = svel0;
-        b->cells = cells0;
-        b->rho = rho0;
-        b->aux = aux0;
-        b->nbr = nbr0;
-        b->nbr_count = cnt0;
+        if (!taped) {
+            r->taped = -1;
+            const int rc = record_segment(b, len);
+            if (rc != SPH_OK) return rc;
+        }
         for (int k = len - 1; k >= 0; --k) {  // reverse through the segment
             adj_lambda_kernel<<<blocks, kTile, 0, st>>>(r->gx, r->gv, r->aux[k], N, r->dt, r->lam);
             // the boundary force's adjoint beside that of the pair forces
