@@ -71,9 +71,9 @@ uint32_t pgrid(const sph_batch* b, uint32_t tiles) {
 
 template <int BS>
 void launch_density(sph_batch* b, int ti) {
-    b_density_kernel<BS><<<pgrid(b, b->ntiles[ti]), BS, 0, b->stream>>>(
-        b->tiles[ti], b->ntiles[ti], b->recs, b->spos, b->cells, b->N, b->rho, b->aux, b->nbr,
-        b->nbr_count, b->xa, b->svel);
+    launch_after(b_density_kernel<BS>, pgrid(b, b->ntiles[ti]), BS, b->stream, b->tiles[ti],
+                 b->ntiles[ti], b->recs, b->spos, b->cells, b->N, b->rho, b->aux, b->nbr,
+                 b->nbr_count, b->xa, b->svel);
 }
 
 template <int BS>
@@ -117,25 +117,26 @@ void enqueue_force(sph_batch* b, float dt) {
 // the same permutation, radix-sorting only the particles that changed cell).
 int enqueue_neighborhood(sph_batch* b) {
     cudaStream_t st = b->stream;
-    cudaMemsetAsync(b->cells, 0xFF, sizeof(uint2) * b->NC, st);
     int o = 1;
+    StepClear clear = {b->cells, b->NC, nullptr, 0u, nullptr};
     if (b->coherent) {
         b_hash_hist_kernel<256><<<pgrid(b, b->ntiles[1]), 256, 0, st>>>(
-            b->tiles[1], b->ntiles[1], b->recs, b->pos, b->shift, 0, b->keys[0], b->sort.hist);
+            b->tiles[1], b->ntiles[1], b->recs, b->pos, b->shift, 0, b->keys[0], b->sort.hist,
+            clear);
         coherent_sort_keys(b->co, b->keys[0], 8 * b->passes, b->keys[1], b->vals[1], b->err, 0,
                            st);
     } else {
-        sort_reset(b->sort, st);
+        clear.words = b->sort.tile_ctr;
+        clear.nwords = sort_step_words(b->N, b->passes);
         b_hash_hist_kernel<256><<<pgrid(b, b->ntiles[1]), 256, 0, st>>>(
             b->tiles[1], b->ntiles[1], b->recs, b->pos, b->shift, b->passes, b->keys[0],
-            b->sort.hist);
-        sort_scan(b->passes, b->sort, st);
-        o = sort_passes_run(b->keys, b->vals, nullptr, b->N, b->passes, b->sort, b->err, 0, st);
+            b->sort.hist, clear);
+        o = sort_step_run(b->keys, b->vals, b->N, b->passes, b->sort, b->err, 0, st);
     }
-    b_gather_cells_kernel<256, true><<<pgrid(b, b->ntiles[1]), 256, 0, st>>>(
-        b->tiles[1], b->ntiles[1], b->recs, b->keys[o], b->vals[o], b->N, b->shift, false, b->pos,
-        b->vel, b->spos, b->svel, b->cells, b->err, 0, b->coherent ? b->co.kprev : nullptr,
-        b->bnear, b->bflag);
+    launch_after(b_gather_cells_kernel<256, true>, pgrid(b, b->ntiles[1]), 256, st, b->tiles[1],
+                 b->ntiles[1], b->recs, b->keys[o], b->vals[o], b->N, b->shift, false, b->pos,
+                 b->vel, b->spos, b->svel, b->cells, b->err, 0,
+                 b->coherent ? b->co.kprev : nullptr, b->bnear, b->bflag, b->sort.hist);
     return o;
 }
 
@@ -262,9 +263,11 @@ int sphb_create(const sph_scene_desc* scenes, uint32_t num_scenes, sph_batch** o
     TRY(dalloc(&b->bflag, b->N, b->owned));
     TRY(check_cuda(cudaMemset(b->bacc, 0, 16 * (size_t)std::max(b->N, 1u)), "memset", __FILE__, __LINE__));
     TRY(dalloc(&b->bpos, b->NB, b->owned));
-    TRY(check_cuda(cudaMalloc(&b->sort_mem, sort_scratch_bytes(nmax)), "sort scratch", __FILE__, __LINE__));
+    const uint32_t plan = std::max(nmax, sort_step_plan_keys(b->N));
+    TRY(check_cuda(cudaMalloc(&b->sort_mem, sort_scratch_bytes(plan)), "sort scratch", __FILE__, __LINE__));
     b->owned.push_back(b->sort_mem);
-    b->sort = sort_scratch_from(b->sort_mem, nmax);
+    b->sort = sort_scratch_from(b->sort_mem, plan);
+    sort_reset(b->sort, b->stream);
     b->coherent = b->N >= 131072u;
     if (b->coherent) {
         TRY(check_cuda(cudaMalloc(&b->co_mem, coherent_bytes(b->N)), "sort scratch", __FILE__, __LINE__));
@@ -336,12 +339,12 @@ int sphb_create(const sph_scene_desc* scenes, uint32_t num_scenes, sph_batch** o
             b_boundary_hash_hist_kernel<256><<<pgrid(b, b->nbtiles), 256, 0, b->stream>>>(
                 b->btiles, b->nbtiles, b->recs, braw, b->shift, qb, bpasses, b->keys[0],
                 b->sort.hist);
-            sort_scan(bpasses, b->sort, b->stream);
             const int o = sort_passes_run(b->keys, b->vals, nullptr, b->NB, bpasses, b->sort,
                                           b->err, 0, b->stream);
             b_gather_cells_kernel<256, false><<<pgrid(b, b->nbtiles), 256, 0, b->stream>>>(
                 b->btiles, b->nbtiles, b->recs, b->keys[o], b->vals[o], b->NB, b->shift, true, braw,
-                nullptr, b->bpos, nullptr, b->bcells, b->err, qb);
+                nullptr, b->bpos, nullptr, b->bcells, b->err, qb, nullptr, nullptr, nullptr,
+                b->sort.hist);
             TRY(check_cuda(cudaStreamSynchronize(b->stream), "boundary presort", __FILE__, __LINE__));
             cudaFree(braw);
             b->owned.pop_back();

@@ -33,9 +33,11 @@ __global__ void __launch_bounds__(BS) b_hash_hist_kernel(const uint2* __restrict
                                                          const float4* __restrict__ pos,
                                                          int shift, int passes,
                                                          uint32_t* __restrict__ keys,
-                                                         uint32_t* __restrict__ hist) {
+                                                         uint32_t* __restrict__ hist,
+                                                         const StepClear clear) {
     __shared__ uint32_t sh[kSortMaxPasses][256];
     for (int i = threadIdx.x; i < kSortMaxPasses * 256; i += blockDim.x) (&sh[0][0])[i] = 0;
+    step_clear(clear);
     __syncthreads();
     for (uint32_t t = blockIdx.x; t < num_tiles; t += gridDim.x) {
         const uint2 tile = tiles[t];
@@ -99,14 +101,18 @@ __global__ void __launch_bounds__(BS) b_gather_cells_kernel(
     int shift, bool boundary, const float4* __restrict__ pos_in, const float4* __restrict__ vel_in,
     float4* __restrict__ pos_out, float4* __restrict__ vel_out, uint2* __restrict__ cells,
     uint32_t* __restrict__ err, int key_shift = 0, uint32_t* __restrict__ kprev_out = nullptr,
-    const uint8_t* __restrict__ bnear = nullptr, uint8_t* __restrict__ bflag = nullptr) {
+    const uint8_t* __restrict__ bnear = nullptr, uint8_t* __restrict__ bflag = nullptr,
+    uint32_t* __restrict__ hist = nullptr) {
+    grid_wait();
+    if (hist && blockIdx.x == 0)  // the sort's histograms, for the next step
+        for (int k = threadIdx.x; k < kSortMaxPasses * 256; k += blockDim.x) hist[k] = 0;
     const uint32_t lmask = (1u << shift) - 1u;
     for (uint32_t t = blockIdx.x; t < num_tiles; t += gridDim.x) {
         const uint2 tile = tiles[t];
         const SceneRec& R = recs[tile.x];
         const uint32_t beg = boundary ? R.b_off : R.p_off;
         const uint32_t end = beg + (boundary ? R.b_n : R.p_n);
-        const uint32_t i = tile.y + threadIdx.x;
+        const uint32_t i = after_wait(tile.y + threadIdx.x);
         if (i >= end) continue;
         if (kprev_out) kprev_out[i] = keys_sorted[i];  // the next coherent sort starts here
         uint32_t q = perm[i];
@@ -143,10 +149,11 @@ __global__ void __launch_bounds__(BS) b_density_kernel(
     const float4* __restrict__ pos, const uint2* __restrict__ cells, uint32_t n,
     float* __restrict__ rho, float2* __restrict__ aux, uint4* __restrict__ nbr4,
     uint32_t* __restrict__ nbr_count, float4* __restrict__ xa, float4* __restrict__ svel) {
+    grid_wait();
     for (uint32_t t = blockIdx.x; t < num_tiles; t += gridDim.x) {
         const uint2 tile = tiles[t];
         const SceneRec& R = recs[tile.x];
-        const uint32_t i = tile.y + threadIdx.x;
+        const uint32_t i = after_wait(tile.y + threadIdx.x);
         if (i >= R.p_off + R.p_n) continue;
         const SimParams P = R.P;
         density_one<false>(i, pos, cells + R.c_off, n, P, rho, aux, nbr4, nbr_count, nullptr, xa,

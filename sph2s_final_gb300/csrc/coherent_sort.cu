@@ -22,8 +22,9 @@ template <bool FROM_POS>
 __global__ void __launch_bounds__(kCoThreads) coherent_flag_kernel(
     const float4* __restrict__ pos, GridParams g, uint32_t* __restrict__ keys, uint32_t n,
     const uint32_t* __restrict__ kprev, uint32_t* __restrict__ flags,
-    uint32_t* __restrict__ toff) {
+    uint32_t* __restrict__ toff, const StepClear clear) {
     __shared__ uint32_t s_cnt[kCoWarps];
+    step_clear(clear);
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const uint32_t base = blockIdx.x * kCoTile;
     uint32_t cnt = 0;
@@ -64,6 +65,7 @@ __global__ void __launch_bounds__(1024) coherent_scan_kernel(uint32_t* __restric
     __shared__ uint32_t s_carry;
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     if (tid == 0) s_carry = 0;
+    grid_wait();
     __syncthreads();
     for (uint32_t b = 0; b < tiles; b += 1024) {
         const uint32_t i = b + tid;
@@ -107,6 +109,10 @@ __global__ void __launch_bounds__(kCoThreads) coherent_compact_kernel(
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     for (int i = tid; i < kSortMaxPasses * 256; i += kCoThreads) (&sh[0][0])[i] = 0;
     const uint32_t nwords = (n + 31) >> 5;
+    grid_wait();
+    flags = after_wait(flags);
+    toff = after_wait(toff);
+    keys = after_wait(keys);
     const uint32_t w0 = blockIdx.x * kWords;
     if (tid < kWords) {
         const uint32_t w = w0 + tid;
@@ -190,7 +196,12 @@ __global__ void __launch_bounds__(256) coherent_merge_kernel(
     uint32_t* __restrict__ perm_out, const float4* __restrict__ rec_a,
     const float4* __restrict__ rec_b, float4* __restrict__ out_a, float4* __restrict__ out_b,
     uint32_t* __restrict__ err) {
-    const uint32_t m = min(*m_dev, n);
+    grid_wait();
+    smk = after_wait(smk);
+    smv = after_wait(smv);
+    flags = after_wait(flags);
+    wpre = after_wait(wpre);
+    const uint32_t m = min(*after_wait(m_dev), n);
     if (blockIdx.x < kMoverBlocks) {
         const uint32_t stride = kMoverBlocks * 256;
         for (uint32_t r = blockIdx.x * 256 + threadIdx.x; r < m; r += stride) {
@@ -363,31 +374,35 @@ inline size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 void coherent_run(const CoherentSort& c, const float4* pos, const GridParams* g,
                   const uint2* cells_prev, uint32_t* keys, int key_bits, uint32_t* keys_out,
                   uint32_t* perm_out, const float4* rec_a, const float4* rec_b, float4* out_a,
-                  float4* out_b, uint32_t* err, int force_timeout, cudaStream_t st) {
+                  float4* out_b, uint32_t* err, int force_timeout, cudaStream_t st,
+                  uint32_t* near_count = nullptr) {
     const SortScratch& s = c.sort;
     const uint32_t n = c.n;
     if (n == 0) return;
     const uint32_t tiles = coherent_tiles(n);
     const int passes = sort_passes(key_bits);
-    sort_reset(s, st);
+    // the sort's histograms, tile counters and look-back words are one block
+    const StepClear clear = {nullptr, 0u, s.hist,
+                             (uint32_t)(s.tile_ctr - s.hist) +
+                                 sort_pass_words(sort_tiles(n, kMoverSmallMax, true), passes),
+                             near_count};
     if (pos)
         coherent_flag_kernel<true><<<tiles, kCoThreads, 0, st>>>(pos, *g, keys, n, c.kprev,
-                                                                 c.flags, c.toff);
+                                                                 c.flags, c.toff, clear);
     else
         coherent_flag_kernel<false><<<tiles, kCoThreads, 0, st>>>(nullptr, GridParams{}, keys, n,
-                                                                  c.kprev, c.flags, c.toff);
-    coherent_scan_kernel<<<1, 1024, 0, st>>>(c.toff, tiles);
-    coherent_compact_kernel<<<tiles, kCoThreads, 0, st>>>(keys, n, c.flags, c.toff, c.wpre,
-                                                          c.mk[0], c.mv[0], passes, s.hist);
-    sort_scan(passes, s, st);
+                                                                  c.kprev, c.flags, c.toff, clear);
+    launch_after(coherent_scan_kernel, 1, 1024, st, c.toff, tiles);
+    launch_after(coherent_compact_kernel, tiles, kCoThreads, st, keys, n, c.flags, c.toff, c.wpre,
+                 c.mk[0], c.mv[0], passes, s.hist);
     uint32_t* mk[2] = {c.mk[0], c.mk[1]};
     uint32_t* mv[2] = {c.mv[0], c.mv[1]};
     const int o = sort_passes_run_dev(mk, mv, c.mv[0], n, c.toff + tiles, kMoverSmallMax, passes,
                                       s, err, force_timeout, st);
     const uint32_t stay_blocks = (n + 255) / 256;
-    coherent_merge_kernel<<<kMoverBlocks + stay_blocks, 256, 0, st>>>(
-        c.kprev, n, c.flags, c.wpre, c.toff + tiles, mk[o], mv[o], cells_prev,
-        g ? *g : GridParams{}, keys_out, perm_out, rec_a, rec_b, out_a, out_b, err);
+    launch_after(coherent_merge_kernel, kMoverBlocks + stay_blocks, 256, st, c.kprev, n, c.flags,
+                 c.wpre, c.toff + tiles, mk[o], mv[o], cells_prev, g ? *g : GridParams{}, keys_out,
+                 perm_out, rec_a, rec_b, out_a, out_b, err);
 }
 
 }  // namespace
@@ -430,7 +445,7 @@ void coherent_sort_cells(const CoherentSort& c, const float4* pos, const float4*
                          uint32_t* keys_out, uint32_t* perm_out, float4* pos_out, float4* vel_out,
                          uint32_t* err, int force_timeout, cudaStream_t st, NearList near) {
     coherent_run(c, pos, &g, cells, keys, key_bits, keys_out, perm_out, pos, vel, pos_out, vel_out,
-                 err, force_timeout, st);
+                 err, force_timeout, st, near.count);
     if (c.n == 0) return;
     cudaMemsetAsync(cells, 0xFF, sizeof(uint2) * (size_t)g.dx * g.dy * g.dz, st);
     coherent_cells_kernel<<<(c.n + kCellsThreads - 1) / kCellsThreads, kCellsThreads, 0, st>>>(

@@ -246,6 +246,56 @@ inline void clear_run(const ClearBatch& b, int sms, cudaStream_t st) {
     clear_kernel<<<(uint32_t)(blocks < most ? blocks : most), 256, 0, st>>>(b);
 }
 
+// What a step starts from cleared, written by its first kernel (one launch and no
+// memsets before the sort): the cell table, the sort's tile counters and look-back
+// words, and the count of the near list (NULL: none).
+struct StepClear {
+    uint2* cells;
+    uint32_t ncells;
+    uint32_t* words;
+    uint32_t nwords;
+    uint32_t* count;
+};
+
+__device__ __forceinline__ void step_clear(const StepClear& c) {
+    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
+    for (uint32_t i = t; i < c.ncells; i += stride) c.cells[i] = make_uint2(~0u, ~0u);
+    for (uint32_t i = t; i < c.nwords; i += stride) c.words[i] = 0u;
+    if (t == 0 && c.count) *c.count = 0u;
+}
+
+// Launches a kernel that waits for its predecessor in the stream by grid_wait()
+// before it touches memory: its blocks are set up while the predecessor drains.
+template <class... P, class... A>
+inline void launch_after(void (*kernel)(P...), uint32_t grid, uint32_t block, cudaStream_t st,
+                         A... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.stream = st;
+    cudaLaunchAttribute at = {};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+}
+
+// Waits for the predecessor's end; its writes are visible after this.  Loads
+// through const __restrict__ pointers count as read-only for the whole kernel and
+// might be moved above: what their addresses follow from (an index, a pointer)
+// passes through after_wait first.
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+template <class T>
+__device__ __forceinline__ T after_wait(T x) {
+    if constexpr (sizeof(T) == 8)
+        asm volatile("" : "+l"(x));
+    else
+        asm volatile("" : "+r"(x));
+    return x;
+}
+
 // Boundary weight shape of evaluateBoundaryWeight (Solver.cu:169-196)
 // without the 0.02 c^2 / r factor: q = 2r/h.
 __device__ __forceinline__ float boundary_shape(float q) {

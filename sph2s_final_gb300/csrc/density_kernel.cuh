@@ -95,7 +95,8 @@ __global__ void __launch_bounds__(kDensityThreads) density_kernel(
     float* __restrict__ rho, float2* __restrict__ aux, uint4* __restrict__ nbr4,
     uint32_t* __restrict__ nbr_count, uint32_t* __restrict__ dbg_count, float4* __restrict__ xa,
     float4* __restrict__ svel) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    grid_wait();
+    const uint32_t i = after_wait(blockIdx.x * blockDim.x + threadIdx.x);
     if (i >= n) return;
     density_one<DEBUG>(i, pos, cells, n, P, rho, aux, nbr4, nbr_count, dbg_count, xa, svel);
 }

@@ -1,5 +1,6 @@
 // radix_sort.cu -- onesweep LSD radix sort (see radix_sort.cuh).
 #include "radix_sort.cuh"
+#include "common.cuh"
 #include "errors.h"
 
 namespace sph {
@@ -25,23 +26,28 @@ __device__ __forceinline__ void st_relaxed(uint32_t* p, uint32_t v) {
     asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
 
-// Exclusive scan of one value per thread over a 256-thread block.
-__device__ __forceinline__ uint32_t block_exclusive_scan(uint32_t v, uint32_t* s_warp) {
+// Exclusive scans of two values per thread over a 256-thread block.
+__device__ __forceinline__ uint2 block_exclusive_scan2(uint32_t v, uint32_t w, uint2* s_warp) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    uint32_t x = v;
+    uint32_t x = v, z = w;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-        uint32_t y = __shfl_up_sync(0xFFFFFFFFu, x, o);
-        if (lane >= o) x += y;
+        const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, x, o), u = __shfl_up_sync(0xFFFFFFFFu, z, o);
+        if (lane >= o) {
+            x += y;
+            z += u;
+        }
     }
-    if (lane == 31) s_warp[warp] = x;
+    if (lane == 31) s_warp[warp] = make_uint2(x, z);
     __syncthreads();
-    uint32_t wpre = 0;
+    uint32_t xp = 0, zp = 0;
 #pragma unroll
-    for (int w = 0; w < kWarps; ++w)
-        if (w < warp) wpre += s_warp[w];
-    __syncthreads();
-    return wpre + x - v;
+    for (int k = 0; k < kWarps; ++k)
+        if (k < warp) {
+            xp += s_warp[k].x;
+            zp += s_warp[k].y;
+        }
+    return make_uint2(xp + x - v, zp + z - w);
 }
 
 __global__ void __launch_bounds__(256) histogram_kernel(const uint32_t* __restrict__ keys,
@@ -59,36 +65,25 @@ __global__ void __launch_bounds__(256) histogram_kernel(const uint32_t* __restri
     }
 }
 
-__global__ void __launch_bounds__(256) scan_kernel(uint32_t* hist, int passes) {
-    __shared__ uint32_t s_warp[kWarps];
-    for (int p = 0; p < passes; ++p) {
-        uint32_t v = hist[p * 256 + threadIdx.x];
-        uint32_t e = block_exclusive_scan(v, s_warp);
-        hist[p * 256 + threadIdx.x] = e;
-    }
-}
-
 __global__ void __launch_bounds__(kSortThreads) onesweep_kernel(
     const uint32_t* __restrict__ keys_in, const uint32_t* __restrict__ vals_in,
     uint32_t* __restrict__ keys_out, uint32_t* __restrict__ vals_out, uint32_t n,
     const uint32_t* __restrict__ n_dev, uint32_t small_max, int shift,
-    const uint32_t* __restrict__ digit_offsets, uint32_t* status, uint32_t* tile_ctr,
+    const uint32_t* __restrict__ hist, uint32_t* status, uint32_t* tile_ctr,
     uint32_t* err, int force_timeout) {
     __shared__ uint32_t s_keys[kSortTile];
     __shared__ uint32_t s_vals[kSortTile];
     __shared__ uint32_t s_whist[kWarps][257];  // column 256 collects out-of-range items
     __shared__ uint32_t s_local_start[256];
     __shared__ uint32_t s_gbase[256];
-    __shared__ uint32_t s_warp[kWarps];
+    __shared__ uint2 s_warp[kWarps];
     __shared__ uint32_t s_tile;
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    int ni = kSortItems;  // keys per thread
-    if (n_dev) {  // key count known on the device only: the grid covers n keys
-        n = min(*n_dev, n);
-        if (n == 0) return;
-        if (n <= small_max) ni = kSortItemsSmall;  // few keys: more, smaller tiles
-    }
+    grid_wait();
+    if (n_dev) n = min(*after_wait(n_dev), n);  // key count known on the device only: the grid covers n keys
+    if (n == 0) return;
+    const int ni = n <= small_max ? kSortItemsSmall : kSortItems;  // keys per thread
     const uint32_t tile_keys = (uint32_t)ni * kSortThreads;
     if (tid == 0) s_tile = atomicAdd(tile_ctr, 1u);
     for (int i = tid; i < kWarps * 257; i += kSortThreads) (&s_whist[0][0])[i] = 0;
@@ -97,6 +92,7 @@ __global__ void __launch_bounds__(kSortThreads) onesweep_kernel(
     const uint32_t base = tile * tile_keys;
     if (base >= n) return;  // tiles are handed out in order: no later tile waits on this one
     const uint32_t seg = base + (uint32_t)warp * ((uint32_t)ni * 32);
+    const uint32_t digit_total = after_wait(hist)[tid];
 
     uint32_t k[kSortItems], v[kSortItems], rank[kSortItems];
 #pragma unroll
@@ -134,7 +130,10 @@ __global__ void __launch_bounds__(kSortThreads) onesweep_kernel(
     uint32_t* my_status = status + (size_t)tile * 256 + tid;
     st_relaxed(my_status, (tile == 0 ? kFlagPfx : kFlagAgg) | total);
 
-    uint32_t local_start = block_exclusive_scan(total, s_warp);
+    // every tile scans the digit histogram itself, beside its own counts: a kernel
+    // for it cost a launch of its own in the chain
+    const uint2 start = block_exclusive_scan2(total, digit_total, s_warp);
+    const uint32_t local_start = start.x;
     s_local_start[tid] = local_start;
 
     uint32_t prefix = 0;
@@ -159,7 +158,7 @@ __global__ void __launch_bounds__(kSortThreads) onesweep_kernel(
         }
         st_relaxed(my_status, kFlagPfx | ((prefix + total) & kValMask));
     }
-    s_gbase[tid] = digit_offsets[tid] + prefix - local_start;
+    s_gbase[tid] = start.y + prefix - local_start;
     __syncthreads();
 
 #pragma unroll
@@ -178,8 +177,10 @@ __global__ void __launch_bounds__(kSortThreads) onesweep_kernel(
     for (uint32_t i = tid; i < tile_n; i += kSortThreads) {
         uint32_t key = s_keys[i];
         uint32_t g = s_gbase[(key >> shift) & 255u] + i;
-        keys_out[g] = key;
-        vals_out[g] = s_vals[i];
+        if (g < n) {
+            keys_out[g] = key;
+            vals_out[g] = s_vals[i];
+        }
     }
 }
 
@@ -215,10 +216,6 @@ void sort_histogram(const uint32_t* keys, uint32_t n, int passes, const SortScra
     histogram_kernel<<<blocks, 256, 0, st>>>(keys, n, passes, s.hist);
 }
 
-void sort_scan(int passes, const SortScratch& s, cudaStream_t st) {
-    scan_kernel<<<1, 256, 0, st>>>(s.hist, passes);
-}
-
 void sort_pass(const uint32_t* keys_in, const uint32_t* vals_in, uint32_t* keys_out,
                uint32_t* vals_out, uint32_t n, int p, const SortScratch& s, uint32_t* err,
                int force_timeout, cudaStream_t st) {
@@ -226,25 +223,27 @@ void sort_pass(const uint32_t* keys_in, const uint32_t* vals_in, uint32_t* keys_
     uint32_t tiles = (n + kSortTile - 1) / kSortTile;
     onesweep_kernel<<<tiles, kSortThreads, 0, st>>>(
         keys_in, vals_in, keys_out, vals_out, n, nullptr, 0u, 8 * p, s.hist + p * 256,
-        s.status + (size_t)p * s.max_tiles * 256, s.tile_ctr + p, err, force_timeout);
+        s.status + (size_t)p * tiles * 256, s.tile_ctr + p, err, force_timeout);
+}
+
+uint32_t sort_tiles(uint32_t n, uint32_t small_max, bool counted) {
+    const uint32_t tiles = (n + kSortTile - 1) / kSortTile;
+    const uint32_t few = counted ? (n < small_max ? n : small_max) : (n <= small_max ? n : 0u);
+    const uint32_t small_tiles = (few + kSortTileSmall - 1) / kSortTileSmall;
+    return small_tiles > tiles ? small_tiles : tiles;
 }
 
 int sort_passes_run_dev(uint32_t* keys[2], uint32_t* vals[2], const uint32_t* first_vals,
                         uint32_t n, const uint32_t* n_dev, uint32_t small_max, int passes,
                         const SortScratch& s, uint32_t* err, int force_timeout, cudaStream_t st) {
     if (n == 0) return 0;
-    uint32_t tiles = (n + kSortTile - 1) / kSortTile;
-    if (n_dev) {
-        const uint32_t few = n < small_max ? n : small_max;
-        const uint32_t small_tiles = (few + kSortTileSmall - 1) / kSortTileSmall;
-        if (small_tiles > tiles) tiles = small_tiles;
-    }
+    const uint32_t tiles = sort_tiles(n, small_max, n_dev != nullptr);
     int cur = 0;
     for (int p = 0; p < passes; ++p) {
         const uint32_t* vin = (p == 0) ? first_vals : vals[cur];
-        onesweep_kernel<<<tiles, kSortThreads, 0, st>>>(
-            keys[cur], vin, keys[cur ^ 1], vals[cur ^ 1], n, n_dev, small_max, 8 * p, s.hist + p * 256,
-            s.status + (size_t)p * s.max_tiles * 256, s.tile_ctr + p, err, force_timeout);
+        launch_after(onesweep_kernel, tiles, kSortThreads, st, keys[cur], vin, keys[cur ^ 1],
+                     vals[cur ^ 1], n, n_dev, small_max, 8 * p, s.hist + p * 256,
+                     s.status + (size_t)p * tiles * 256, s.tile_ctr + p, err, force_timeout);
         cur ^= 1;
     }
     return cur;
@@ -257,12 +256,17 @@ int sort_passes_run(uint32_t* keys[2], uint32_t* vals[2], const uint32_t* first_
                                force_timeout, st);
 }
 
+int sort_step_run(uint32_t* keys[2], uint32_t* vals[2], uint32_t n, int passes,
+                  const SortScratch& s, uint32_t* err, int force_timeout, cudaStream_t st) {
+    return sort_passes_run_dev(keys, vals, nullptr, n, nullptr, kSortStepSmall, passes, s, err,
+                               force_timeout, st);
+}
+
 int sort_pairs(uint32_t* keys[2], uint32_t* vals[2], uint32_t n, int key_bits,
                const SortScratch& s, uint32_t* err, int force_timeout, cudaStream_t st) {
     int passes = sort_passes(key_bits);
     sort_reset(s, st);
     sort_histogram(keys[0], n, passes, s, st);
-    sort_scan(passes, s, st);
     return sort_passes_run(keys, vals, vals[0], n, passes, s, err, force_timeout, st);
 }
 

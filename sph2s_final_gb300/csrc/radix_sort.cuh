@@ -27,13 +27,17 @@ constexpr int kSortTile = kSortThreads * kSortItems;  // 4096 keys
 constexpr int kSortItemsSmall = 2;
 constexpr int kSortTileSmall = kSortThreads * kSortItemsSmall;
 constexpr int kSortMaxPasses = 4;
+// A step's sort of at most this many keys uses the small tiles: 4,096 keys are
+// then 8 tiles instead of one (58 -> 56 us per step); at 32,768 both take the
+// same, and 94,608 in 185 small tiles look back too far (89 -> 94 us per step).
+constexpr uint32_t kSortStepSmall = 1u << 14;
 
 // Device scratch of one sort plan.  Everything that must start at zero lives
 // in one contiguous block so a single memset resets it.
 struct SortScratch {
-    uint32_t* hist;      // [kSortMaxPasses][256] histograms, then exclusive offsets
+    uint32_t* hist;      // [kSortMaxPasses][256] histograms
     uint32_t* tile_ctr;  // [kSortMaxPasses]
-    uint32_t* status;    // [kSortMaxPasses][max_tiles][256] look-back words
+    uint32_t* status;    // [passes][tiles][256] look-back words
     uint32_t max_tiles;
     size_t zero_bytes;   // bytes from hist through status
 };
@@ -65,9 +69,6 @@ void sort_reset(const SortScratch& s, cudaStream_t st);
 void sort_histogram(const uint32_t* keys, uint32_t n, int passes, const SortScratch& s,
                     cudaStream_t st);
 
-// Turns the histograms into exclusive digit offsets (in place).
-void sort_scan(int passes, const SortScratch& s, cudaStream_t st);
-
 // Runs the digit passes.  keys[0] holds the input keys and first_vals the
 // input values (NULL: the values are the input indices 0..n-1, generated in
 // the first pass); keys[1]/vals[1] and vals[0] are ping-pong buffers.  Returns
@@ -88,14 +89,36 @@ int sort_passes_run_dev(uint32_t* keys[2], uint32_t* vals[2], const uint32_t* fi
                         uint32_t n, const uint32_t* n_dev, uint32_t small_max, int passes,
                         const SortScratch& s, uint32_t* err, int force_timeout, cudaStream_t st);
 
+// Tiles of one pass over n keys (counted: of at most n, as in sort_passes_run_dev),
+// and the words from s.tile_ctr that `passes` such passes need cleared.
+uint32_t sort_tiles(uint32_t n, uint32_t small_max, bool counted);
+inline uint32_t sort_pass_words(uint32_t tiles, int passes) {
+    return 64u + (uint32_t)passes * tiles * 256u;
+}
+
+// A step's sort: keys in keys[0], values the indices 0..n-1.  The step's first
+// kernel clears sort_step_words(n, passes) words from s.tile_ctr and adds the
+// histograms to s.hist, which a kernel after the sort zeroes for the next step.
+// The plan holds sort_step_plan_keys(n) keys.
+inline uint32_t sort_step_plan_keys(uint32_t n) {
+    const uint32_t few = n < kSortStepSmall ? n : kSortStepSmall;
+    const uint32_t small = few * (uint32_t)(kSortTile / kSortTileSmall);
+    return n > small ? n : small;
+}
+inline uint32_t sort_step_words(uint32_t n, int passes) {
+    return sort_pass_words(sort_tiles(n, kSortStepSmall, false), passes);
+}
+int sort_step_run(uint32_t* keys[2], uint32_t* vals[2], uint32_t n, int passes,
+                  const SortScratch& s, uint32_t* err, int force_timeout, cudaStream_t st);
+
 // One digit pass p (bits 8p..8p+7) from explicit input to output buffers
 // (vals_in NULL: values are the input indices).  Needs the histograms of
-// sort_histogram + sort_scan in `s`.
+// sort_histogram in `s`.
 void sort_pass(const uint32_t* keys_in, const uint32_t* vals_in, uint32_t* keys_out,
                uint32_t* vals_out, uint32_t n, int p, const SortScratch& s, uint32_t* err,
                int force_timeout, cudaStream_t st);
 
-// Convenience: reset + histogram + scan + passes.
+// Convenience: reset + histogram + passes.
 int sort_pairs(uint32_t* keys[2], uint32_t* vals[2], uint32_t n, int key_bits,
                const SortScratch& s, uint32_t* err, int force_timeout, cudaStream_t st);
 

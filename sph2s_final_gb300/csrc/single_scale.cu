@@ -72,27 +72,31 @@ int enqueue_neighborhood(sph_solver* s) {
     near.list = s->blist;
     near.count = s->bcount;
     near.flag = s->bflag;
-    cudaMemsetAsync(s->bcount, 0, 4, st);
     if (!coherent || s->force_timeout) {
         const int passes = sort_passes(s->key_bits);
-        sort_reset(s->sort, st);
-        uint32_t hb = blocks_for(s->n);
-        if (hb > 152 * 8) hb = 152 * 8;
-        hash_hist_kernel<<<hb, 256, 0, st>>>(s->pos, s->n, s->P.g, passes, s->keys[0], s->sort.hist);
-        sort_scan(passes, s->sort, st);
-        out = sort_passes_run(s->keys, s->vals, nullptr, s->n, passes, s->sort, s->err, s->force_timeout, st);
+        const uint32_t hb = std::min(std::max(blocks_for(s->n), blocks_for(s->ncells, 1024)), 152u * 8u);
+        const StepClear clear = {s->cells, s->ncells, s->sort.tile_ctr, sort_step_words(s->n, passes),
+                                 s->bcount};
+        hash_hist_kernel<<<hb, 256, 0, st>>>(s->pos, s->n, s->P.g, passes, s->keys[0], s->sort.hist,
+                                             clear);
+        out = sort_step_run(s->keys, s->vals, s->n, passes, s->sort, s->err, s->force_timeout, st);
     } else {  // sort, reorder and cell table in one sequence
         coherent_sort_cells(s->co, s->pos, s->vel, s->P.g, s->cells, s->key_bits, s->keys[0],
                             s->keys[1], s->vals[1], s->spos, s->svel, s->err, s->force_timeout, st,
                             near);
         return out;
     }
-    cudaMemsetAsync(s->cells, 0xFF, sizeof(uint2) * s->ncells, st);
-    gather_cells_kernel<true><<<blocks_for(s->n), 256, 0, st>>>(
-        s->keys[out], s->vals[out], s->n, s->P.g, s->pos, s->vel, s->spos, s->svel, s->cells,
-        s->err, 0, s->co.kprev, near);
+    launch_after(gather_cells_kernel<true>, blocks_for(s->n), 256, st, s->keys[out], s->vals[out],
+                 s->n, s->P.g, s->pos, s->vel, s->spos, s->svel, s->cells, s->err, 0, s->co.kprev,
+                 near, s->sort.hist);
     return out;
 }
+
+// Below this many particles the density pass's blocks are set up while the pass
+// before it drains (launch_after: 262,144 particles 158.3 -> 156.9 us per step).
+// At 2,097,152 they then hold every SM before the boundary pass gets a block, and
+// the force pass waits for that one: 788 -> 792 us; 1,000,000: 420 either way.
+constexpr uint32_t kDensityAfterMost = 1u << 20;
 
 // The density pass, and beside it on the second branch (fork/join events,
 // captured into the step graph as a parallel branch) the boundary force sums
@@ -107,8 +111,14 @@ void enqueue_density(sph_solver* s, uint32_t* xall) {
                                                       s->P, s->bacc);
     cudaEventRecord(s->join, s->side);
     const auto kernel = xall ? density_kernel<true> : density_kernel<false>;
-    kernel<<<blocks_for(s->n, kDensityThreads), kDensityThreads, 0, s->stream>>>(
-        s->spos, s->cells, s->n, s->P, s->rho, s->aux, s->nbr, s->nbr_count, xall, s->xa, s->svel);
+    const uint32_t blocks = blocks_for(s->n, kDensityThreads);
+    if (s->n < kDensityAfterMost)
+        launch_after(kernel, blocks, kDensityThreads, s->stream, s->spos, s->cells, s->n, s->P,
+                     s->rho, s->aux, s->nbr, s->nbr_count, xall, s->xa, s->svel);
+    else
+        kernel<<<blocks, kDensityThreads, 0, s->stream>>>(s->spos, s->cells, s->n, s->P, s->rho,
+                                                          s->aux, s->nbr, s->nbr_count, xall,
+                                                          s->xa, s->svel);
 }
 
 void enqueue_force(sph_solver* s, float dt) {
@@ -229,8 +239,10 @@ int create_solver(const sph_config* config, const HostInit& init, uint32_t n_flu
     TRY(dalloc(&s->bcells, s->ncells));
     TRY(dalloc(&s->bpos, n_boundary));
     TRY(dalloc(&s->pos0, n_fluid));
-    TRY(check_cuda(cudaMalloc(&s->sort_mem, sort_scratch_bytes(nmax)), "sort scratch", __FILE__, __LINE__));
-    s->sort = sort_scratch_from(s->sort_mem, nmax);
+    const uint32_t plan = std::max(nmax, sort_step_plan_keys(n_fluid));
+    TRY(check_cuda(cudaMalloc(&s->sort_mem, sort_scratch_bytes(plan)), "sort scratch", __FILE__, __LINE__));
+    s->sort = sort_scratch_from(s->sort_mem, plan);
+    sort_reset(s->sort, s->stream);
     TRY(dalloc(&s->cells, s->ncells));  // read by the first coherent sort: no stale ranges
     TRY(check_cuda(cudaMemsetAsync(s->cells, 0xFF, sizeof(uint2) * s->ncells, s->stream), "memset", __FILE__, __LINE__));
     TRY(check_cuda(cudaMalloc(&s->co_mem, coherent_bytes(n_fluid)), "sort scratch", __FILE__, __LINE__));
@@ -299,11 +311,10 @@ int create_solver(const sph_config* config, const HostInit& init, uint32_t n_flu
                 boundary_hash_hist_kernel<<<blocks_for(n_boundary) > 1216 ? 1216 : blocks_for(n_boundary), 256, 0, s->stream>>>(
                     braw, n_boundary, s->P.g, qb, boundary_quantum(s->P.h), passes, s->keys[0],
                     s->sort.hist);
-                sort_scan(passes, s->sort, s->stream);
                 int o = sort_passes_run(s->keys, s->vals, nullptr, n_boundary, passes, s->sort, s->err, 0, s->stream);
                 gather_cells_kernel<false><<<blocks_for(n_boundary), 256, 0, s->stream>>>(
                     s->keys[o], s->vals[o], n_boundary, s->P.g, braw, nullptr, s->bpos, nullptr, s->bcells,
-                    s->err, qb);
+                    s->err, qb, nullptr, NearList{}, s->sort.hist);
                 e = cudaGetLastError();
                 if (e == cudaSuccess) e = cudaStreamSynchronize(s->stream);
             }

@@ -16,13 +16,16 @@
 
 namespace sph {
 
-// Morton key per particle, fused with the digit histograms of every sort pass.
+// Morton key per particle, fused with the digit histograms of every sort pass and
+// with what the step clears.
 static __global__ void __launch_bounds__(256) hash_hist_kernel(const float4* __restrict__ pos, uint32_t n,
                                                         GridParams g, int passes,
                                                         uint32_t* __restrict__ keys,
-                                                        uint32_t* __restrict__ hist) {
+                                                        uint32_t* __restrict__ hist,
+                                                        const StepClear clear) {
     __shared__ uint32_t sh[kSortMaxPasses][256];
     for (int i = threadIdx.x; i < kSortMaxPasses * 256; i += blockDim.x) (&sh[0][0])[i] = 0;
+    step_clear(clear);
     __syncthreads();
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         float4 p = pos[i];
@@ -64,7 +67,8 @@ static __global__ void __launch_bounds__(256) boundary_hash_hist_kernel(
 
 // Reorders the state by the sorted permutation and records cell ranges (keys
 // shifted right by key_shift first: the boundary presort's depth bits); with
-// kprev_out, also stores the sorted keys for the next coherent sort.
+// kprev_out, also stores the sorted keys for the next coherent sort; with hist,
+// zeroes the sort's histograms for the next step.
 // Every index read from the sort output is range-checked: if a bounded wait in
 // the sort gave up, its output is garbage, and this kernel then records an
 // error and stays in bounds instead of faulting.
@@ -74,8 +78,11 @@ __global__ void __launch_bounds__(256) gather_cells_kernel(
     GridParams g, const float4* __restrict__ pos_in, const float4* __restrict__ vel_in,
     float4* __restrict__ pos_out, float4* __restrict__ vel_out, uint2* __restrict__ cells,
     uint32_t* __restrict__ err, int key_shift = 0, uint32_t* __restrict__ kprev_out = nullptr,
-    NearList near = NearList{}) {
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    NearList near = NearList{}, uint32_t* __restrict__ hist = nullptr) {
+    grid_wait();
+    const uint32_t i = after_wait(blockIdx.x * blockDim.x + threadIdx.x);
+    if (hist && blockIdx.x == 0)
+        for (int k = threadIdx.x; k < kSortMaxPasses * 256; k += blockDim.x) hist[k] = 0;
     if (i >= n) return;
     if (kprev_out) kprev_out[i] = keys_sorted[i];  // the next step's coherent sort starts here
     uint32_t q = perm[i];

@@ -38,7 +38,6 @@ extern "C" int sph_sort_pairs(const uint32_t* keys_in, const uint32_t* vals_in, 
         uint32_t* vb = (passes & 1) ? tmp + n : vals_out;
         sort_reset(s, st);
         sort_histogram(keys_in, n, passes, s, st);
-        sort_scan(passes, s, st);
         const uint32_t* kin = keys_in;
         const uint32_t* vin = vals_in;
         for (int p = 0; p < passes; ++p) {

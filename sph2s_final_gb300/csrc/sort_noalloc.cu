@@ -129,7 +129,6 @@ extern "C" int sph_sort_pairs_noalloc(const uint32_t* keys_in, const uint32_t* v
     SPH_CUDA(cudaMemsetAsync(err, 0, 4, st));
     sort_reset(s, st);  // histograms, tile counters and look-back words start at zero
     sort_histogram(keys_in, n, passes, s, st);
-    sort_scan(passes, s, st);
     const uint32_t* kin = keys_in;
     const uint32_t* vin = vals_in;
     for (int p = 0; p < passes; ++p) {

@@ -231,6 +231,10 @@ TSOut outputs(Pop& p, float* acc, uint32_t* nbr_bnd, float* colour = nullptr) {
     return o;
 }
 
+int ts_sort_passes(const sph_solver2* s) {  // digits of (population bit, cell key)
+    return sort_passes(std::max(s->pop[0].key_bits, s->pop[1].key_bits) + 1);
+}
+
 // hash -> sort -> reorder + cell ranges of both populations (Solver.cu:1616-1680):
 // one stable sort of (population bit, cell key) pairs gives each population the
 // order of its own sort with half the sort launches.  ts_front has cleared the
@@ -241,13 +245,12 @@ void ts_neighborhoods(sph_solver2* s) {
     const uint32_t n = L.n + H.n;
     if (n == 0) return;
     const int pop_bit = std::max(L.key_bits, H.key_bits);
-    const int passes = sort_passes(pop_bit + 1);
+    const int passes = ts_sort_passes(s);
     uint32_t hb = blocks_for(n);
     if (hb > 1216) hb = 1216;
     ts_hash_hist_kernel<<<hb, 256, 0, st>>>(L.pos, L.n, s->P.g[0], H.pos, H.n, s->P.g[1], pop_bit,
                                             passes, s->keys[0], s->sort.hist);
-    sort_scan(passes, s->sort, st);
-    const int o = sort_passes_run(s->keys, s->vals, nullptr, n, passes, s->sort, s->err, 0, st);
+    const int o = sort_step_run(s->keys, s->vals, n, passes, s->sort, s->err, 0, st);
     const uint32_t mask = (1u << pop_bit) - 1u;
     if (H.n)
         ts_gather_kernel<true><<<blocks_for(H.n), 256, 0, st>>>(
@@ -271,7 +274,9 @@ void ts_front(sph_solver2* s, float dt, bool debug, int dbg_pop, uint32_t* dnb_s
         ClearBatch c;
         c.add(s->pop[1].cells, sizeof(uint2) * s->pop[1].ncells, 0xFFFFFFFFu);
         c.add(s->pop[0].cells, sizeof(uint2) * s->pop[0].ncells, 0xFFFFFFFFu);
-        c.add(s->sort.hist, s->sort.zero_bytes, 0u);
+        c.add(s->sort.hist, 4 * kSortMaxPasses * 256, 0u);
+        c.add(s->sort.tile_ctr,
+              4 * (size_t)sort_step_words(s->pop[0].n + s->pop[1].n, ts_sort_passes(s)), 0u);
         c.add(s->occ, s->occ_bytes, 0u);
         c.add(s->near_count, 4, 0u);
         c.add(s->ctl + kCtlFadedL, 8, 0u);
@@ -603,9 +608,10 @@ int create_solver2(const sph_config2* config, const TSParams& P, uint64_t capL, 
         TRY(dalloc(&s->keys[b], nmax, s->owned));
         TRY(dalloc(&s->vals[b], nmax, s->owned));
     }
-    TRY(check_cuda(cudaMalloc(&s->sort_mem, sort_scratch_bytes(nmax)), "sort scratch", __FILE__, __LINE__));
+    const uint32_t plan = std::max(nmax, sort_step_plan_keys((uint32_t)(capL + capH)));
+    TRY(check_cuda(cudaMalloc(&s->sort_mem, sort_scratch_bytes(plan)), "sort scratch", __FILE__, __LINE__));
     s->owned.push_back(s->sort_mem);
-    s->sort = sort_scratch_from(s->sort_mem, nmax);
+    s->sort = sort_scratch_from(s->sort_mem, plan);
     TRY(dalloc(&s->scan_scratch,
                scan_scratch_words((uint32_t)capH) + 2 * scan_scratch_words((uint32_t)capL) +
                    scan_scratch_words(s->cap_groups),
@@ -661,7 +667,6 @@ int create_solver2(const sph_config2* config, const TSParams& P, uint64_t capL, 
             boundary_hash_hist_kernel<<<hbk, 256, 0, s->stream>>>(
                 braw, n_boundary, s->P.g[0], qb, boundary_quantum(s->P.h[0]), passes, s->keys[0],
                 s->sort.hist);
-            sort_scan(passes, s->sort, s->stream);
             const int o = sort_passes_run(s->keys, s->vals, nullptr, n_boundary, passes, s->sort,
                                           s->err, 0, s->stream);
             gather_cells_kernel<false><<<blocks_for(n_boundary), 256, 0, s->stream>>>(
