@@ -111,6 +111,13 @@ void enqueue_density(sph_solver* s, uint32_t* xall) {
                                                       s->P, s->bacc);
     cudaEventRecord(s->join, s->side);
     const auto kernel = xall ? density_kernel<true> : density_kernel<false>;
+    if (s->n < kDensitySplitMost) {
+        launch_after(xall ? density_split_kernel<true> : density_split_kernel<false>,
+                     blocks_for(s->n, kSplitWarps * kSplitPer), 32 * kSplitWarps, s->stream, s->spos,
+                     s->cells, s->n, s->P, s->rho, s->aux, s->nbr, s->nbr_count, xall, s->xa,
+                     s->svel);
+        return;
+    }
     const uint32_t blocks = blocks_for(s->n, kDensityThreads);
     if (s->n < kDensityAfterMost)
         launch_after(kernel, blocks, kDensityThreads, s->stream, s->spos, s->cells, s->n, s->P,
