@@ -27,10 +27,11 @@ constexpr int kSortTile = kSortThreads * kSortItems;  // 4096 keys
 constexpr int kSortItemsSmall = 2;
 constexpr int kSortTileSmall = kSortThreads * kSortItemsSmall;
 constexpr int kSortMaxPasses = 4;
-// A step's sort of at most this many keys uses the small tiles: 4,096 keys are
-// then 8 tiles instead of one (58 -> 56 us per step); at 32,768 both take the
-// same, and 94,608 in 185 small tiles look back too far (89 -> 94 us per step).
-constexpr uint32_t kSortStepSmall = 1u << 14;
+// A step's sort of at most this many keys uses the small tiles: more of the chip
+// sorts (us per step, large tiles and small: 4,096 keys 58 and 56, 32,768 65.8 and
+// 64.2, 64,000 86.5 and 86.1).  Beyond, the walk back over them costs more (110,592:
+// 92.6 and 93.8).
+constexpr uint32_t kSortStepSmall = 1u << 16;
 
 // Device scratch of one sort plan.  Everything that must start at zero lives
 // in one contiguous block so a single memset resets it.
