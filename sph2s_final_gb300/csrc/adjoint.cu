@@ -38,6 +38,9 @@ struct Rollout {
     std::vector<uint4*> nbr;
     std::vector<uint32_t*> cnt;
     std::vector<uint2*> cells;
+    std::vector<uint32_t*> nlist;   // near-boundary particles, their number and flags
+    std::vector<uint32_t*> ncount;
+    std::vector<uint8_t*> nflag;
     float4 *gx = nullptr, *gv = nullptr, *gx2 = nullptr, *gv2 = nullptr, *lam = nullptr;
     float4* gb = nullptr;  // the boundary force's part of gx2
     float4* gxT = nullptr;
@@ -93,11 +96,16 @@ int alloc_rollout(sph_solver* s, int T, int K, Rollout** out) {
     r->nbr.resize(K);
     r->cnt.resize(K);
     r->cells.resize(K);
+    r->nlist.resize(K);
+    r->ncount.resize(K);
+    r->nflag.resize(K);
     for (int k = 0; k < K && rc == SPH_OK; ++k) {
         if ((rc = ralloc(r, &r->perm[k], n)) || (rc = ralloc(r, &r->xh[k], n)) ||
             (rc = ralloc(r, &r->vh[k], n)) || (rc = ralloc(r, &r->rho[k], n)) ||
             (rc = ralloc(r, &r->aux[k], n)) || (rc = ralloc(r, &r->nbr[k], (size_t)n * (kMaxNbr / 4))) ||
-            (rc = ralloc(r, &r->cnt[k], n)) || (rc = ralloc(r, &r->cells[k], s->ncells)))
+            (rc = ralloc(r, &r->cnt[k], n)) || (rc = ralloc(r, &r->cells[k], s->ncells)) ||
+            (rc = ralloc(r, &r->nlist[k], n)) || (rc = ralloc(r, &r->ncount[k], 1)) ||
+            (rc = ralloc(r, &r->nflag[k], n)))
             break;
     }
     const uint32_t blocks = blocks_for(n);
@@ -128,6 +136,9 @@ int record_segment(sph_solver* s, int len) {
     uint4* nbr0 = s->nbr;
     uint32_t* cnt0 = s->nbr_count;
     uint2* cells0 = s->cells;
+    uint32_t* blist0 = s->blist;
+    uint32_t* bcount0 = s->bcount;
+    uint8_t* bflag0 = s->bflag;
     for (int k = 0; k < len; ++k) {
         s->spos = r->xh[k];
         s->svel = r->vh[k];
@@ -136,6 +147,9 @@ int record_segment(sph_solver* s, int len) {
         s->aux = r->aux[k];
         s->nbr = r->nbr[k];
         s->nbr_count = r->cnt[k];
+        s->blist = r->nlist[k];
+        s->bcount = r->ncount[k];
+        s->bflag = r->nflag[k];
         const int out = enqueue_neighborhood(s);
         cudaMemcpyAsync(r->perm[k], s->vals[out], 4 * (size_t)s->n, cudaMemcpyDeviceToDevice,
                         s->stream);
@@ -149,6 +163,9 @@ int record_segment(sph_solver* s, int len) {
     s->aux = aux0;
     s->nbr = nbr0;
     s->nbr_count = cnt0;
+    s->blist = blist0;
+    s->bcount = bcount0;
+    s->bflag = bflag0;
     SPH_CUDA(cudaGetLastError());
     return SPH_OK;
 }
@@ -336,9 +353,9 @@ int sph_rollout_backward(sph_solver* s, float* grad_v0, float* grad_x0, double* 
             // the boundary force's adjoint beside that of the pair forces
             SPH_CUDA(cudaEventRecord(s->fork, st));
             SPH_CUDA(cudaStreamWaitEvent(s->side, s->fork, 0));
-            adj_boundary_kernel<<<blocks_for(n, 256 / 32 * kBndLanes), 256, 0, s->side>>>(
-                r->xh[k], r->lam, s->bpos, s->bcells, s->bnear, s->bstart, s->bcand, n, s->nb, s->P,
-                r->gb);
+            adj_boundary_kernel<<<std::min(blocks_for(n, 256 / kBndLanes), 4u * (uint32_t)std::max(s->sms, 1)), 256, 0,
+                                  s->side>>>(r->nlist[k], r->ncount[k], r->xh[k], r->lam, s->bpos,
+                                             s->bcells, s->bstart, s->bcand, n, s->nb, s->P, r->gb);
             SPH_CUDA(cudaEventRecord(s->join, s->side));
             adj_force_kernel<<<blocks, 256, 0, st>>>(
                 r->xh[k], r->vh[k], r->rho[k], r->nbr[k], r->cnt[k], r->cells[k], n, s->P, r->mu,
@@ -346,7 +363,7 @@ int sph_rollout_backward(sph_solver* s, float* grad_v0, float* grad_x0, double* 
             adj_sum_kernel<<<1, 32, 0, st>>>(r->gmu_part, blocks, r->gmu_acc);
             SPH_CUDA(cudaStreamWaitEvent(st, s->join, 0));
             adj_density_kernel<<<blocks, 256, 0, st>>>(r->xh[k], r->nbr[k], r->cnt[k], r->cells[k],
-                                                       n, s->P, r->grho, r->gb, r->gx2);
+                                                       n, s->P, r->grho, r->gb, r->nflag[k], r->gx2);
             adj_unpermute_kernel<<<blocks, 256, 0, st>>>(r->perm[k], n, r->gx2, r->gv2, r->gx, r->gv);
         }
         SPH_CUDA(cudaGetLastError());

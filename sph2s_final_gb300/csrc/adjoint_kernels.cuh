@@ -154,7 +154,7 @@ struct AdjForcePair {
 };
 
 // Adjoint of force + integrate for particle i of the step's sorted order,
-// without the boundary force (adj_boundary_warp); returns particle i's share of
+// without the boundary force (adj_boundary_lanes); returns particle i's share of
 // d L / d mu.  cells are the particle's own grid's (the batched rollout passes
 // per-scene tables, P and mu).
 __device__ __forceinline__ float adj_force_one(
@@ -189,94 +189,88 @@ __device__ __forceinline__ float adj_force_one(
 }
 
 // Adjoint of the boundary force b_i = sum_k beta(r) x_ik, beta = Bc shape(2r/h) /
-// r^2, of one warp's kBndLanes particles (lane l < kBndLanes holds the l-th's
-// index i, below `end`): gb[i] = its part of gx_i, 0 away from the boundary.
-// It needs the positions and lam alone and runs beside adj_force; inside it, one
+// r^2, of the step's listed near-boundary particles: gb[i] = its part of gx_i.  It
+// needs the positions and lam alone and runs beside adj_force; inside it, one
 // lane's ~70 candidates in a row held the warp.  Eight lanes take a particle,
-// each every eighth candidate, their sums added in a fixed order: 16 us at 65,536
-// particles, most of it under adj_force's 20.
+// each every eighth candidate, their sums added in a fixed order (65,536
+// particles: 15 us, under adj_force's 20).  The list and the flags (adj_density) are
+// the forward step's own, kept in the tape: looking the particles up in each warp
+// left most of its rounds part empty (eight scenes: 52 us, now 32).
 constexpr uint32_t kBndLanes = 8;
 
-__device__ __forceinline__ void adj_boundary_warp(
-    uint32_t i, uint32_t end, const float4* __restrict__ pos, const float4* __restrict__ lam,
+// One particle p per eight lanes (work: whether these have one).
+__device__ __forceinline__ void adj_boundary_lanes(
+    bool work, uint32_t p, const float4* __restrict__ pos, const float4* __restrict__ lam,
     const float4* __restrict__ bpos, const uint2* __restrict__ bcells,
-    const uint8_t* __restrict__ bnear, const uint32_t* __restrict__ bstart,
-    const uint32_t* __restrict__ bcand, uint32_t nb, const SimParams& P,
-    float4* __restrict__ gb) {
+    const uint32_t* __restrict__ bstart, const uint32_t* __restrict__ bcand, uint32_t nb,
+    const SimParams& P, float4* __restrict__ gb) {
     constexpr uint32_t kAll = 0xFFFFFFFFu;
-    const uint32_t lane = threadIdx.x & 31u, sub = lane & (kBndLanes - 1u);
-    bool near = false;
-    if (lane < kBndLanes && i < end) {
-        near = __ldg(&bnear[home_cell(P.g, pos[i])]) != 0;
-        if (!near) gb[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-    }
-    uint32_t m = __ballot_sync(kAll, near);
-    while (m) {
-        uint32_t mine = m;
-        for (uint32_t g = 0; g < lane / kBndLanes; ++g) mine &= mine - 1u;  // the earlier groups'
-        const bool work = mine != 0u;
-        const uint32_t p = __shfl_sync(kAll, i, work ? __ffs((int)mine) - 1 : 0);
-        float bx = 0.f, by = 0.f, bz = 0.f;
-        if (work) {
-            const float4 xi = pos[p], li = lam[p];
-            auto pair = [&](const float4& xk) {
-                float dx, dy, dz;
-                const float r2 = dist2(xi.x, xi.y, xi.z, xk.x, xk.y, xk.z, dx, dy, dz);
-                if (!(r2 < P.T)) return;
-                const float rs = rsqrtf(r2);
-                const float q = r2 * rs * P.two_over_h;
-                float sh, shp;
-                if (q < 2.0f / 3.0f) {
-                    sh = 2.0f / 3.0f;
-                    shp = 0.0f;
-                } else if (q < 1.0f) {
-                    sh = q * (2.0f - 1.5f * q);
-                    shp = 2.0f - 3.0f * q;
-                } else {
-                    const float t2 = 2.0f - q;
-                    sh = 0.5f * t2 * t2;
-                    shp = -t2;
-                }
-                const float beta = P.bnd_coef * sh * rs * rs;
-                const float betap =
-                    P.bnd_coef * (shp * P.two_over_h * rs * rs - 2.0f * sh * rs * rs * rs);
-                const float rad = betap * rs * (li.x * dx + li.y * dy + li.z * dz);
-                bx += beta * li.x + rad * dx;
-                by += beta * li.y + rad * dy;
-                bz += beta * li.z + rad * dz;
-            };
-            const int hx = cell_coord(xi.x, P.g.ox, P.g.spacing, P.g.dx);
-            const int hy = cell_coord(xi.y, P.g.oy, P.g.spacing, P.g.dy);
-            const int hz = cell_coord(xi.z, P.g.oz, P.g.spacing, P.g.dz);
-            if (boundary_listed(xi, hx, hy, hz, P)) {
-                const uint32_t home = linear_cell(P.g, hx, hy, hz);
-                const uint32_t e = __ldg(&bstart[home + 1]);
-                for (uint32_t k = __ldg(&bstart[home]) + sub; k < e; k += kBndLanes)
-                    pair(__ldg(&bpos[min(__ldg(&bcand[k]), nb - 1)]));
-            } else if (sub == 0) {
-                scan_boundary(xi, bpos, bcells, nb, P, pair);
+    const uint32_t sub = threadIdx.x & (kBndLanes - 1u);
+    float bx = 0.f, by = 0.f, bz = 0.f;
+    if (work) {
+        const float4 xi = pos[p], li = lam[p];
+        auto pair = [&](const float4& xk) {
+            float dx, dy, dz;
+            const float r2 = dist2(xi.x, xi.y, xi.z, xk.x, xk.y, xk.z, dx, dy, dz);
+            if (!(r2 < P.T)) return;
+            const float rs = rsqrtf(r2);
+            const float q = r2 * rs * P.two_over_h;
+            float sh, shp;
+            if (q < 2.0f / 3.0f) {
+                sh = 2.0f / 3.0f;
+                shp = 0.0f;
+            } else if (q < 1.0f) {
+                sh = q * (2.0f - 1.5f * q);
+                shp = 2.0f - 3.0f * q;
+            } else {
+                const float t2 = 2.0f - q;
+                sh = 0.5f * t2 * t2;
+                shp = -t2;
             }
+            const float beta = P.bnd_coef * sh * rs * rs;
+            const float betap =
+                P.bnd_coef * (shp * P.two_over_h * rs * rs - 2.0f * sh * rs * rs * rs);
+            const float rad = betap * rs * (li.x * dx + li.y * dy + li.z * dz);
+            bx += beta * li.x + rad * dx;
+            by += beta * li.y + rad * dy;
+            bz += beta * li.z + rad * dz;
+        };
+        const int hx = cell_coord(xi.x, P.g.ox, P.g.spacing, P.g.dx);
+        const int hy = cell_coord(xi.y, P.g.oy, P.g.spacing, P.g.dy);
+        const int hz = cell_coord(xi.z, P.g.oz, P.g.spacing, P.g.dz);
+        if (boundary_listed(xi, hx, hy, hz, P)) {
+            const uint32_t home = linear_cell(P.g, hx, hy, hz);
+            const uint32_t e = __ldg(&bstart[home + 1]);
+            for (uint32_t k = __ldg(&bstart[home]) + sub; k < e; k += kBndLanes)
+                pair(__ldg(&bpos[min(__ldg(&bcand[k]), nb - 1)]));
+        } else if (sub == 0) {
+            scan_boundary(xi, bpos, bcells, nb, P, pair);
         }
-#pragma unroll
-        for (uint32_t o = kBndLanes / 2; o; o >>= 1) {
-            bx += __shfl_xor_sync(kAll, bx, o);
-            by += __shfl_xor_sync(kAll, by, o);
-            bz += __shfl_xor_sync(kAll, bz, o);
-        }
-        if (work && sub == 0) gb[p] = make_float4(bx, by, bz, 0.f);
-        for (uint32_t g = 0; g < 32 / kBndLanes; ++g) m &= m - 1u;
     }
+#pragma unroll
+    for (uint32_t o = kBndLanes / 2; o; o >>= 1) {
+        bx += __shfl_xor_sync(kAll, bx, o);
+        by += __shfl_xor_sync(kAll, by, o);
+        bz += __shfl_xor_sync(kAll, bz, o);
+    }
+    if (work && sub == 0) gb[p] = make_float4(bx, by, bz, 0.f);
 }
 
 static __global__ void __launch_bounds__(256) adj_boundary_kernel(
+    const uint32_t* __restrict__ list, const uint32_t* __restrict__ count,
     const float4* __restrict__ pos, const float4* __restrict__ lam,
     const float4* __restrict__ bpos, const uint2* __restrict__ bcells,
-    const uint8_t* __restrict__ bnear, const uint32_t* __restrict__ bstart,
-    const uint32_t* __restrict__ bcand, uint32_t n, uint32_t nb,
-    const __grid_constant__ SimParams P, float4* __restrict__ gb) {
+    const uint32_t* __restrict__ bstart, const uint32_t* __restrict__ bcand, uint32_t n,
+    uint32_t nb, const __grid_constant__ SimParams P, float4* __restrict__ gb) {
+    constexpr uint32_t kPer = 32 / kBndLanes;  // particles of a warp
+    const uint32_t cnt = min(*count, n), warps = gridDim.x * (blockDim.x >> 5);
     const uint32_t w = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    adj_boundary_warp(w * kBndLanes + (threadIdx.x & 31u), n, pos, lam, bpos, bcells, bnear, bstart,
-                      bcand, nb, P, gb);
+    for (uint32_t t = w * kPer; t < cnt; t += warps * kPer) {
+        const uint32_t k = t + (threadIdx.x & 31u) / kBndLanes;
+        const bool work = k < cnt;
+        adj_boundary_lanes(work, work ? min(list[k], n - 1) : 0u, pos, lam, bpos, bcells, bstart,
+                           bcand, nb, P, gb);
+    }
 }
 
 // Block sum of one value per thread in a fixed order (warp shuffles, then the
@@ -324,14 +318,15 @@ struct AdjDensityPair {
     }
 };
 
-// Density adjoint, and the boundary force's part (gb, adj_boundary_warp):
-// gx_i += gb_i - 6 m C6 sum_j (h^2 - r^2)^2 (grho_i + grho_j) x_ij.
+// Density adjoint, and the boundary force's part (gb, adj_boundary_lanes) where
+// near[i]: gx_i += gb_i - 6 m C6 sum_j (h^2 - r^2)^2 (grho_i + grho_j) x_ij.
 __device__ __forceinline__ void adj_density_one(uint32_t i, const float4* __restrict__ pos,
                                                 const uint4* __restrict__ nbr4,
                                                 const uint32_t* __restrict__ nbr_count,
                                                 const uint2* __restrict__ cells, uint32_t n,
                                                 const SimParams& P, const float* __restrict__ grho,
                                                 const float4* __restrict__ gb,
+                                                const uint8_t* __restrict__ near,
                                                 float4* __restrict__ gx) {
     const float4 xi = pos[i];
     AdjDensityPair A;
@@ -342,10 +337,12 @@ __device__ __forceinline__ void adj_density_one(uint32_t i, const float4* __rest
     visit_force_neighbors<4>(i, xi, pos, nbr4, nbr_count, cells, n, P,
                              [&](uint32_t j) { return __ldg(&grho[j]); }, A);
     float4 g = gx[i];
-    const float4 b = gb[i];
-    g.x += b.x;
-    g.y += b.y;
-    g.z += b.z;
+    if (near[i]) {
+        const float4 b = gb[i];
+        g.x += b.x;
+        g.y += b.y;
+        g.z += b.z;
+    }
     g.x += A.gx;
     g.y += A.gy;
     g.z += A.gz;
@@ -356,10 +353,10 @@ static __global__ void __launch_bounds__(256) adj_density_kernel(
     const float4* __restrict__ pos, const uint4* __restrict__ nbr4,
     const uint32_t* __restrict__ nbr_count, const uint2* __restrict__ cells, uint32_t n,
     const __grid_constant__ SimParams P, const float* __restrict__ grho,
-    const float4* __restrict__ gb, float4* __restrict__ gx) {
+    const float4* __restrict__ gb, const uint8_t* __restrict__ near, float4* __restrict__ gx) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    adj_density_one(i, pos, nbr4, nbr_count, cells, n, P, grho, gb, gx);
+    adj_density_one(i, pos, nbr4, nbr_count, cells, n, P, grho, gb, near, gx);
 }
 
 // Scatter from the step's sorted order back to the order before the sort:

@@ -118,7 +118,12 @@ void enqueue_force(sph_batch* b, float dt) {
 int enqueue_neighborhood(sph_batch* b) {
     cudaStream_t st = b->stream;
     int o = 1;
-    StepClear clear = {b->cells, b->NC, nullptr, 0u, nullptr};
+    StepClear clear = {b->cells, b->NC, nullptr, 0u, b->bcount};
+    NearList near;  // the near-boundary particles, for the boundary and force passes
+    near.bnear = b->bnear;
+    near.scene_list = b->blist;
+    near.count = b->bcount;
+    near.flag = b->bflag;
     if (b->coherent) {
         b_hash_hist_kernel<256><<<pgrid(b, b->ntiles[1]), 256, 0, st>>>(
             b->tiles[1], b->ntiles[1], b->recs, b->pos, b->shift, 0, b->keys[0], b->sort.hist,
@@ -136,7 +141,7 @@ int enqueue_neighborhood(sph_batch* b) {
     launch_after(b_gather_cells_kernel<256, true>, pgrid(b, b->ntiles[1]), 256, st, b->tiles[1],
                  b->ntiles[1], b->recs, b->keys[o], b->vals[o], b->N, b->shift, false, b->pos,
                  b->vel, b->spos, b->svel, b->cells, b->err, 0,
-                 b->coherent ? b->co.kprev : nullptr, b->bnear, b->bflag, b->sort.hist);
+                 b->coherent ? b->co.kprev : nullptr, near, b->sort.hist);
     return o;
 }
 
@@ -343,7 +348,7 @@ int sphb_create(const sph_scene_desc* scenes, uint32_t num_scenes, sph_batch** o
                                           b->err, 0, b->stream);
             b_gather_cells_kernel<256, false><<<pgrid(b, b->nbtiles), 256, 0, b->stream>>>(
                 b->btiles, b->nbtiles, b->recs, b->keys[o], b->vals[o], b->NB, b->shift, true, braw,
-                nullptr, b->bpos, nullptr, b->bcells, b->err, qb, nullptr, nullptr, nullptr,
+                nullptr, b->bpos, nullptr, b->bcells, b->err, qb, nullptr, NearList{},
                 b->sort.hist);
             TRY(check_cuda(cudaStreamSynchronize(b->stream), "boundary presort", __FILE__, __LINE__));
             cudaFree(braw);
@@ -365,7 +370,7 @@ int sphb_create(const sph_scene_desc* scenes, uint32_t num_scenes, sph_batch** o
         for (uint32_t s = 0; s < num_scenes; ++s) {
             const SceneRec& R = b->recs_h[s];
             const uint32_t nc = sph_grid_num_cells(&scenes[s].config.grid);
-            lims[s] = R.P.h * 1.01f + 4.0f * R.P.bmargin;
+            lims[s] = R.P.h * kBoundaryLim + 4.0f * R.P.bmargin;
             if (!nc) continue;
             boundary_cand_kernel<false><<<(nc + 255) / 256, 256, 0, b->stream>>>(
                 b->bcells + R.c_off, b->bpos, b->bnear + R.c_off, R.P.g, b->NB, lims[s],

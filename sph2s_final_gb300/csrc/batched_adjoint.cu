@@ -38,6 +38,9 @@ struct BRollout {
     std::vector<uint4*> nbr;
     std::vector<uint32_t*> cnt;
     std::vector<uint2*> cells;
+    std::vector<uint2*> nlist;   // near-boundary particles, their number and flags
+    std::vector<uint32_t*> ncount;
+    std::vector<uint8_t*> nflag;
     float4 *gx = nullptr, *gv = nullptr, *gx2 = nullptr, *gv2 = nullptr, *lam = nullptr;
     float4* gb = nullptr;  // the boundary force's part of gx2
     float4* gxT = nullptr;
@@ -91,19 +94,21 @@ static __global__ void __launch_bounds__(kTile) b_adj_force_kernel(
 }
 
 static __global__ void __launch_bounds__(kTile) b_adj_boundary_kernel(
-    const uint2* __restrict__ tiles, uint32_t num_tiles, const SceneRec* __restrict__ recs,
-    const float4* __restrict__ pos, const float4* __restrict__ lam,
-    const float4* __restrict__ bpos, const uint2* __restrict__ bcells,
-    const uint8_t* __restrict__ bnear, const uint32_t* __restrict__ bstart,
+    const uint2* __restrict__ list, const uint32_t* __restrict__ count, uint32_t n,
+    uint32_t scenes, const SceneRec* __restrict__ recs, const float4* __restrict__ pos,
+    const float4* __restrict__ lam, const float4* __restrict__ bpos,
+    const uint2* __restrict__ bcells, const uint32_t* __restrict__ bstart,
     const uint32_t* __restrict__ bcand, uint32_t nb, float4* __restrict__ gb) {
-    for (uint32_t t = blockIdx.x; t < num_tiles; t += gridDim.x) {
-        const uint2 tile = tiles[t];
-        const SceneRec& R = recs[tile.x];
-        const uint32_t end = min(tile.y + (uint32_t)kTile, R.p_off + R.p_n);
-        const SimParams P = R.P;
-        for (uint32_t k = tile.y + (threadIdx.x >> 5) * kBndLanes; k < end; k += kTile / 32 * kBndLanes)
-            adj_boundary_warp(k + (threadIdx.x & 31u), end, pos, lam, bpos, bcells + R.c_off,
-                              bnear + R.c_off, bstart + R.c_off, bcand, nb, P, gb);
+    constexpr uint32_t kPer = 32 / kBndLanes;  // particles of a warp
+    const uint32_t cnt = min(*count, n), warps = gridDim.x * (blockDim.x >> 5);
+    const uint32_t w = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    for (uint32_t t = w * kPer; t < cnt; t += warps * kPer) {
+        const uint32_t k = t + (threadIdx.x & 31u) / kBndLanes;
+        const bool work = k < cnt;
+        const uint2 e = work ? list[k] : make_uint2(0u, 0u);
+        const SceneRec& R = recs[min(e.y, scenes - 1)];
+        adj_boundary_lanes(work, min(e.x, n - 1), pos, lam, bpos, bcells + R.c_off,
+                           bstart + R.c_off, bcand, nb, R.P, gb);
     }
 }
 
@@ -111,14 +116,14 @@ static __global__ void __launch_bounds__(kTile) b_adj_density_kernel(
     const uint2* __restrict__ tiles, uint32_t num_tiles, const SceneRec* __restrict__ recs,
     const float4* __restrict__ pos, const uint4* __restrict__ nbr4, const uint32_t* __restrict__ cnt,
     const uint2* __restrict__ cells, uint32_t n, const float* __restrict__ grho,
-    const float4* __restrict__ gb, float4* __restrict__ gx) {
+    const float4* __restrict__ gb, const uint8_t* __restrict__ near, float4* __restrict__ gx) {
     for (uint32_t t = blockIdx.x; t < num_tiles; t += gridDim.x) {
         const uint2 tile = tiles[t];
         const SceneRec& R = recs[tile.x];
         const uint32_t i = tile.y + threadIdx.x;
         if (i >= R.p_off + R.p_n) continue;
         const SimParams P = R.P;
-        adj_density_one(i, pos, nbr4, cnt, cells + R.c_off, n, P, grho, gb, gx);
+        adj_density_one(i, pos, nbr4, cnt, cells + R.c_off, n, P, grho, gb, near, gx);
     }
 }
 
@@ -200,12 +205,17 @@ int alloc_brollout(sph_batch* b, int T, int K, BRollout** out) {
     r->nbr.resize(K);
     r->cnt.resize(K);
     r->cells.resize(K);
+    r->nlist.resize(K);
+    r->ncount.resize(K);
+    r->nflag.resize(K);
     for (int k = 0; k < K && rc == SPH_OK; ++k) {
         if ((rc = ralloc(r, &r->perm[k], N)) || (rc = ralloc(r, &r->xh[k], N)) ||
             (rc = ralloc(r, &r->vh[k], N)) || (rc = ralloc(r, &r->rho[k], N)) ||
             (rc = ralloc(r, &r->aux[k], N)) ||
             (rc = ralloc(r, &r->nbr[k], (size_t)N * (kMaxNbr / 4))) ||
-            (rc = ralloc(r, &r->cnt[k], N)) || (rc = ralloc(r, &r->cells[k], b->NC)))
+            (rc = ralloc(r, &r->cnt[k], N)) || (rc = ralloc(r, &r->cells[k], b->NC)) ||
+            (rc = ralloc(r, &r->nlist[k], N)) || (rc = ralloc(r, &r->ncount[k], 1)) ||
+            (rc = ralloc(r, &r->nflag[k], N)))
             break;
     }
     if (rc == SPH_OK &&
@@ -242,6 +252,9 @@ int record_segment(sph_batch* b, int len) {
     uint4* nbr0 = b->nbr;
     uint32_t* cnt0 = b->nbr_count;
     uint2* cells0 = b->cells;
+    uint2* blist0 = b->blist;
+    uint32_t* bcount0 = b->bcount;
+    uint8_t* bflag0 = b->bflag;
     for (int k = 0; k < len; ++k) {
         b->spos = r->xh[k];
         b->svel = r->vh[k];
@@ -250,6 +263,9 @@ int record_segment(sph_batch* b, int len) {
         b->aux = r->aux[k];
         b->nbr = r->nbr[k];
         b->nbr_count = r->cnt[k];
+        b->blist = r->nlist[k];
+        b->bcount = r->ncount[k];
+        b->bflag = r->nflag[k];
         const int out = enqueue_neighborhood(b);
         cudaMemcpyAsync(r->perm[k], b->vals[out], 4 * (size_t)b->N, cudaMemcpyDeviceToDevice,
                         b->stream);
@@ -263,6 +279,9 @@ int record_segment(sph_batch* b, int len) {
     b->aux = aux0;
     b->nbr = nbr0;
     b->nbr_count = cnt0;
+    b->blist = blist0;
+    b->bcount = bcount0;
+    b->bflag = bflag0;
     SPH_CUDA(cudaGetLastError());
     return SPH_OK;
 }
@@ -459,9 +478,11 @@ int sphb_rollout_backward(sph_batch* b, float* grad_v0, float* grad_x0, double* 
             // the boundary force's adjoint beside that of the pair forces
             SPH_CUDA(cudaEventRecord(b->fork, st));
             SPH_CUDA(cudaStreamWaitEvent(b->side, b->fork, 0));
-            b_adj_boundary_kernel<<<grid, kTile, 0, b->side>>>(
-                b->tiles[1], nt, b->recs, r->xh[k], r->lam, b->bpos, b->bcells, b->bnear, b->bstart,
-                b->bcand, b->NB, r->gb);
+            b_adj_boundary_kernel<<<std::min((N + kTile / kBndLanes - 1) / (kTile / kBndLanes),
+                                             4u * (uint32_t)std::max(b->sms, 1)),
+                                    kTile, 0, b->side>>>(
+                r->nlist[k], r->ncount[k], N, b->S, b->recs, r->xh[k], r->lam, b->bpos, b->bcells,
+                b->bstart, b->bcand, b->NB, r->gb);
             SPH_CUDA(cudaEventRecord(b->join, b->side));
             b_adj_force_kernel<<<grid, kTile, 0, st>>>(
                 b->tiles[1], nt, b->recs, r->mu, r->xh[k], r->vh[k], r->rho[k], r->nbr[k],
@@ -472,7 +493,7 @@ int sphb_rollout_backward(sph_batch* b, float* grad_v0, float* grad_x0, double* 
             SPH_CUDA(cudaStreamWaitEvent(st, b->join, 0));
             b_adj_density_kernel<<<grid, kTile, 0, st>>>(b->tiles[1], nt, b->recs, r->xh[k],
                                                          r->nbr[k], r->cnt[k], r->cells[k], N,
-                                                         r->grho, r->gb, r->gx2);
+                                                         r->grho, r->gb, r->nflag[k], r->gx2);
             adj_unpermute_kernel<<<blocks, kTile, 0, st>>>(r->perm[k], N, r->gx2, r->gv2, r->gx, r->gv);
         }
         SPH_CUDA(cudaGetLastError());

@@ -92,8 +92,9 @@ __global__ void __launch_bounds__(BS) b_boundary_hash_hist_kernel(
 
 // Reorder + per-scene cell ranges; indices stored in the tables are global.
 // Keys are shifted right by key_shift first (the boundary presort's depth bits).
-// With bflag, also bflag[i] = bnear of particle i's cell (1 if boundary
-// particles lie within its stencil reach), for the boundary and force passes.
+// With near, also flags the particles that boundary particles may reach (bnear of
+// their cell) for the boundary and force passes, and lists them with their scene
+// where a list is wanted.
 template <int BS, bool WITH_VEL>
 __global__ void __launch_bounds__(BS) b_gather_cells_kernel(
     const uint2* __restrict__ tiles, uint32_t num_tiles, const SceneRec* __restrict__ recs,
@@ -101,8 +102,7 @@ __global__ void __launch_bounds__(BS) b_gather_cells_kernel(
     int shift, bool boundary, const float4* __restrict__ pos_in, const float4* __restrict__ vel_in,
     float4* __restrict__ pos_out, float4* __restrict__ vel_out, uint2* __restrict__ cells,
     uint32_t* __restrict__ err, int key_shift = 0, uint32_t* __restrict__ kprev_out = nullptr,
-    const uint8_t* __restrict__ bnear = nullptr, uint8_t* __restrict__ bflag = nullptr,
-    uint32_t* __restrict__ hist = nullptr) {
+    NearList near = NearList{}, uint32_t* __restrict__ hist = nullptr) {
     grid_wait();
     if (hist && blockIdx.x == 0)  // the sort's histograms, for the next step
         for (int k = threadIdx.x; k < kSortMaxPasses * 256; k += blockDim.x) hist[k] = 0;
@@ -126,7 +126,11 @@ __global__ void __launch_bounds__(BS) b_gather_cells_kernel(
         uint32_t* cw = reinterpret_cast<uint32_t*>(cells + R.c_off);
         const uint32_t c = (key >> shift) == tile.x ? morton_to_linear_checked(R.P.g, key & lmask)
                                                     : kEmptyCell;
-        if (bflag) bflag[i] = (c != kEmptyCell && __ldg(&bnear[R.c_off + c]) != 0) ? 1 : 0;
+        if (near.flag) {
+            const bool want = c != kEmptyCell && __ldg(&near.bnear[R.c_off + c]) != 0;
+            near.flag[i] = want ? 1 : 0;
+            if (near.scene_list) near_append(near.count, near.scene_list, want, make_uint2(i, tile.x));
+        }
         if (c == kEmptyCell) {
             atomicOr(err, 2u);
             continue;

@@ -35,6 +35,8 @@ struct sph_batch {
     uint8_t* bnear = nullptr;
     uint32_t *bstart = nullptr, *bcand = nullptr;  // static boundary candidate tables
     float4* bacc = nullptr;              // the step's boundary force sums
+    uint2* blist = nullptr;              // where set (a rollout records): (index, scene) of the flagged
+    uint32_t* bcount = nullptr;          // particles, and their number
     uint8_t* bflag = nullptr;            // per sorted particle: bnear of its cell
     cudaStream_t side = nullptr;         // second branch of the step: the boundary force
     cudaEvent_t fork = nullptr, join = nullptr;

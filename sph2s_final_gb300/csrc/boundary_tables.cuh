@@ -29,7 +29,7 @@ inline cudaError_t build_boundary_tables(const uint2* bcells, const float4* bpos
     e = cudaMalloc(&scratch, 4 * ((size_t)words + 1));
     if (e != cudaSuccess) return e;
     uint32_t* total_d = scratch + words;
-    const float lim = h * 1.01f + 4.0f * bmargin;  // any superset of the neighbours will do
+    const float lim = h * kBoundaryLim + 4.0f * bmargin;  // any superset of the neighbours will do
     if (ncells) {
         boundary_cand_kernel<false><<<blocks, 256, 0, st>>>(bcells, bpos, bnear, g, nb, lim,
                                                             t.start, nullptr);

@@ -185,26 +185,33 @@ __device__ __forceinline__ DepthClass depth_class(const GridParams& g, float x, 
 struct NearList {
     const uint8_t* bnear = nullptr;  // per cell (static); nullptr: no list
     uint32_t* list = nullptr;        // capacity n
+    uint2* scene_list = nullptr;     // or, in a batch: (index, scene)
     uint32_t* count = nullptr;       // zeroed before the kernel
     uint8_t* flag = nullptr;         // per sorted particle, or nullptr
 };
 
-// Appends sorted index i if its cell c is near the boundary: one atomic per
-// warp, each lane's slot from its rank among the appending lanes.  c may be
-// kEmptyCell (a key outside the grid after a failed sort): not listed.
-__device__ __forceinline__ void near_append(const NearList& L, uint32_t c, uint32_t i) {
-    if (!L.list) return;
-    const bool want = c != kEmptyCell && L.bnear[c] != 0;
-    if (L.flag) L.flag[i] = want ? 1 : 0;
+// Appends the entry of the lanes that want to: one atomic per warp, each lane's
+// slot from its rank among the appending lanes.
+template <class T>
+__device__ __forceinline__ void near_append(uint32_t* count, T* list, bool want, T entry) {
     const uint32_t am = __activemask();
     const uint32_t b = __ballot_sync(am, want);
     if (!b) return;
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t leader = (uint32_t)__ffs(b) - 1u;
     uint32_t base = 0;
-    if (lane == leader) base = atomicAdd(L.count, (uint32_t)__popc(b));
+    if (lane == leader) base = atomicAdd(count, (uint32_t)__popc(b));
     base = __shfl_sync(am, base, (int)leader);
-    if (want) L.list[base + (uint32_t)__popc(b & ((1u << lane) - 1u))] = i;
+    if (want) list[base + (uint32_t)__popc(b & ((1u << lane) - 1u))] = entry;
+}
+
+// The same for sorted index i, if its cell c is near the boundary.  c may be
+// kEmptyCell (a key outside the grid after a failed sort): not listed.
+__device__ __forceinline__ void near_append(const NearList& L, uint32_t c, uint32_t i) {
+    if (!L.list) return;
+    const bool want = c != kEmptyCell && L.bnear[c] != 0;
+    if (L.flag) L.flag[i] = want ? 1 : 0;
+    near_append(L.count, L.list, want, i);
 }
 
 // Fills several arrays of 32-bit words in one launch: a step's memsets, each a
@@ -295,6 +302,15 @@ __device__ __forceinline__ T after_wait(T x) {
         asm volatile("" : "+r"(x));
     return x;
 }
+
+// The static boundary candidates of a cell lie within kBoundaryLim h (and 4
+// bmargin) of its box, so they serve particles up to kBoundaryOut h outside the
+// grid's box as well.  Fluid set down on its walls with a jitter is that: its
+// particles each scanned ~700 boundary particles in a lane, 53 us of a step of
+// eight scenes at rest (129 us) and as much of its adjoint.  Moving fluid stays
+// inside; a wider margin only lengthens the lists.
+constexpr float kBoundaryLim = 1.01f;
+constexpr float kBoundaryOut = 0.008f;
 
 // Boundary weight shape of evaluateBoundaryWeight (Solver.cu:169-196)
 // without the 0.02 c^2 / r factor: q = 2r/h.

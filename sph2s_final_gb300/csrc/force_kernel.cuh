@@ -84,16 +84,16 @@ __device__ __forceinline__ void boundary_sum(const float4& xi, const float4* __r
 }
 
 // Whether the static candidate list of a particle's home cell (hx, hy, hz)
-// holds all its boundary neighbours: it lies inside the grid's box and its
-// stencil is home +-1 (clamped); see boundary_force_kernel.
+// holds all its boundary neighbours: its stencil lies within home +-1 and it is
+// inside the grid's box or no further out than the list's margin allows.
 __device__ __forceinline__ bool boundary_listed(const float4& xi, int hx, int hy, int hz,
                                                 const SimParams& P) {
     const Stencil S = stencil(P.g, xi.x, xi.y, xi.z, P.h);
-    const bool inside = xi.x >= P.g.ox && xi.x < P.g.ex && xi.y >= P.g.oy && xi.y < P.g.ey &&
-                        xi.z >= P.g.oz && xi.z < P.g.ez;
-    return inside && S.x0 == max(hx - 1, 0) && S.x1 == min(hx + 1, P.g.dx - 1) &&
-           S.y0 == max(hy - 1, 0) && S.y1 == min(hy + 1, P.g.dy - 1) &&
-           S.z0 == max(hz - 1, 0) && S.z1 == min(hz + 1, P.g.dz - 1);
+    const float out = fmaxf(fmaxf(P.g.ox - xi.x, xi.x - P.g.ex), 0.0f) +
+                      fmaxf(fmaxf(P.g.oy - xi.y, xi.y - P.g.ey), 0.0f) +
+                      fmaxf(fmaxf(P.g.oz - xi.z, xi.z - P.g.ez), 0.0f);
+    return out <= kBoundaryOut * P.h && S.x0 >= hx - 1 && S.x1 <= hx + 1 && S.y0 >= hy - 1 &&
+           S.y1 <= hy + 1 && S.z0 >= hz - 1 && S.z1 <= hz + 1;
 }
 
 // Calls f(xk) for the boundary particles of the stencil at xi, each cell's scan
