@@ -89,10 +89,10 @@ void launch_force(sph_batch* b, int ti, float dt) {
 void enqueue_density(sph_batch* b) {
     cudaEventRecord(b->fork, b->stream);
     cudaStreamWaitEvent(b->side, b->fork, 0);
-    // two blocks per SM: the density blocks fit beside them (a full persistent
-    // grid here would hold every SM until it drained, and density would wait)
-    b_boundary_force_kernel<256><<<std::min(pgrid(b, b->ntiles[1]), 2u * (uint32_t)b->sms), 256,
-                                   0, b->side>>>(
+    // (the density blocks, launched after the pass before them, come first; with two
+    // blocks per SM here the force pass waited for these: 32 scenes 540 / 562 / 583
+    // us per step, now 525 / 543 / 558)
+    b_boundary_force_kernel<256><<<pgrid(b, b->ntiles[1]), 256, 0, b->side>>>(
         b->tiles[1], b->ntiles[1], b->recs, b->spos, b->bpos, b->bcells, b->bnear, b->bstart,
         b->bcand, b->NB, b->bacc, b->bflag);
     cudaEventRecord(b->join, b->side);
@@ -520,7 +520,7 @@ int sphb_get_scene(sph_batch* b, uint32_t scene, float* xyz, float* vel, float* 
 }
 
 // Picks the block size of the density and force passes (128, 256 or 512
-// threads) and the persistent grid (2, 4 or 8 blocks per SM) by timing each
+// threads) and the persistent grid (4, 8 or 12 blocks per SM) by timing each
 // candidate on the batch's own data; the particle state is restored after.
 int sphb_autotune(sph_batch* b, float dt, int32_t* choice) {
     if (!b) return fail(SPH_E_INVALID, "sphb_autotune: NULL handle");
@@ -535,9 +535,9 @@ int sphb_autotune(sph_batch* b, float dt, int32_t* choice) {
     cudaEventCreate(&e0);
     cudaEventCreate(&e1);
     cudaEventCreate(&e2);
-    const int mults[3] = {2, 4, 8};
+    const int mults[3] = {4, 8, 12};
     float best_d = 1e30f, best_f = 1e30f;
-    int bd = 1, bf = 1, bm = 4;
+    int bd = 1, bf = 1, bm = 12;
     float best_total = 1e30f;
     for (int m : mults) {
         b->grid_mult = m;

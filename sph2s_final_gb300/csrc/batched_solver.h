@@ -54,7 +54,12 @@ struct sph_batch {
     uint2* btiles = nullptr;
     uint32_t nbtiles = 0;
     int bs_density = 1, bs_force = 1;  // index into kBlockChoices
-    int grid_mult = 4;                 // persistent grid = grid_mult * SMs
+    // Persistent grids of grid_mult * SMs blocks.  Six density blocks fit on an SM;
+    // twice that many take the tiles half by turn, half as SMs fall free, which
+    // evens out scenes of different density (32 scenes of 1.17M particles, three
+    // phases of a run: 4 blocks per SM 570 / 577 / 582 us per step, 8 535 / 555 /
+    // 572, 12 525 / 543 / 558, one tile per block 552 / 574 / 595).
+    int grid_mult = 12;
     int sms = 152;
     cudaGraphExec_t graph = nullptr;
     float graph_dt = 0.0f;
