@@ -775,12 +775,12 @@ def run_ours(args):
                 "phase_ms": phases,
                 "phase_sum_ms": phases["neighborhood"] + phases["density"] + phases["force"]}
     passes = sort_passes_for(sc.config.grid)
-    # kernels per step: from 131,072 particles the step sorts coherently (keys and
-    # flags, offsets, compaction, digit offsets, the passes, placement, cell
-    # ranges), below from scratch (hash, digit offsets, the passes, gather);
-    # then the boundary force pass beside density, density and force
-    coherent = sc.fluid.num_particles >= 131072
-    launches = ((9 if coherent else 6) + passes) * args.steps
+    # kernels per step: from 524,288 particles the step sorts coherently (keys and
+    # flags, offsets, compaction, the passes, placement, cell ranges), below from
+    # scratch (hash, the passes, gather); then the boundary force pass beside
+    # density, density and force
+    coherent = sc.fluid.num_particles >= 524288
+    launches = ((8 if coherent else 5) + passes) * args.steps
     line = {
         "metric": METRIC, "value": value, "unit": UNIT, "n_gpus": ws, "steps": args.steps,
         "warmup": args.warmup, "ms_per_step": ms / args.steps, "higher_is_better": True,

@@ -113,7 +113,7 @@ void enqueue_force(sph_batch* b, float dt) {
 }
 
 // hash -> stable sort of (scene, cell key, index) -> reorder + cell ranges.
-// From 131,072 fluid particles the sort is the coherent one (coherent_sort.cuh:
+// From 524,288 fluid particles the sort is the coherent one (coherent_sort.cuh:
 // the same permutation, radix-sorting only the particles that changed cell).
 int enqueue_neighborhood(sph_batch* b) {
     cudaStream_t st = b->stream;
@@ -273,7 +273,7 @@ int sphb_create(const sph_scene_desc* scenes, uint32_t num_scenes, sph_batch** o
     b->owned.push_back(b->sort_mem);
     b->sort = sort_scratch_from(b->sort_mem, plan);
     sort_reset(b->sort, b->stream);
-    b->coherent = b->N >= 131072u;
+    b->coherent = b->N >= 1u << 19;  // as kCoherentMinParticles
     if (b->coherent) {
         TRY(check_cuda(cudaMalloc(&b->co_mem, coherent_bytes(b->N)), "sort scratch", __FILE__, __LINE__));
         b->owned.push_back(b->co_mem);

@@ -43,7 +43,7 @@ struct sph_batch {
     float4* bpos = nullptr;
     void* sort_mem = nullptr;
     SortScratch sort;
-    void* co_mem = nullptr;  // the step's coherent sort (from 131,072 fluid particles on)
+    void* co_mem = nullptr;  // the step's coherent sort (from 524,288 fluid particles on)
     sph::CoherentSort co;
     bool coherent = false;
     uint32_t* err = nullptr;

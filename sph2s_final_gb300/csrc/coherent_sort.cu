@@ -384,7 +384,7 @@ void coherent_run(const CoherentSort& c, const float4* pos, const GridParams* g,
     // the sort's histograms, tile counters and look-back words are one block
     const StepClear clear = {nullptr, 0u, s.hist,
                              (uint32_t)(s.tile_ctr - s.hist) +
-                                 sort_pass_words(sort_tiles(n, kMoverSmallMax, true), passes),
+                                 sort_pass_words(sort_tiles(n, kMoverSmallMax), passes),
                              near_count};
     if (pos)
         coherent_flag_kernel<true><<<tiles, kCoThreads, 0, st>>>(pos, *g, keys, n, c.kprev,

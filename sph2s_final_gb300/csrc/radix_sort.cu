@@ -69,7 +69,7 @@ __global__ void __launch_bounds__(256) histogram_kernel(const uint32_t* __restri
 __global__ void __launch_bounds__(kSortThreads) onesweep_kernel(
     const uint32_t* __restrict__ keys_in, const uint32_t* __restrict__ vals_in,
     uint32_t* __restrict__ keys_out, uint32_t* __restrict__ vals_out, uint32_t n,
-    const uint32_t* __restrict__ n_dev, uint32_t small_max, int shift,
+    const uint32_t* __restrict__ n_dev, uint32_t small_max, int items, int shift,
     const uint32_t* __restrict__ hist, uint32_t* status, uint32_t* tile_ctr,
     uint32_t* err, int force_timeout) {
     __shared__ uint32_t s_keys[kSortTile];
@@ -84,7 +84,7 @@ __global__ void __launch_bounds__(kSortThreads) onesweep_kernel(
     grid_wait();
     if (n_dev) n = min(*after_wait(n_dev), n);  // key count known on the device only: the grid covers n keys
     if (n == 0) return;
-    const int ni = n <= small_max ? kSortItemsSmall : kSortItems;  // keys per thread
+    const int ni = n_dev && n <= small_max ? kSortItemsSmall : items;  // keys per thread
     const uint32_t tile_keys = (uint32_t)ni * kSortThreads;
     if (tid == 0) s_tile = atomicAdd(tile_ctr, 1u);
     for (int i = tid; i < kWarps * 257; i += kSortThreads) (&s_whist[0][0])[i] = 0;
@@ -237,44 +237,58 @@ void sort_pass(const uint32_t* keys_in, const uint32_t* vals_in, uint32_t* keys_
     if (n == 0) return;
     uint32_t tiles = (n + kSortTile - 1) / kSortTile;
     onesweep_kernel<<<tiles, kSortThreads, 0, st>>>(
-        keys_in, vals_in, keys_out, vals_out, n, nullptr, 0u, 8 * p, s.hist + p * 256,
+        keys_in, vals_in, keys_out, vals_out, n, nullptr, 0u, kSortItems, 8 * p, s.hist + p * 256,
         s.status + (size_t)p * tiles * 256, s.tile_ctr + p, err, force_timeout);
 }
 
-uint32_t sort_tiles(uint32_t n, uint32_t small_max, bool counted) {
+uint32_t sort_tiles(uint32_t n, uint32_t small_max) {
     const uint32_t tiles = (n + kSortTile - 1) / kSortTile;
-    const uint32_t few = counted ? (n < small_max ? n : small_max) : (n <= small_max ? n : 0u);
+    const uint32_t few = n < small_max ? n : small_max;
     const uint32_t small_tiles = (few + kSortTileSmall - 1) / kSortTileSmall;
     return small_tiles > tiles ? small_tiles : tiles;
 }
 
-int sort_passes_run_dev(uint32_t* keys[2], uint32_t* vals[2], const uint32_t* first_vals,
-                        uint32_t n, const uint32_t* n_dev, uint32_t small_max, int passes,
-                        const SortScratch& s, uint32_t* err, int force_timeout, cudaStream_t st) {
-    if (n == 0) return 0;
-    const uint32_t tiles = sort_tiles(n, small_max, n_dev != nullptr);
+namespace {
+
+int passes_run(uint32_t* keys[2], uint32_t* vals[2], const uint32_t* first_vals, uint32_t n,
+               const uint32_t* n_dev, uint32_t small_max, int items, uint32_t tiles, int passes,
+               const SortScratch& s, uint32_t* err, int force_timeout, cudaStream_t st) {
     int cur = 0;
     for (int p = 0; p < passes; ++p) {
         const uint32_t* vin = (p == 0) ? first_vals : vals[cur];
         launch_after(onesweep_kernel, tiles, kSortThreads, st, keys[cur], vin, keys[cur ^ 1],
-                     vals[cur ^ 1], n, n_dev, small_max, 8 * p, s.hist + p * 256,
+                     vals[cur ^ 1], n, n_dev, small_max, items, 8 * p, s.hist + p * 256,
                      s.status + (size_t)p * tiles * 256, s.tile_ctr + p, err, force_timeout);
         cur ^= 1;
     }
     return cur;
 }
 
+}  // namespace
+
+int sort_passes_run_dev(uint32_t* keys[2], uint32_t* vals[2], const uint32_t* first_vals,
+                        uint32_t n, const uint32_t* n_dev, uint32_t small_max, int passes,
+                        const SortScratch& s, uint32_t* err, int force_timeout, cudaStream_t st) {
+    if (n == 0) return 0;
+    return passes_run(keys, vals, first_vals, n, n_dev, small_max, kSortItems,
+                      sort_tiles(n, small_max), passes, s, err, force_timeout, st);
+}
+
 int sort_passes_run(uint32_t* keys[2], uint32_t* vals[2], const uint32_t* first_vals, uint32_t n,
                     int passes, const SortScratch& s, uint32_t* err, int force_timeout,
                     cudaStream_t st) {
-    return sort_passes_run_dev(keys, vals, first_vals, n, nullptr, 0u, passes, s, err,
-                               force_timeout, st);
+    if (n == 0) return 0;
+    return passes_run(keys, vals, first_vals, n, nullptr, 0u, kSortItems,
+                      (n + kSortTile - 1) / kSortTile, passes, s, err, force_timeout, st);
 }
 
 int sort_step_run(uint32_t* keys[2], uint32_t* vals[2], uint32_t n, int passes,
                   const SortScratch& s, uint32_t* err, int force_timeout, cudaStream_t st) {
-    return sort_passes_run_dev(keys, vals, nullptr, n, nullptr, kSortStepSmall, passes, s, err,
-                               force_timeout, st);
+    if (n == 0) return 0;
+    const int items = sort_step_items(n);
+    const uint32_t tile = (uint32_t)(kSortThreads * items);
+    return passes_run(keys, vals, nullptr, n, nullptr, 0u, items, (n + tile - 1) / tile, passes, s,
+                      err, force_timeout, st);
 }
 
 int sort_pairs(uint32_t* keys[2], uint32_t* vals[2], uint32_t n, int key_bits,

@@ -27,11 +27,14 @@ constexpr int kSortTile = kSortThreads * kSortItems;  // 4096 keys
 constexpr int kSortItemsSmall = 2;
 constexpr int kSortTileSmall = kSortThreads * kSortItemsSmall;
 constexpr int kSortMaxPasses = 4;
-// A step's sort of at most this many keys uses the small tiles: more of the chip
-// sorts (us per step, large tiles and small: 4,096 keys 58 and 56, 32,768 65.8 and
-// 64.2, 64,000 86.5 and 86.1).  Beyond, the walk back over them costs more (110,592:
-// 92.6 and 93.8).
-constexpr uint32_t kSortStepSmall = 1u << 16;
+// Keys per thread of a step's sort of n keys: fewer let more of the chip sort, more
+// keep the walk back over the tiles short.  Us per step with 2, 8 and 16: 32,768 keys
+// 64.2, -, 65.8; 64,000 86.1, -, 86.5; 110,592 93.8, 91.4, 92.6; 175,616 -, 112.9, 114.6;
+// 512,000 -, 239.8, 239.6; 1,000,000 -, 419, 413 (4 at 262,144: 157 against 155 with 8).
+constexpr uint32_t kSortStepFew = 1u << 16, kSortStepMid = 1u << 19;
+inline int sort_step_items(uint32_t n) {
+    return n <= kSortStepFew ? kSortItemsSmall : n <= kSortStepMid ? 8 : kSortItems;
+}
 
 // Device scratch of one sort plan.  Everything that must start at zero lives
 // in one contiguous block so a single memset resets it.
@@ -90,9 +93,9 @@ int sort_passes_run_dev(uint32_t* keys[2], uint32_t* vals[2], const uint32_t* fi
                         uint32_t n, const uint32_t* n_dev, uint32_t small_max, int passes,
                         const SortScratch& s, uint32_t* err, int force_timeout, cudaStream_t st);
 
-// Tiles of one pass over n keys (counted: of at most n, as in sort_passes_run_dev),
-// and the words from s.tile_ctr that `passes` such passes need cleared.
-uint32_t sort_tiles(uint32_t n, uint32_t small_max, bool counted);
+// Tiles of one pass over at most n keys, a number that the device knows
+// (sort_passes_run_dev), and the words from s.tile_ctr that `passes` such passes need cleared.
+uint32_t sort_tiles(uint32_t n, uint32_t small_max);
 inline uint32_t sort_pass_words(uint32_t tiles, int passes) {
     return 64u + (uint32_t)passes * tiles * 256u;
 }
@@ -102,12 +105,17 @@ inline uint32_t sort_pass_words(uint32_t tiles, int passes) {
 // histograms to s.hist, which a kernel after the sort zeroes for the next step.
 // The plan holds sort_step_plan_keys(n) keys.
 inline uint32_t sort_step_plan_keys(uint32_t n) {
-    const uint32_t few = n < kSortStepSmall ? n : kSortStepSmall;
-    const uint32_t small = few * (uint32_t)(kSortTile / kSortTileSmall);
-    return n > small ? n : small;
+    uint32_t most = n;  // as many tiles as any count up to n takes
+    for (uint32_t k : {kSortStepFew, kSortStepMid}) {
+        const uint32_t m = n < k ? n : k;
+        const uint32_t keys = m * (uint32_t)(kSortItems / sort_step_items(m));
+        most = most > keys ? most : keys;
+    }
+    return most;
 }
 inline uint32_t sort_step_words(uint32_t n, int passes) {
-    return sort_pass_words(sort_tiles(n, kSortStepSmall, false), passes);
+    const uint32_t tile = (uint32_t)(kSortThreads * sort_step_items(n));
+    return sort_pass_words((n + tile - 1) / tile, passes);
 }
 int sort_step_run(uint32_t* keys[2], uint32_t* vals[2], uint32_t n, int passes,
                   const SortScratch& s, uint32_t* err, int force_timeout, cudaStream_t st);

@@ -67,9 +67,13 @@ struct sph_solver {
 
 namespace sph_ss {
 // The step's sort: automatic (coherent from kCoherentMinParticles on, where it
-// is faster on GB300), from scratch, or coherent.
+// is faster on GB300), from scratch, or coherent.  Us per step from scratch and
+// coherent: 110,592 particles 92.7 and 97.3, 262,144 152 and 156, 512,000 240 and
+// 244, 1,000,000 410 and 415, 1,481,544 587 and 583, 2,097,152 798 and 787; with
+// several solvers on the GPU at once, where the memory it saves counts more than its
+// launches, 1.17M particles of a batch 585 and 569.
 constexpr int kSortAuto = 0, kSortFull = 1, kSortCoherent = 2;
-constexpr uint32_t kCoherentMinParticles = 131072;
+constexpr uint32_t kCoherentMinParticles = 1u << 19;
 // hash -> sort (coherent or from scratch, sort_mode) -> reorder + cell ranges;
 // returns the index of the key/value buffers that hold the sorted keys and
 // the permutation.
