@@ -264,6 +264,13 @@ void ts_neighborhoods(sph_solver2* s) {
             s->occ + s->occ_low);
 }
 
+// Steps of fewer particles take several lanes for every particle: one each leaves
+// the chip to a few chains of candidates.  Us per step, one lane and several:
+// 7,290 particles 128 and 83, 19,565 140 and 105, 38,397 154 and 132, 65,416 173 and
+// 177, 88,587 189 and 213.
+constexpr uint32_t kTsSmall = 49152;
+constexpr int kTsSmallLow = 16, kTsSmallHigh = 8, kTsForceLow = 16, kTsForceHigh = 2;
+
 // Everything up to and including the force/integrate pass; DEBUG variants
 // also write accelerations and neighbour counts of population `dbg_pop`.
 void ts_front(sph_solver2* s, float dt, bool debug, int dbg_pop, uint32_t* dnb_same,
@@ -310,7 +317,8 @@ void ts_front(sph_solver2* s, float dt, bool debug, int dbg_pop, uint32_t* dnb_s
     cudaStream_t lo = s->lowst;
     // LOW particles beside HIGH ones have passes of their own, several lanes
     // each, on a third stream (not in the debug passes)
-    const bool lanes = !debug && L.n && H.n;
+    const bool small = !debug && L.n + H.n < kTsSmall;
+    const bool lanes = !debug && !small && L.n && H.n;
     const uint8_t* skip = lanes ? s->near_flag : nullptr;
     if (lanes) {
         ts_near_kernel<<<blocks_for(L.n), 256, 0, st>>>(L.spos, L.n, s->P.g[0], s->P.h[0], s->occ,
@@ -322,13 +330,19 @@ void ts_front(sph_solver2* s, float dt, bool debug, int dbg_pop, uint32_t* dnb_s
         cudaStreamWaitEvent(s->nearst, s->pfork, 0);
         const uint32_t blocks = std::min(blocks_for(L.n, 32 * kTsWarps / kTsLanes),
                                          (uint32_t)(4 * s->sms));
-        ts_density_lanes_kernel<<<blocks, 32 * kTsWarps, 0, s->nearst>>>(
+        ts_density_lanes_kernel<0, kTsLanes, 32, 56><<<blocks, 32 * kTsWarps, 0, s->nearst>>>(
             s->near_list, s->near_count, L.spos, L.cells, L.n, H.spos, H.cells, H.n, s->P, L.rho,
             L.aux, L.list, L.list_count, L.clist, L.clist_count);
         cudaEventRecord(s->njoin, s->nearst);
     }
     if (H.n) {
-        if (debug && dbg_pop == 1)
+        if (small)
+            ts_density_lanes_kernel<1, kTsSmallHigh, 48, 24>
+                <<<blocks_for(H.n, 32 * kTsWarps / kTsSmallHigh), 32 * kTsWarps, 0, st>>>(
+                    nullptr, nullptr, H.spos, H.cells, H.n, L.spos, L.cells, L.n, s->P, H.rho, H.aux,
+                    H.list, H.list_count, H.clist, H.clist_count, H.sgrp, gb, s->gsum,
+                    L.n ? s->occ + s->occ_low : nullptr);
+        else if (debug && dbg_pop == 1)
             ts_density_kernel<1, true><<<blocks_for(H.n), 256, 0, st>>>(
                 H.spos, H.cells, H.n, L.spos, L.cells, L.n, s->P, H.rho, H.aux, dnb_same, dnb_compl,
                 H.sgrp, gb, s->gsum, H.list, H.list_count, H.clist, H.clist_count);
@@ -339,7 +353,12 @@ void ts_front(sph_solver2* s, float dt, bool debug, int dbg_pop, uint32_t* dnb_s
                 lanes ? s->occ + s->occ_low : nullptr);
     }
     if (L.n) {
-        if (debug && dbg_pop == 0)
+        if (small)
+            ts_density_lanes_kernel<0, kTsSmallLow, 32, 40>
+                <<<blocks_for(L.n, 32 * kTsWarps / kTsSmallLow), 32 * kTsWarps, 0, lo>>>(
+                    nullptr, nullptr, L.spos, L.cells, L.n, H.spos, H.cells, H.n, s->P, L.rho, L.aux,
+                    L.list, L.list_count, L.clist, L.clist_count);
+        else if (debug && dbg_pop == 0)
             ts_density_kernel<0, true><<<blocks_for(L.n), 256, 0, lo>>>(
                 L.spos, L.cells, L.n, H.spos, H.cells, H.n, s->P, L.rho, L.aux, dnb_same, dnb_compl,
                 L.sgrp, gb, s->gsum, L.list, L.list_count, L.clist, L.clist_count);
@@ -373,7 +392,12 @@ void ts_front(sph_solver2* s, float dt, bool debug, int dbg_pop, uint32_t* dnb_s
     }
     if (H.n) {
         TSOut o = outputs(H, dacc, dnb_bnd, (s->colour_on && !debug) ? s->colour[1] : nullptr);
-        if (debug && dbg_pop == 1)
+        if (small)
+            ts_force_kernel<1, false, kTsForceHigh><<<blocks_for(H.n, 256 / kTsForceHigh), 256, 0, st>>>(
+                H.spos, H.svel, H.sstt, H.sgrp, H.aux, H.cells, H.n, L.spos, L.svel, L.aux, L.cells,
+                L.n, s->bpos, s->bcells, s->bnear, s->nb, s->P, dt, gm, gb, s->gacc, s->ctl, H.rho,
+                H.list, H.list_count, H.clist, H.clist_count, o, H.bacc);
+        else if (debug && dbg_pop == 1)
             ts_force_kernel<1, true><<<blocks_for(H.n), 256, 0, st>>>(
                 H.spos, H.svel, H.sstt, H.sgrp, H.aux, H.cells, H.n, L.spos, L.svel, L.aux, L.cells,
                 L.n, s->bpos, s->bcells, s->bnear, s->nb, s->P, dt, gm, gb, s->gacc, s->ctl, H.rho, H.list, H.list_count, H.clist, H.clist_count, o, nullptr);
@@ -384,7 +408,12 @@ void ts_front(sph_solver2* s, float dt, bool debug, int dbg_pop, uint32_t* dnb_s
     }
     if (L.n) {
         TSOut o = outputs(L, dacc, dnb_bnd, (s->colour_on && !debug) ? s->colour[0] : nullptr);
-        if (debug && dbg_pop == 0)
+        if (small)
+            ts_force_kernel<0, false, kTsForceLow><<<blocks_for(L.n, 256 / kTsForceLow), 256, 0, lo>>>(
+                L.spos, L.svel, L.sstt, L.sgrp, L.aux, L.cells, L.n, H.spos, H.svel, H.aux, H.cells,
+                H.n, s->bpos, s->bcells, s->bnear, s->nb, s->P, dt, gm, gb, s->gacc, s->ctl, L.rho,
+                L.list, L.list_count, L.clist, L.clist_count, o, L.bacc);
+        else if (debug && dbg_pop == 0)
             ts_force_kernel<0, true><<<blocks_for(L.n), 256, 0, lo>>>(
                 L.spos, L.svel, L.sstt, L.sgrp, L.aux, L.cells, L.n, H.spos, H.svel, H.aux, H.cells,
                 H.n, s->bpos, s->bcells, s->bnear, s->nb, s->P, dt, gm, gb, s->gacc, s->ctl, L.rho, L.list, L.list_count, L.clist, L.clist_count, o, nullptr);

@@ -196,6 +196,28 @@ __device__ __forceinline__ float ts_density_out(uint32_t i, float s, float sc, c
     return rh;
 }
 
+// Counts a HIGH member of a group at the surface.
+__device__ __forceinline__ void ts_surface(uint32_t i, float rh, const TSParams& P,
+                                           const uint32_t* __restrict__ sgrp, uint32_t group_base,
+                                           unsigned long long* __restrict__ gsurf) {
+    if (!P.surface || !(rh < P.surf_rho)) return;
+    const uint32_t gid = sgrp[i];
+    if (gid != kNoGroup && gid < group_base) atomicAdd(&gsurf[gid], 1ull);
+}
+
+// Whether the blocks of LOW cells that a HIGH particle's stencil meets hold any
+// LOW particle: most HIGH particles have none near.
+__device__ __forceinline__ bool ts_any_low(const TSParams& P, const float4& xi,
+                                           const uint8_t* __restrict__ low_blocks) {
+    const Stencil st = stencil(P.g[0], xi.x, xi.y, xi.z, P.h[0]);
+    bool any = false;
+    for (int bz = st.z0 >> 2; bz <= st.z1 >> 2; ++bz)
+        for (int by = st.y0 >> 2; by <= st.y1 >> 2; ++by)
+            for (int bx = st.x0 >> 2; bx <= st.x1 >> 2; ++bx)
+                any |= __ldg(&low_blocks[ts_block(P.g[0], bx, by, bz)]) != 0;
+    return any;
+}
+
 // LOW particles with HIGH particles in the cells of their stencil on the LOW
 // grid (occ, marked by ts_gather_kernel): every HIGH particle within h_LOW lies
 // in one of them.  flag[i], and their sorted indices in no particular order.
@@ -282,13 +304,7 @@ __global__ void __launch_bounds__(256) ts_density_kernel(
     bool any = n_c > 0 && !skip;  // where skip tells who has any, none is left here
     Stencil st = {0, -1, 0, -1, 0, -1};
     if (any) st = stencil(P.g[C], xi.x, xi.y, xi.z, P.h[0]);
-    if (R == 1 && low_blocks) {  // most HIGH particles have no LOW ones near
-        any = false;
-        for (int bz = st.z0 >> 2; bz <= st.z1 >> 2; ++bz)
-            for (int by = st.y0 >> 2; by <= st.y1 >> 2; ++by)
-                for (int bx = st.x0 >> 2; bx <= st.x1 >> 2; ++bx)
-                    any |= __ldg(&low_blocks[ts_block(P.g[0], bx, by, bz)]) != 0;
-    }
+    if (R == 1 && low_blocks) any = ts_any_low(P, xi, low_blocks);
     if (any) {
         for (int cz = st.z0; cz <= st.z1; ++cz)
             for (int cy = st.y0; cy <= st.y1; ++cy) {
@@ -323,10 +339,7 @@ __global__ void __launch_bounds__(256) ts_density_kernel(
         nbr_same[i] = ns;
         nbr_compl[i] = nc;
     }
-    if (R == 1 && P.surface && rh < P.surf_rho) {  // members of a group at the surface
-        const uint32_t gid = sgrp_r[i];
-        if (gid != kNoGroup && gid < group_base) atomicAdd(&gsurf[gid], 1ull);
-    }
+    if (R == 1) ts_surface(i, rh, P, sgrp_r, group_base, gsurf);
 }
 
 // The same for the listed LOW particles (ts_near_kernel), kTsLanes lanes each:
@@ -336,57 +349,60 @@ __global__ void __launch_bounds__(256) ts_density_kernel(
 // us beside 39 / 68 us for the other LOW particles.  Each lane scans a
 // contiguous share of the stencil's rows, its hits go through shared memory
 // into the lists in stencil order, and the lanes' sums are added in a fixed
-// order.  A lane that runs out of room leaves the particle's list to the force
-// pass's rescan.
+// order.  A lane that runs out of room scans its share again and writes the list
+// itself (leaving the list to the force pass's rescan, one lane for the whole
+// stencil, took 332-357 us per step where the coupled fluid of 338,367 is
+// compressed, now 272).  Every particle of a small scene goes this way (kTsSmall).
 constexpr uint32_t kTsLanes = 8;
-constexpr uint32_t kTsSame = 32, kTsCompl = 56;  // hits per lane
 constexpr int kTsWarps = 4;
 
-// Appends the lanes' hits (hit[e * 32], e < k) in lane order to particle i's
-// list; returns the particle's count, beyond `cap` if some lane had no room.
-__device__ __forceinline__ uint32_t ts_lanes_list(const uint32_t* hit, uint32_t k, uint32_t room,
-                                                  uint32_t cap, uint32_t i, uint32_t n, bool on,
-                                                  uint4* __restrict__ list4) {
+// Where a lane's k hits start in its particle's list (lane order); total: the
+// particle's count.
+template <uint32_t LANES>
+__device__ __forceinline__ uint32_t ts_lanes_start(uint32_t k, uint32_t& total) {
     constexpr uint32_t kAll = 0xFFFFFFFFu;
-    const uint32_t sub = threadIdx.x & (kTsLanes - 1u), lane = threadIdx.x & 31u;
+    const uint32_t lane = threadIdx.x & 31u, sub = lane & (LANES - 1u);
     uint32_t at = k;
 #pragma unroll
-    for (uint32_t d = 1; d < kTsLanes; d <<= 1) {
+    for (uint32_t d = 1; d < LANES; d <<= 1) {
         const uint32_t y = __shfl_up_sync(kAll, at, d);
         if (sub >= d) at += y;
     }
-    const uint32_t total = __shfl_sync(kAll, at, (int)(lane | (kTsLanes - 1u)));
-    const uint32_t full = __ballot_sync(kAll, k > room) >> (lane & ~(kTsLanes - 1u));
-    at -= k;
-    if (on) {
-        uint32_t* out = reinterpret_cast<uint32_t*>(list4) + 4 * ((size_t)(at >> 2) * n + i) + (at & 3u);
-        const uint32_t next_group = 4u * n - 3u;
-        for (uint32_t e = 0; e < min(k, room) && at < cap; ++e, ++at) {
-            __stcs(out, hit[e * 32]);
-            out += (at & 3u) == 3u ? next_group : 1u;
-        }
-    }
-    return full & ((1u << kTsLanes) - 1u) ? max(total, cap + 1u) : total;
+    total = __shfl_sync(kAll, at, (int)(lane | (LANES - 1u)));
+    return at - k;
 }
 
-static __global__ void __launch_bounds__(32 * kTsWarps) ts_density_lanes_kernel(
+// Entry `at` of particle i's list (grouped layout).
+__device__ __forceinline__ void ts_list_put(uint4* __restrict__ list4, uint32_t at, uint32_t i,
+                                            uint32_t n, uint32_t j) {
+    __stcs(reinterpret_cast<uint32_t*>(list4) + 4 * ((size_t)(at >> 2) * n + i) + (at & 3u), j);
+}
+
+// R the population, SAME and COMPL the hits a lane has room for; without a list
+// (near NULL) every particle.
+template <int R, uint32_t LANES, uint32_t SAME, uint32_t COMPL>
+__global__ void __launch_bounds__(32 * kTsWarps) ts_density_lanes_kernel(
     const uint32_t* __restrict__ near, const uint32_t* __restrict__ near_count,
-    const float4* __restrict__ spos_l, const uint2* __restrict__ cells_l, uint32_t n_l,
-    const float4* __restrict__ spos_h, const uint2* __restrict__ cells_h, uint32_t n_h,
+    const float4* __restrict__ spos_r, const uint2* __restrict__ cells_r, uint32_t n_r,
+    const float4* __restrict__ spos_c, const uint2* __restrict__ cells_c, uint32_t n_c,
     TSParams P, float* __restrict__ rho, float2* __restrict__ aux, uint4* __restrict__ list4,
     uint32_t* __restrict__ list_count, uint4* __restrict__ clist4,
-    uint32_t* __restrict__ clist_count) {
-    __shared__ uint32_t s_hit[kTsWarps][(kTsSame + kTsCompl) * 32];
-    const uint32_t lane = threadIdx.x & 31u, sub = lane & (kTsLanes - 1u);
-    const uint32_t count = min(*near_count, n_l);
-    const uint32_t per = 32 / kTsLanes, warps = gridDim.x * kTsWarps;
+    uint32_t* __restrict__ clist_count, const uint32_t* __restrict__ sgrp_r = nullptr,
+    uint32_t group_base = 0, unsigned long long* __restrict__ gsurf = nullptr,
+    const uint8_t* __restrict__ low_blocks = nullptr) {
+    constexpr int C = 1 - R;
+    __shared__ uint32_t s_hit[kTsWarps][(SAME + COMPL) * 32];
+    const uint32_t lane = threadIdx.x & 31u, sub = lane & (LANES - 1u);
+    const uint32_t count = near ? min(*near_count, n_r) : n_r;
+    const uint32_t per = 32 / LANES, warps = gridDim.x * kTsWarps;
     uint32_t* hs = s_hit[threadIdx.x >> 5] + lane;
-    uint32_t* hc = hs + kTsSame * 32;
+    uint32_t* hc = hs + SAME * 32;
     for (uint32_t t = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * per; t < count;
          t += warps * per) {
-        const bool on = t + lane / kTsLanes < count;
-        const uint32_t i = on ? min(near[t + lane / kTsLanes], n_l - 1u) : 0u;
-        const float4 xi = spos_l[i];
+        const bool on = t + lane / LANES < count;
+        const uint32_t e = t + lane / LANES;
+        const uint32_t i = !on ? 0u : near ? min(near[e], n_r - 1u) : e;
+        const float4 xi = spos_r[i];
         float s = 0.0f, sc = 0.0f;
         uint32_t k = 0, kc = 0;
         // f(j, xj, r2) for this lane's share of the stencil's candidates with r2 < T
@@ -395,8 +411,8 @@ static __global__ void __launch_bounds__(32 * kTsWarps) ts_density_lanes_kernel(
             const Stencil st = stencil(g, xi.x, xi.y, xi.z, h);
             const uint32_t ny = (uint32_t)(st.y1 - st.y0 + 1);
             const uint32_t rows = ny * (uint32_t)(st.z1 - st.z0 + 1);
-            const uint32_t last = (sub + 1) * rows / kTsLanes;
-            for (uint32_t r = sub * rows / kTsLanes; r < last; ++r) {
+            const uint32_t last = (sub + 1) * rows / LANES;
+            for (uint32_t r = sub * rows / LANES; r < last; ++r) {
                 const uint32_t row = linear_cell(g, 0, st.y0 + (int)(r % ny), st.z0 + (int)(r / ny));
                 for (int cx = st.x0; cx <= st.x1; ++cx) {
                     const uint2 c = __ldg(&cells[row + cx]);
@@ -411,37 +427,58 @@ static __global__ void __launch_bounds__(32 * kTsWarps) ts_density_lanes_kernel(
             }
         };
         if (on) {
-            scan(P.g[0], cells_l, spos_l, n_l, P.h[0], P.T[0], [&](uint32_t j, const float4& xj, float r2) {
-                const float a = P.h2[0] - r2;
+            scan(P.g[R], cells_r, spos_r, n_r, P.h[R], P.T[R], [&](uint32_t j, const float4& xj, float r2) {
+                const float a = P.h2[R] - r2;
                 s = fmaf(P.coupled ? 1.0f : xj.w, a * a * a, s);
                 if (r2 != 0.0f) {
-                    if (k < kTsSame) hs[k * 32] = j;
+                    if (k < SAME) hs[k * 32] = j;
                     ++k;
                 }
             });
-            scan(P.g[1], cells_h, spos_h, n_h, P.h[0], P.T[0], [&](uint32_t j, const float4& xj, float r2) {
+        }
+        bool any = on && n_c > 0;
+        if (R == 1 && low_blocks && any) any = ts_any_low(P, xi, low_blocks);
+        if (any) {
+            scan(P.g[C], cells_c, spos_c, n_c, P.h[0], P.T[0], [&](uint32_t j, const float4& xj, float r2) {
                 const float a0 = P.h2[0] - r2, a1 = P.h2[1] - r2;
                 float w = P.poly6[0] * a0 * a0 * a0;
                 if (r2 < P.T[1]) w += P.poly6[1] * a1 * a1 * a1;
                 sc = fmaf(P.coupled ? 1.0f : xj.w, 0.5f * w, sc);
                 if (r2 != 0.0f) {
-                    if (kc < kTsCompl) hc[kc * 32] = j;
+                    if (kc < COMPL) hc[kc * 32] = j;
                     ++kc;
                 }
             });
         }
         __syncwarp();
-        const uint32_t same = ts_lanes_list(hs, k, kTsSame, (uint32_t)kMaxNbr, i, n_l, on, list4);
-        const uint32_t compl_ = ts_lanes_list(hc, kc, kTsCompl, ComplCap<0>::value, i, n_l, on, clist4);
+        uint32_t same, compl_;
+        uint32_t at = ts_lanes_start<LANES>(k, same), cat = ts_lanes_start<LANES>(kc, compl_);
+        if (k <= SAME) {
+            for (uint32_t e = 0; e < k && at < (uint32_t)kMaxNbr; ++e, ++at)
+                ts_list_put(list4, at, i, n_r, hs[e * 32]);
+        } else {
+            scan(P.g[R], cells_r, spos_r, n_r, P.h[R], P.T[R], [&](uint32_t j, const float4&, float r2) {
+                if (r2 != 0.0f && at < (uint32_t)kMaxNbr) ts_list_put(list4, at++, i, n_r, j);
+            });
+        }
+        if (kc <= COMPL) {
+            for (uint32_t e = 0; e < kc && cat < ComplCap<R>::value; ++e, ++cat)
+                ts_list_put(clist4, cat, i, n_r, hc[e * 32]);
+        } else {
+            scan(P.g[C], cells_c, spos_c, n_c, P.h[0], P.T[0], [&](uint32_t j, const float4&, float r2) {
+                if (r2 != 0.0f && cat < ComplCap<R>::value) ts_list_put(clist4, cat++, i, n_r, j);
+            });
+        }
 #pragma unroll
-        for (uint32_t d = kTsLanes / 2; d; d >>= 1) {
+        for (uint32_t d = LANES / 2; d; d >>= 1) {
             s += __shfl_xor_sync(0xFFFFFFFFu, s, d);
             sc += __shfl_xor_sync(0xFFFFFFFFu, sc, d);
         }
         if (on && sub == 0) {
-            ts_density_out<0>(i, s, sc, P, rho, aux);
+            const float rh = ts_density_out<R>(i, s, sc, P, rho, aux);
             list_count[i] = same;
             clist_count[i] = compl_;
+            if (R == 1) ts_surface(i, rh, P, sgrp_r, group_base, gsurf);
         }
         __syncwarp();
     }
@@ -511,10 +548,10 @@ __global__ void __launch_bounds__(256) ts_force_kernel(
     uint32_t i = blockIdx.x * (blockDim.x / LANES) + threadIdx.x / LANES;
     bool on = true;
     if (LANES > 1) {
-        const uint32_t count = min(*near_count, n_r);
+        const uint32_t count = near ? min(*near_count, n_r) : n_r;
         if (i - (threadIdx.x & 31u) / LANES >= count) return;  // whole warps: sums are shuffled
         on = i < count;
-        i = on ? min(near[i], n_r - 1u) : 0u;
+        i = !on ? 0u : near ? min(near[i], n_r - 1u) : i;
     } else if (i >= n_r || (skip && skip[i])) {
         return;
     }

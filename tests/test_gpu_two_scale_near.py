@@ -3,7 +3,8 @@ a particle: one step against the oracle (the bounds of test_gpu_two_scale) where
 that can go wrong: a single neighbour, counts around the lanes, fine particles
 in one row of cells (one lane's share overflows, the list does not), a ball with
 more fine particles than a list holds, populations that appear later, and steps
-far enough on to run as an updated graph."""
+far enough on to run as an updated graph.  Small scenes (below 49,152 particles)
+give every particle several lanes; one larger scene has them near alone."""
 import numpy as np
 import pytest
 
@@ -40,6 +41,17 @@ def test_near_particles(kind, coupled):
     for low in (sc.low.positions, sc.low.positions[:1], sc.low.positions[:33]):
         with Solver2(low, high, sc.boundary, sc.config) as s:
             check_step(s, sc)
+
+
+@pytest.mark.parametrize("coupled", [False, True])
+@pytest.mark.parametrize("kind", ["one", "ragged", "row", "ball"])
+def test_near_particles_of_a_larger_scene(kind, coupled):
+    sc = scenes.two_scale_dam_break(1 / 80, (40, 36, 36), dt=8e-6, slab=(2.0, 3.0))
+    sc.config.mode = 1 if coupled else 0
+    high = (0.4 * fine(kind, np.random.default_rng(6))).astype(np.float32)
+    assert len(sc.low.positions) >= 49152
+    with Solver2(sc.low.positions, high, sc.boundary, sc.config) as s:
+        check_step(s, sc)
 
 
 def test_sizes_that_change_while_the_step_is_a_graph():
