@@ -101,15 +101,17 @@ __global__ void __launch_bounds__(kDensityThreads) density_kernel(
     density_one<DEBUG>(i, pos, cells, n, P, rho, aux, nbr4, nbr_count, dbg_count, xa, svel);
 }
 
-// Up to this many particles (excluded) the density pass takes nine lanes to one:
-// 4,096 particles are 16 blocks otherwise, and the pass is one lane's chain of ~100
-// candidates (a step 56 -> 34 us, 64 -> 42 where the fluid is compressed; 13,824:
-// 62 -> 47 and 70 -> 60; 21,952: 65 -> 58 and 73 -> 69).  At 32,768 the chip is
-// filled by one lane each: 66 -> 69 and 74 -> 75.
-constexpr uint32_t kDensitySplitMost = 24576;
+// Below this many particles the density pass takes nine lanes to one: 4,096
+// particles are 16 blocks otherwise, and the pass is one lane's chain of ~100
+// candidates.  Us per step alone, and of three solvers in turn, one lane and nine:
+// 4,096 particles 64 and 39, 25 and 17; 8,000 68 and 44, 27 and 20; 13,824 70 and
+// 52, 28 and 25; 21,952 72 and 62, but 29 and 34: nine lanes are more work, which
+// pays while the chip has room.
+constexpr uint32_t kDensitySplitMost = 16384;
 constexpr uint32_t kSplitLanes = 9, kSplitPer = 32 / kSplitLanes, kSplitWarps = 4;
-// Neighbours that a lane keeps: a lane has one row of three cells, which hold 27
-// where particles lie closest (with 32, 54 us at 4,096 where 40 take 42).
+// Neighbours that a lane keeps; one with more scans its share again, for the list
+// and for the sum.  A lane has one row of three cells, which hold 27 each where
+// particles lie closest: 39 us per step at 4,096 with 40, 43 with 24.
 constexpr uint32_t kSplitHits = 40;
 
 struct SplitScratch {  // of one warp
@@ -119,8 +121,8 @@ struct SplitScratch {  // of one warp
 
 // The density pass with nine lanes to a particle, each scanning its share of the
 // stencil's cell rows.  Lane 0 adds the terms in the scan's order, and the list is
-// written in it: the results are density_one's bit for bit.  A particle with a
-// lane whose neighbours the scratch does not hold is scanned by lane 0 alone.
+// written in it: the results are density_one's bit for bit.  The neighbours
+// of a lane that the scratch does not hold are found again.
 template <bool DEBUG>
 __global__ void __launch_bounds__(32 * kSplitWarps) density_split_kernel(
     const float4* __restrict__ pos, const uint2* __restrict__ cells, uint32_t n, SimParams P,
@@ -138,11 +140,12 @@ __global__ void __launch_bounds__(32 * kSplitWarps) density_split_kernel(
     const bool on = g < kSplitPer && i < n;
     const float4 xi = pos[min(i, n - 1u)];
     uint32_t hits = 0, listed = 0;
-    if (on) {
+    // f(j, r2) for the neighbours in lane l's share of the rows
+    auto scan = [&](uint32_t l, auto&& f) {
         const Stencil s = stencil(P.g, xi.x, xi.y, xi.z, P.h);
         const int ny = s.y1 - s.y0 + 1, rows = ny * (s.z1 - s.z0 + 1);
-        const int last = ((int)q + 1) * rows / (int)L;
-        for (int r = (int)q * rows / (int)L; r < last; ++r) {
+        const int last = ((int)l + 1) * rows / (int)L;
+        for (int r = (int)l * rows / (int)L; r < last; ++r) {
             const uint32_t row = linear_cell(P.g, 0, s.y0 + r % ny, s.z0 + r / ny);
             for (int cx = s.x0; cx <= s.x1; ++cx) {
                 const uint2 c = __ldg(&cells[row + cx]);
@@ -151,63 +154,73 @@ __global__ void __launch_bounds__(32 * kSplitWarps) density_split_kernel(
                     const float4 xj = __ldg(&pos[j]);
                     float dx, dy, dz;
                     const float r2 = dist2(xi.x, xi.y, xi.z, xj.x, xj.y, xj.z, dx, dy, dz);
-                    if (r2 < P.T) {
-                        if (hits < kSplitHits) {
-                            S.a[hits][lane] = P.h2 - r2;
-                            S.j[hits][lane] = r2 != 0.0f ? j : 0xFFFFFFFFu;  // not itself
-                        }
-                        ++hits;
-                        listed += r2 != 0.0f;
-                    }
+                    if (r2 < P.T) f(j, r2);
                 }
             }
         }
-    }
+    };
+    if (on)
+        scan(q, [&](uint32_t j, float r2) {
+            if (hits < kSplitHits) {
+                S.a[hits][lane] = P.h2 - r2;
+                S.j[hits][lane] = r2 != 0.0f ? j : 0xFFFFFFFFu;  // not itself
+            }
+            ++hits;
+            listed += r2 != 0.0f;
+        });
     __syncwarp();
-    // hits and listed neighbours of the group's earlier lanes (16 bits each: beyond
-    // the scratch the sums are not used)
-    const uint32_t own = (min(hits, 0xFFFu) << 16) | min(listed, 0xFFFu);
-    uint32_t at = own;
+    uint32_t at = listed, all = hits;
 #pragma unroll
     for (uint32_t d = 1; d < L; d <<= 1) {
-        const uint32_t y = __shfl_up_sync(kAll, at, d);
-        if (q >= d) at += y;
+        const uint32_t y = __shfl_up_sync(kAll, at, d), z = __shfl_up_sync(kAll, all, d);
+        if (q >= d) {
+            at += y;
+            all += z;
+        }
     }
-    const uint32_t total = __shfl_sync(kAll, at, (int)min(L * g + L - 1u, 31u));
-    const uint32_t over = __ballot_sync(kAll, hits > kSplitHits);
-    const bool alone = ((over >> min(L * g, 31u)) & ((1u << L) - 1u)) != 0u;
-    at -= own;
-    if (on && !alone) {
-        uint32_t k = at & 0xFFFFu;
+    const int end = (int)min(L * g + L - 1u, 31u);
+    const uint32_t total = __shfl_sync(kAll, at, end);
+    all = __shfl_sync(kAll, all, end);
+    at -= listed;
+    if (on) {
+        uint32_t k = at;
         uint32_t* out =
             reinterpret_cast<uint32_t*>(nbr4) + 4 * ((size_t)(k >> 2) * n + i) + (k & 3u);
         const uint32_t next_group = 4u * n - 3u;
-        for (uint32_t t = 0; t < hits; ++t) {
-            const uint32_t j = S.j[t][lane];
-            if (j != 0xFFFFFFFFu) {
-                if (k < (uint32_t)kMaxNbr) __stcs(out, j);
-                out += (k & 3u) == 3u ? next_group : 1u;
-                ++k;
-            }
+        auto put = [&](uint32_t j) {
+            if (k < (uint32_t)kMaxNbr) __stcs(out, j);
+            out += (k & 3u) == 3u ? next_group : 1u;
+            ++k;
+        };
+        if (hits <= kSplitHits) {
+            for (uint32_t t = 0; t < hits; ++t)
+                if (S.j[t][lane] != 0xFFFFFFFFu) put(S.j[t][lane]);
+        } else {
+            scan(q, [&](uint32_t j, float r2) {
+                if (r2 != 0.0f) put(j);
+            });
         }
     }
     float sum = 0.0f;
 #pragma unroll
     for (uint32_t l = 0; l < L; ++l) {
         const uint32_t from = min(L * g + l, 31u), m = __shfl_sync(kAll, hits, (int)from);
-        if (on && q == 0 && !alone) {
+        if (on && q == 0) {
+            if (m <= kSplitHits) {
 #pragma unroll 4
-            for (uint32_t t = 0; t < m; ++t) {
-                const float a = S.a[t][from];
-                sum = fmaf(a * a, a, sum);
+                for (uint32_t t = 0; t < m; ++t) {
+                    const float a = S.a[t][from];
+                    sum = fmaf(a * a, a, sum);
+                }
+            } else {
+                scan(l, [&](uint32_t, float r2) {
+                    const float a = P.h2 - r2;
+                    sum = fmaf(a * a, a, sum);
+                });
             }
         }
     }
     if (!on || q != 0) return;
-    if (alone) {
-        density_one<DEBUG>(i, pos, cells, n, P, rho, aux, nbr4, nbr_count, dbg_count, xa, svel);
-        return;
-    }
     const float rh = P.dens_coef * sum;
     const float p = P.bulk * (rh - P.rho0);
     const float inv = 1.0f / rh;
@@ -215,8 +228,8 @@ __global__ void __launch_bounds__(32 * kSplitWarps) density_split_kernel(
     aux[i] = make_float2(p * inv * inv, inv);
     xa[i] = make_float4(xi.x, xi.y, xi.z, p * inv * inv);
     reinterpret_cast<float*>(svel + i)[3] = inv;
-    nbr_count[i] = total & 0xFFFFu;
-    if (DEBUG) dbg_count[i] = total >> 16;
+    nbr_count[i] = total;
+    if (DEBUG) dbg_count[i] = all;
 }
 
 }  // namespace sph

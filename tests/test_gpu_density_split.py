@@ -1,4 +1,4 @@
-"""The density pass with several lanes to a particle (below 24,576 particles):
+"""The density pass with several lanes to a particle (below 16,384 particles):
 counts around a warp's three and a block's twelve particles and on both sides of
 the limit, and clusters that overflow a lane's share or the list, against the
 batched solver, which takes one lane to a particle.  Equal bit for bit."""
@@ -14,7 +14,7 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("n,cluster", [(1, 0), (2, 0), (3, 0), (4, 0), (11, 0), (12, 0), (13, 0),
                                        (2000, 39), (2000, 41), (2000, 95), (2000, 300),
-                                       (24575, 50), (24576, 50)])
+                                       (16383, 50), (16384, 50)])
 def test_split_density_equals_one_lane(n, cluster):
     sc = scenes.dam_break(1 / 64, (32, 32, 24))
     x = sc.fluid.positions[:n].copy()
