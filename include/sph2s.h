@@ -383,7 +383,7 @@ int sphb_counts(sph_batch* b, uint32_t* num_scenes, uint32_t* total_fluid,
  * sorted order or by the scene-local creation index; each pointer optional. */
 int sphb_get_scene(sph_batch* b, uint32_t scene, float* xyz, float* vel, float* rho,
                    int32_t order);
-/* Times block sizes 128/256/512 for the density and force passes and 2/4/8
+/* Times block sizes 128/256/512 for the density and force passes and 4/8/12
  * resident blocks per SM for the persistent grid on the batch's own data,
  * keeps the fastest (choice3 = density block, force block, blocks per SM),
  * and restores the particle state. */
