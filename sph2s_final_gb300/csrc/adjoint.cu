@@ -45,7 +45,7 @@ struct Rollout {
     float4* gb = nullptr;  // the boundary force's part of gx2
     float4* gxT = nullptr;
     float* grho = nullptr;
-    float* gmu_part = nullptr;
+    float* gmu_part = nullptr;  // [K][blocks]
     double* gmu_acc = nullptr;
     bool forward_done = false, have_loss = false;
     // The segment whose steps the tape holds (-1: none), and the constants they
@@ -113,7 +113,7 @@ int alloc_rollout(sph_solver* s, int T, int K, Rollout** out) {
         ((rc = ralloc(r, &r->gx, n)) || (rc = ralloc(r, &r->gv, n)) || (rc = ralloc(r, &r->gx2, n)) ||
          (rc = ralloc(r, &r->gv2, n)) || (rc = ralloc(r, &r->lam, n)) || (rc = ralloc(r, &r->gxT, n)) ||
          (rc = ralloc(r, &r->gb, n)) ||
-         (rc = ralloc(r, &r->grho, n)) || (rc = ralloc(r, &r->gmu_part, blocks)) ||
+         (rc = ralloc(r, &r->grho, n)) || (rc = ralloc(r, &r->gmu_part, (size_t)blocks * K)) ||
          (rc = ralloc(r, &r->gmu_acc, 1)) ||
          (nseg == 1 && ((rc = ralloc(r, &r->end_pos, n)) || (rc = ralloc(r, &r->end_vel, n)))))) {
     }
@@ -349,7 +349,8 @@ int sph_rollout_backward(sph_solver* s, float* grad_v0, float* grad_x0, double* 
             if (rc != SPH_OK) return rc;
         }
         for (int k = len - 1; k >= 0; --k) {  // reverse through the segment
-            adj_lambda_kernel<<<blocks, 256, 0, st>>>(r->gx, r->gv, r->aux[k], n, r->dt, r->lam);
+            if (k == len - 1)
+                adj_lambda_kernel<<<blocks, 256, 0, st>>>(r->gx, r->gv, r->aux[k], n, r->dt, r->lam);
             // the boundary force's adjoint beside that of the pair forces
             SPH_CUDA(cudaEventRecord(s->fork, st));
             SPH_CUDA(cudaStreamWaitEvent(s->side, s->fork, 0));
@@ -359,13 +360,16 @@ int sph_rollout_backward(sph_solver* s, float* grad_v0, float* grad_x0, double* 
             SPH_CUDA(cudaEventRecord(s->join, s->side));
             adj_force_kernel<<<blocks, 256, 0, st>>>(
                 r->xh[k], r->vh[k], r->rho[k], r->nbr[k], r->cnt[k], r->cells[k], n, s->P, r->mu,
-                r->dt, r->lam, r->gx, r->gv, r->gx2, r->gv2, r->grho, r->gmu_part);
-            adj_sum_kernel<<<1, 32, 0, st>>>(r->gmu_part, blocks, r->gmu_acc);
+                r->dt, r->lam, r->gx, r->gv, r->gx2, r->gv2, r->grho,
+                r->gmu_part + (size_t)k * blocks);
             SPH_CUDA(cudaStreamWaitEvent(st, s->join, 0));
+            const AdjScatter scatter = {r->perm[k], r->gv2, k ? r->aux[k - 1] : nullptr, r->dt,
+                                        r->gx, r->gv, r->lam};
             adj_density_kernel<<<blocks, 256, 0, st>>>(r->xh[k], r->nbr[k], r->cnt[k], r->cells[k],
-                                                       n, s->P, r->grho, r->gb, r->nflag[k], r->gx2);
-            adj_unpermute_kernel<<<blocks, 256, 0, st>>>(r->perm[k], n, r->gx2, r->gv2, r->gx, r->gv);
+                                                       n, s->P, r->grho, r->gb, r->nflag[k], r->gx2,
+                                                       scatter);
         }
+        adj_sum_kernel<<<1, 32, 0, st>>>(r->gmu_part, blocks, len, r->gmu_acc);
         SPH_CUDA(cudaGetLastError());
     }
     // gx, gv are now the adjoints of the creation-order initial state

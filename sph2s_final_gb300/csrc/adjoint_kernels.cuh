@@ -92,17 +92,20 @@ __device__ __forceinline__ void visit_force_neighbors(uint32_t i, const float4& 
 }
 
 // lam = dt (gv' + dt gx'), with A = p / rho^2 in w: beside the position and the
-// step's velocity (1 / rho in w) a neighbour's third and last gather.
+// step's velocity (1 / rho in w) a neighbour's third and last gather.  A segment's
+// last step starts from this kernel; the others from adj_scatter.
+__device__ __forceinline__ float4 adj_lambda(const float4& gx, const float4& gv, float A, float dt) {
+    return make_float4(dt * fmaf(dt, gx.x, gv.x), dt * fmaf(dt, gx.y, gv.y),
+                       dt * fmaf(dt, gx.z, gv.z), A);
+}
+
 static __global__ void __launch_bounds__(256) adj_lambda_kernel(const float4* __restrict__ gx,
                                                                 const float4* __restrict__ gv,
                                                                 const float2* __restrict__ aux,
                                                                 uint32_t n, float dt,
                                                                 float4* __restrict__ lam) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const float4 a = gx[i], b = gv[i];
-    lam[i] = make_float4(dt * fmaf(dt, a.x, b.x), dt * fmaf(dt, a.y, b.y), dt * fmaf(dt, a.z, b.z),
-                         aux[i].x);
+    if (i < n) lam[i] = adj_lambda(gx[i], gv[i], aux[i].x, dt);
 }
 
 struct AdjNeighbor {
@@ -320,14 +323,14 @@ struct AdjDensityPair {
 
 // Density adjoint, and the boundary force's part (gb, adj_boundary_lanes) where
 // near[i]: gx_i += gb_i - 6 m C6 sum_j (h^2 - r^2)^2 (grho_i + grho_j) x_ij.
-__device__ __forceinline__ void adj_density_one(uint32_t i, const float4* __restrict__ pos,
+__device__ __forceinline__ float4 adj_density_one(uint32_t i, const float4* __restrict__ pos,
                                                 const uint4* __restrict__ nbr4,
                                                 const uint32_t* __restrict__ nbr_count,
                                                 const uint2* __restrict__ cells, uint32_t n,
                                                 const SimParams& P, const float* __restrict__ grho,
                                                 const float4* __restrict__ gb,
                                                 const uint8_t* __restrict__ near,
-                                                float4* __restrict__ gx) {
+                                                const float4* __restrict__ gx) {
     const float4 xi = pos[i];
     AdjDensityPair A;
     A.gi = grho[i];
@@ -346,17 +349,40 @@ __device__ __forceinline__ void adj_density_one(uint32_t i, const float4* __rest
     g.x += A.gx;
     g.y += A.gy;
     g.z += A.gz;
-    gx[i] = g;
+    return g;
+}
+
+// Where a backward step ends: particle i's gradients go back to the order before
+// the step's sort, and there the earlier step's lambda (aux_prev, NULL: none in the
+// tape) is formed.  As kernels of their own the scatter and lambda took 4 us each
+// with their launches, of 57 per backward step at 65,536 particles.
+struct AdjScatter {
+    const uint32_t* perm;
+    const float4* gv;
+    const float2* aux_prev;
+    float dt;
+    float4 *gx_out, *gv_out, *lam;
+};
+
+__device__ __forceinline__ void adj_scatter(const AdjScatter& S, uint32_t i, uint32_t n,
+                                            const float4& gx) {
+    const uint32_t q = min(S.perm[i], n - 1);
+    const float4 gv = S.gv[i];
+    S.gx_out[q] = gx;
+    S.gv_out[q] = gv;
+    if (S.aux_prev) S.lam[q] = adj_lambda(gx, gv, S.aux_prev[q].x, S.dt);
 }
 
 static __global__ void __launch_bounds__(256) adj_density_kernel(
     const float4* __restrict__ pos, const uint4* __restrict__ nbr4,
     const uint32_t* __restrict__ nbr_count, const uint2* __restrict__ cells, uint32_t n,
     const __grid_constant__ SimParams P, const float* __restrict__ grho,
-    const float4* __restrict__ gb, const uint8_t* __restrict__ near, float4* __restrict__ gx) {
+    const float4* __restrict__ gb, const uint8_t* __restrict__ near, const float4* __restrict__ gx,
+    const AdjScatter scatter) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    adj_density_one(i, pos, nbr4, nbr_count, cells, n, P, grho, gb, near, gx);
+    adj_scatter(scatter, i, n,
+                adj_density_one(i, pos, nbr4, nbr_count, cells, n, P, grho, gb, near, gx));
 }
 
 // Scatter from the step's sorted order back to the order before the sort:
@@ -385,11 +411,13 @@ __device__ __forceinline__ double adj_sum_warp(const float* __restrict__ part, u
     return s;
 }
 
-// The per-block mu partials into acc (one warp).
-static __global__ void adj_sum_kernel(const float* __restrict__ part, uint32_t count,
+// The per-block mu partials of a segment's steps, the last first, into acc (one
+// warp).  Once per segment: per step it held the density adjoint up for 4 us.
+static __global__ void adj_sum_kernel(const float* __restrict__ part, uint32_t count, int steps,
                                       double* __restrict__ acc) {
-    const double s = adj_sum_warp(part, count);
-    if (threadIdx.x == 0) *acc += s;
+    double total = *acc;
+    for (int k = steps - 1; k >= 0; --k) total += adj_sum_warp(part + (size_t)k * count, count);
+    if (threadIdx.x == 0) *acc = total;
 }
 
 // Poly6 splat of the particles on the cell centres of a node grid:

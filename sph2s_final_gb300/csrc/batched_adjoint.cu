@@ -45,7 +45,7 @@ struct BRollout {
     float4* gb = nullptr;  // the boundary force's part of gx2
     float4* gxT = nullptr;
     float* grho = nullptr;
-    float* gmu_part = nullptr;  // one partial per 256-particle tile
+    float* gmu_part = nullptr;  // [K][tiles]: one partial per 256-particle tile
     double* gmu_acc = nullptr;  // per scene
     float* mu = nullptr;        // per scene
     uint32_t *tfirst = nullptr, *tcount = nullptr;
@@ -116,26 +116,30 @@ static __global__ void __launch_bounds__(kTile) b_adj_density_kernel(
     const uint2* __restrict__ tiles, uint32_t num_tiles, const SceneRec* __restrict__ recs,
     const float4* __restrict__ pos, const uint4* __restrict__ nbr4, const uint32_t* __restrict__ cnt,
     const uint2* __restrict__ cells, uint32_t n, const float* __restrict__ grho,
-    const float4* __restrict__ gb, const uint8_t* __restrict__ near, float4* __restrict__ gx) {
+    const float4* __restrict__ gb, const uint8_t* __restrict__ near, const float4* __restrict__ gx,
+    const AdjScatter scatter) {
     for (uint32_t t = blockIdx.x; t < num_tiles; t += gridDim.x) {
         const uint2 tile = tiles[t];
         const SceneRec& R = recs[tile.x];
         const uint32_t i = tile.y + threadIdx.x;
         if (i >= R.p_off + R.p_n) continue;
         const SimParams P = R.P;
-        adj_density_one(i, pos, nbr4, cnt, cells + R.c_off, n, P, grho, gb, near, gx);
+        adj_scatter(scatter, i, n,
+                    adj_density_one(i, pos, nbr4, cnt, cells + R.c_off, n, P, grho, gb, near, gx));
     }
 }
 
-// d L_s / d mu_s: the scene's tile partials by one warp (adj_sum_warp, the order of
-// the single-scale sum over its blocks).
+// d L_s / d mu_s: the scene's tile partials of a segment's steps by one warp, in the
+// order of the single-scale sum (adj_sum_kernel).
 static __global__ void __launch_bounds__(128) b_adj_sum_kernel(
-    const float* __restrict__ part, const uint32_t* __restrict__ first,
+    const float* __restrict__ part, uint32_t tiles, int steps, const uint32_t* __restrict__ first,
     const uint32_t* __restrict__ count, uint32_t S, double* __restrict__ acc) {
     const uint32_t s = blockIdx.x * 4 + (threadIdx.x >> 5);
     if (s >= S) return;
-    const double sum = adj_sum_warp(part + first[s], count[s]);
-    if ((threadIdx.x & 31u) == 0) acc[s] += sum;
+    double total = acc[s];
+    for (int k = steps - 1; k >= 0; --k)
+        total += adj_sum_warp(part + (size_t)k * tiles + first[s], count[s]);
+    if ((threadIdx.x & 31u) == 0) acc[s] = total;
 }
 
 // tiles[t] = (scene, first node of the tile within the scene's node grid)
@@ -222,7 +226,7 @@ int alloc_brollout(sph_batch* b, int T, int K, BRollout** out) {
         ((rc = ralloc(r, &r->gx, N)) || (rc = ralloc(r, &r->gv, N)) || (rc = ralloc(r, &r->gx2, N)) ||
          (rc = ralloc(r, &r->gv2, N)) || (rc = ralloc(r, &r->lam, N)) || (rc = ralloc(r, &r->gxT, N)) ||
          (rc = ralloc(r, &r->gb, N)) ||
-         (rc = ralloc(r, &r->grho, N)) || (rc = ralloc(r, &r->gmu_part, b->ntiles[1])) ||
+         (rc = ralloc(r, &r->grho, N)) || (rc = ralloc(r, &r->gmu_part, (size_t)b->ntiles[1] * K)) ||
          (rc = ralloc(r, &r->gmu_acc, b->S)) || (rc = ralloc(r, &r->mu, b->S)) ||
          (rc = ralloc(r, &r->tfirst, b->S)) || (rc = ralloc(r, &r->tcount, b->S)) ||
          (nseg == 1 && ((rc = ralloc(r, &r->end_pos, N)) || (rc = ralloc(r, &r->end_vel, N)))))) {
@@ -474,7 +478,8 @@ int sphb_rollout_backward(sph_batch* b, float* grad_v0, float* grad_x0, double* 
             if (rc != SPH_OK) return rc;
         }
         for (int k = len - 1; k >= 0; --k) {  // reverse through the segment
-            adj_lambda_kernel<<<blocks, kTile, 0, st>>>(r->gx, r->gv, r->aux[k], N, r->dt, r->lam);
+            if (k == len - 1)
+                adj_lambda_kernel<<<blocks, kTile, 0, st>>>(r->gx, r->gv, r->aux[k], N, r->dt, r->lam);
             // the boundary force's adjoint beside that of the pair forces
             SPH_CUDA(cudaEventRecord(b->fork, st));
             SPH_CUDA(cudaStreamWaitEvent(b->side, b->fork, 0));
@@ -487,15 +492,16 @@ int sphb_rollout_backward(sph_batch* b, float* grad_v0, float* grad_x0, double* 
             b_adj_force_kernel<<<grid, kTile, 0, st>>>(
                 b->tiles[1], nt, b->recs, r->mu, r->xh[k], r->vh[k], r->rho[k], r->nbr[k],
                 r->cnt[k], r->cells[k], N, r->dt, r->lam, r->gx, r->gv, r->gx2, r->gv2, r->grho,
-                r->gmu_part);
-            b_adj_sum_kernel<<<(b->S + 3) / 4, 128, 0, st>>>(r->gmu_part, r->tfirst, r->tcount,
-                                                            b->S, r->gmu_acc);
+                r->gmu_part + (size_t)k * nt);
             SPH_CUDA(cudaStreamWaitEvent(st, b->join, 0));
+            const AdjScatter scatter = {r->perm[k], r->gv2, k ? r->aux[k - 1] : nullptr, r->dt,
+                                        r->gx, r->gv, r->lam};
             b_adj_density_kernel<<<grid, kTile, 0, st>>>(b->tiles[1], nt, b->recs, r->xh[k],
                                                          r->nbr[k], r->cnt[k], r->cells[k], N,
-                                                         r->grho, r->gb, r->nflag[k], r->gx2);
-            adj_unpermute_kernel<<<blocks, kTile, 0, st>>>(r->perm[k], N, r->gx2, r->gv2, r->gx, r->gv);
+                                                         r->grho, r->gb, r->nflag[k], r->gx2, scatter);
         }
+        b_adj_sum_kernel<<<(b->S + 3) / 4, 128, 0, st>>>(r->gmu_part, nt, len, r->tfirst, r->tcount,
+                                                        b->S, r->gmu_acc);
         SPH_CUDA(cudaGetLastError());
     }
     std::vector<float4> hg(N);
