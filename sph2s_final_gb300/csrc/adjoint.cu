@@ -176,6 +176,7 @@ int record_segment(sph_solver* s, int len) {
 // left: densities and cell table are copied out of the last step's record.
 int advance_recorded(sph_solver* s, int seg, int len) {
     Rollout* r = s->rollout;
+    if (!std::isfinite(r->dt)) return fail(SPH_E_INVALID, "sph_rollout_forward: bad dt");
     int rc = record_segment(s, len);
     if (rc != SPH_OK) return rc;
     SPH_CUDA(cudaMemcpyAsync(s->rho, r->rho[len - 1], 4 * (size_t)s->n, cudaMemcpyDeviceToDevice,

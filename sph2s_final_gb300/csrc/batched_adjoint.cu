@@ -295,6 +295,7 @@ int record_segment(sph_batch* b, int len) {
 int advance_recorded(sph_batch* b, int seg, int len) {
     BRollout* r = b->rollout;
     const size_t N = b->N;
+    if (!std::isfinite(r->dt)) return fail(SPH_E_INVALID, "sphb_rollout_forward: bad dt");
     int rc = record_segment(b, len);
     if (rc != SPH_OK) return rc;
     SPH_CUDA(cudaMemcpyAsync(b->rho, r->rho[len - 1], 4 * N, cudaMemcpyDeviceToDevice, b->stream));
