@@ -463,6 +463,9 @@ int sphb_get_scene(sph_batch* b, uint32_t scene, float* xyz, float* vel, float* 
     const size_t n = R.p_n;
     const size_t floats = n * ((xyz ? 3 : 0) + (vel ? 3 : 0) + (rho ? 1 : 0));
     if (!floats) return sphb_sync(b);
+    // several threads may read a batch: the pack and pinned buffers are one reader's
+    // from its first launch to its last copy
+    const std::lock_guard<std::mutex> one_reader(b->reading);
     constexpr size_t kChunk = 4u << 20;
     for (int k = 0; k < 2; ++k) {
         if (!b->pinned[k]) SPH_CUDA(cudaMallocHost((void**)&b->pinned[k], kChunk));

@@ -2,6 +2,7 @@
 // (batched.cu) and the batched differentiable rollout (batched_adjoint.cu).
 #pragma once
 #include <cuda_runtime.h>
+#include <mutex>
 #include <vector>
 #include "../../include/sph2s.h"
 #include "batched_kernels.cuh"
@@ -68,7 +69,8 @@ struct sph_batch {
     float4* pos0 = nullptr;           // creation positions, packed by scene (rollout restarts)
     std::vector<uint32_t> tile_first; // first 256-particle tile of each scene in tiles[1]
     // readback of a scene: packed on the device, copied out through two pinned
-    // buffers (allocated on first use)
+    // buffers (allocated on first use); one reader at a time
+    std::mutex reading;
     float* pack = nullptr;
     size_t pack_floats = 0;
     char* pinned[2] = {nullptr, nullptr};
