@@ -29,6 +29,21 @@ int dalloc(T** p, size_t count, std::vector<void*>& owned) {
     return SPH_OK;
 }
 
+// Makes a device the calling thread's current one for a scope.
+struct OnDevice {
+    explicit OnDevice(int device) {
+        err = cudaGetDevice(&before);
+        moved = err == cudaSuccess && device != before;
+        if (moved) err = cudaSetDevice(device);
+    }
+    ~OnDevice() {
+        if (moved) cudaSetDevice(before);
+    }
+    cudaError_t err = cudaSuccess;
+    int before = 0;
+    bool moved = false;
+};
+
 }  // namespace
 
 namespace sph_b {
@@ -236,9 +251,8 @@ int sphb_create(const sph_scene_desc* scenes, uint32_t num_scenes, sph_batch** o
             return fail(_r, m);               \
         }                                     \
     } while (0)
-    int dev = 0;
-    TRY(check_cuda(cudaGetDevice(&dev), "device", __FILE__, __LINE__));
-    TRY(check_cuda(cudaDeviceGetAttribute(&b->sms, cudaDevAttrMultiProcessorCount, dev), "attr", __FILE__, __LINE__));
+    TRY(check_cuda(cudaGetDevice(&b->device), "device", __FILE__, __LINE__));
+    TRY(check_cuda(cudaDeviceGetAttribute(&b->sms, cudaDevAttrMultiProcessorCount, b->device), "attr", __FILE__, __LINE__));
     TRY(check_cuda(cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking), "stream", __FILE__, __LINE__));
     TRY(check_cuda(cudaStreamCreateWithFlags(&b->side, cudaStreamNonBlocking), "stream", __FILE__, __LINE__));
     TRY(check_cuda(cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming), "event", __FILE__, __LINE__));
@@ -466,6 +480,10 @@ int sphb_get_scene(sph_batch* b, uint32_t scene, float* xyz, float* vel, float* 
     // several threads may read a batch: the pack and pinned buffers are one reader's
     // from its first launch to its last copy
     const std::lock_guard<std::mutex> one_reader(b->reading);
+    // the copies alone worked from a thread whose current device is another (a new
+    // thread's is device 0); the pack kernel, the events and the allocations do not
+    const OnDevice here(b->device);
+    SPH_CUDA(here.err);
     constexpr size_t kChunk = 4u << 20;
     for (int k = 0; k < 2; ++k) {
         if (!b->pinned[k]) SPH_CUDA(cudaMallocHost((void**)&b->pinned[k], kChunk));

@@ -62,6 +62,7 @@ struct sph_batch {
     // 572, 12 525 / 543 / 558, one tile per block 552 / 574 / 595).
     int grid_mult = 12;
     int sms = 152;
+    int device = 0;  // the handle's GPU
     cudaGraphExec_t graph = nullptr;
     float graph_dt = 0.0f;
     std::vector<void*> owned;
