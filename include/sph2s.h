@@ -206,6 +206,12 @@ int sph_debug_force_lookback_timeout(sph_solver* s, int32_t on);
  * since the last step are radix-sorted, the rest merged around them). */
 int sph_debug_sort_mode(sph_solver* s, int32_t mode);
 
+/* Test hook setting how many entries the handle's neighbour lists have (4, 8, ...
+ * 96): 96, or fewer where the device memory does not hold them.  A particle with
+ * more neighbours finds them again, with the same result.  Drops the handle's
+ * rollout, whose tape has lists of as many entries at most. */
+int sph_debug_list_capacity(sph_solver* s, uint32_t entries);
+
 /* ---- differentiable rollout (no counterpart in the reference) ------------ */
 
 /* Restarts the solver from its creation positions with initial velocities
@@ -330,6 +336,8 @@ int sph2_get_states_device(sph_solver2* s, int32_t population, int32_t* d_state)
 int sph2_debug_step_fields(sph_solver2* s, int32_t population, uint32_t* ids_sorted, float* rho,
                            float* acc, uint32_t* nbr_same, uint32_t* nbr_compl,
                            uint32_t* nbr_boundary);
+/* sph_debug_list_capacity for the same-population lists. */
+int sph2_debug_list_capacity(sph_solver2* s, uint32_t entries);
 int sph2_destroy(sph_solver2* s);
 /* Colour / energy output of the two-scale force pass (dColorValues,
  * SPH2S_FINAL_TWO_SCALE/Solver.cu:206-213, 378-387, 897-907, 1050-1070): per
@@ -388,6 +396,7 @@ int sphb_get_scene(sph_batch* b, uint32_t scene, float* xyz, float* vel, float* 
  * keeps the fastest (choice3 = density block, force block, blocks per SM),
  * and restores the particle state. */
 int sphb_autotune(sph_batch* b, float dt, int32_t* choice3);
+int sphb_debug_list_capacity(sph_batch* b, uint32_t entries); /* as sph_debug_list_capacity */
 int sphb_destroy(sph_batch* b);
 
 /* Batched differentiable rollout (no counterpart in the reference): the

@@ -117,6 +117,9 @@ SIGNATURES = {
     "sph_profile_phases": (C.c_int, [_vp, C.c_float, C.c_int32, _f]),
     "sph_debug_force_lookback_timeout": (C.c_int, [_vp, C.c_int32]),
     "sph_debug_sort_mode": (C.c_int, [_vp, C.c_int32]),
+    "sph_debug_list_capacity": (C.c_int, [_vp, C.c_uint32]),
+    "sph2_debug_list_capacity": (C.c_int, [_vp, C.c_uint32]),
+    "sphb_debug_list_capacity": (C.c_int, [_vp, C.c_uint32]),
     "sph_rollout_forward": (C.c_int, [_vp, _f, C.c_float, C.c_float, C.c_int32, C.c_int32]),
     "sph_rollout_density_loss": (C.c_int, [_vp, C.POINTER(sph_grid), _f, _f,
                                            C.POINTER(C.c_double)]),

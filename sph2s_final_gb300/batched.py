@@ -68,6 +68,10 @@ class Batch:
         check(lib().sphb_autotune(self._h, C.c_float(dt), c))
         return {"density_block": c[0], "force_block": c[1], "blocks_per_sm": c[2]}
 
+    def debug_list_capacity(self, entries: int) -> None:
+        """Test hook: entries of the neighbour lists (4, 8, ... 96); same results."""
+        check(lib().sphb_debug_list_capacity(self._h, int(entries)))
+
     # ---- batched differentiable rollout (every scene at once) ----
     def _split(self, packed, width):
         out, o = [], 0

@@ -35,7 +35,8 @@ struct Rollout {
     std::vector<float4*> xh, vh;
     std::vector<float*> rho;
     std::vector<float2*> aux;
-    std::vector<uint4*> nbr;
+    std::vector<uint4*> nbr;  // list_cap entries each
+    uint32_t list_cap = kMaxNbr;
     std::vector<uint32_t*> cnt;
     std::vector<uint2*> cells;
     std::vector<uint32_t*> nlist;   // near-boundary particles, their number and flags
@@ -73,8 +74,9 @@ void free_rollout(Rollout* r) {
     delete r;
 }
 
-int alloc_rollout(sph_solver* s, int T, int K, Rollout** out) {
+int alloc_rollout(sph_solver* s, int T, int K, uint32_t list_cap, Rollout** out) {
     Rollout* r = new Rollout();
+    r->list_cap = list_cap;
     r->T = T;
     r->K = K;
     r->n = s->n;
@@ -102,7 +104,7 @@ int alloc_rollout(sph_solver* s, int T, int K, Rollout** out) {
     for (int k = 0; k < K && rc == SPH_OK; ++k) {
         if ((rc = ralloc(r, &r->perm[k], n)) || (rc = ralloc(r, &r->xh[k], n)) ||
             (rc = ralloc(r, &r->vh[k], n)) || (rc = ralloc(r, &r->rho[k], n)) ||
-            (rc = ralloc(r, &r->aux[k], n)) || (rc = ralloc(r, &r->nbr[k], (size_t)n * (kMaxNbr / 4))) ||
+            (rc = ralloc(r, &r->aux[k], n)) || (rc = ralloc(r, &r->nbr[k], (size_t)n * (list_cap / 4))) ||
             (rc = ralloc(r, &r->cnt[k], n)) || (rc = ralloc(r, &r->cells[k], s->ncells)) ||
             (rc = ralloc(r, &r->nlist[k], n)) || (rc = ralloc(r, &r->ncount[k], 1)) ||
             (rc = ralloc(r, &r->nflag[k], n)))
@@ -135,6 +137,8 @@ int record_segment(sph_solver* s, int len) {
     float2* aux0 = s->aux;
     uint4* nbr0 = s->nbr;
     uint32_t* cnt0 = s->nbr_count;
+    const uint32_t cap0 = s->list_cap;
+    s->list_cap = r->list_cap;
     uint2* cells0 = s->cells;
     uint32_t* blist0 = s->blist;
     uint32_t* bcount0 = s->bcount;
@@ -163,6 +167,7 @@ int record_segment(sph_solver* s, int len) {
     s->aux = aux0;
     s->nbr = nbr0;
     s->nbr_count = cnt0;
+    s->list_cap = cap0;
     s->blist = blist0;
     s->bcount = bcount0;
     s->bflag = bflag0;
@@ -243,7 +248,9 @@ int sph_rollout_forward(sph_solver* s, const float* v0_xyz, float viscosity, flo
     const int K = checkpoint_every > steps ? steps : checkpoint_every;
     if (s->rollout && (s->rollout->T != steps || s->rollout->K != K)) sph_rollout_release(s);
     if (!s->rollout) {
-        int rc = alloc_rollout(s, steps, K, &s->rollout);
+        const int rc = with_list_capacity((uint64_t)s->n * K, s->list_cap, [&](uint32_t list_cap) {
+            return alloc_rollout(s, steps, K, list_cap, &s->rollout);
+        });
         if (rc != SPH_OK) return rc;
     }
     Rollout* r = s->rollout;

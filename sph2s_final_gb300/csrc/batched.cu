@@ -55,6 +55,7 @@ int free_batch(sph_batch* b) {
     sphb_rollout_release(b);
     if (b->graph) cudaGraphExecDestroy(b->graph);
     for (void* p : b->owned) cudaFree(p);
+    if (b->nbr) cudaFree(b->nbr);
     if (b->pack) cudaFree(b->pack);
     for (int k = 0; k < 2; ++k) {
         if (b->pinned[k]) cudaFreeHost(b->pinned[k]);
@@ -86,9 +87,11 @@ uint32_t pgrid(const sph_batch* b, uint32_t tiles) {
 
 template <int BS>
 void launch_density(sph_batch* b, int ti) {
-    launch_after(b_density_kernel<BS>, pgrid(b, b->ntiles[ti]), BS, b->stream, b->tiles[ti],
-                 b->ntiles[ti], b->recs, b->spos, b->cells, b->N, b->rho, b->aux, b->nbr,
-                 b->nbr_count, b->xa, b->svel);
+    with_lists(b->list_cap, [&](auto lists) {
+        launch_after(b_density_kernel<BS, decltype(lists)>, pgrid(b, b->ntiles[ti]), BS, b->stream,
+                     b->tiles[ti], b->ntiles[ti], b->recs, b->spos, b->cells, b->N, b->rho, b->aux,
+                     b->nbr, b->nbr_count, lists, b->xa, b->svel);
+    });
 }
 
 template <int BS>
@@ -196,13 +199,12 @@ int check_err(sph_batch* b) {
 
 using namespace sph_b;
 
-extern "C" {
+namespace {
 
-int sphb_create(const sph_scene_desc* scenes, uint32_t num_scenes, sph_batch** out) {
-    if (!scenes || !out || num_scenes == 0)
-        return fail(SPH_E_INVALID, "sphb_create: need at least one scene and an output handle");
-    *out = nullptr;
+int create_with_lists(const sph_scene_desc* scenes, uint32_t num_scenes, uint32_t list_cap,
+                      sph_batch** out) {
     sph_batch* b = new sph_batch();
+    b->list_cap = list_cap;
     b->S = num_scenes;
     uint64_t N = 0, NB = 0, NC = 0;
     int maxbits = 1;
@@ -266,7 +268,7 @@ int sphb_create(const sph_scene_desc* scenes, uint32_t num_scenes, sph_batch** o
     TRY(dalloc(&b->rho, b->N, b->owned));
     TRY(dalloc(&b->aux, b->N, b->owned));
     TRY(dalloc(&b->xa, b->N, b->owned));
-    TRY(dalloc(&b->nbr, (size_t)b->N * (kMaxNbr / 4), b->owned));
+    TRY(check_cuda(cudaMalloc(&b->nbr, 4 * (size_t)list_cap * std::max(b->N, 1u)), "lists", __FILE__, __LINE__));
     TRY(dalloc(&b->nbr_count, b->N, b->owned));
     for (int k = 0; k < 2; ++k) {
         TRY(dalloc(&b->keys[k], nmax, b->owned));
@@ -418,6 +420,39 @@ int sphb_create(const sph_scene_desc* scenes, uint32_t num_scenes, sph_batch** o
     TRY(check_err(b));
 #undef TRY
     *out = b;
+    return SPH_OK;
+}
+
+}  // namespace
+
+extern "C" {
+
+int sphb_create(const sph_scene_desc* scenes, uint32_t num_scenes, sph_batch** out) {
+    if (!scenes || !out || num_scenes == 0)
+        return fail(SPH_E_INVALID, "sphb_create: need at least one scene and an output handle");
+    *out = nullptr;
+    uint64_t n = 0;
+    for (uint32_t s = 0; s < num_scenes; ++s) n += scenes[s].n_fluid;
+    return with_list_capacity(n, kMaxNbr, [&](uint32_t list_cap) {
+        return create_with_lists(scenes, num_scenes, list_cap, out);
+    });
+}
+
+int sphb_debug_list_capacity(sph_batch* b, uint32_t entries) {
+    if (!b) return fail(SPH_E_INVALID, "NULL handle");
+    const int rc = check_list_capacity(entries, "sphb_debug_list_capacity");
+    if (rc != SPH_OK) return rc;
+    SPH_CUDA(cudaStreamSynchronize(b->stream));
+    sphb_rollout_release(b);
+    if (b->graph) {
+        cudaGraphExecDestroy(b->graph);
+        b->graph = nullptr;
+    }
+    uint4* lists = nullptr;
+    SPH_CUDA(cudaMalloc(&lists, 4 * (size_t)entries * std::max(b->N, 1u)));
+    cudaFree(b->nbr);
+    b->nbr = lists;
+    b->list_cap = entries;
     return SPH_OK;
 }
 

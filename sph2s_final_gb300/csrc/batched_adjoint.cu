@@ -35,7 +35,8 @@ struct BRollout {
     std::vector<float4*> xh, vh;
     std::vector<float*> rho;
     std::vector<float2*> aux;
-    std::vector<uint4*> nbr;
+    std::vector<uint4*> nbr;  // list_cap entries each
+    uint32_t list_cap = kMaxNbr;
     std::vector<uint32_t*> cnt;
     std::vector<uint2*> cells;
     std::vector<uint2*> nlist;   // near-boundary particles, their number and flags
@@ -188,8 +189,9 @@ void free_brollout(BRollout* r) {
     delete r;
 }
 
-int alloc_brollout(sph_batch* b, int T, int K, BRollout** out) {
+int alloc_brollout(sph_batch* b, int T, int K, uint32_t list_cap, BRollout** out) {
     BRollout* r = new BRollout();
+    r->list_cap = list_cap;
     r->T = T;
     r->K = K;
     const uint32_t N = b->N;
@@ -216,7 +218,7 @@ int alloc_brollout(sph_batch* b, int T, int K, BRollout** out) {
         if ((rc = ralloc(r, &r->perm[k], N)) || (rc = ralloc(r, &r->xh[k], N)) ||
             (rc = ralloc(r, &r->vh[k], N)) || (rc = ralloc(r, &r->rho[k], N)) ||
             (rc = ralloc(r, &r->aux[k], N)) ||
-            (rc = ralloc(r, &r->nbr[k], (size_t)N * (kMaxNbr / 4))) ||
+            (rc = ralloc(r, &r->nbr[k], (size_t)N * (list_cap / 4))) ||
             (rc = ralloc(r, &r->cnt[k], N)) || (rc = ralloc(r, &r->cells[k], b->NC)) ||
             (rc = ralloc(r, &r->nlist[k], N)) || (rc = ralloc(r, &r->ncount[k], 1)) ||
             (rc = ralloc(r, &r->nflag[k], N)))
@@ -255,6 +257,8 @@ int record_segment(sph_batch* b, int len) {
     float2* aux0 = b->aux;
     uint4* nbr0 = b->nbr;
     uint32_t* cnt0 = b->nbr_count;
+    const uint32_t cap0 = b->list_cap;
+    b->list_cap = r->list_cap;
     uint2* cells0 = b->cells;
     uint2* blist0 = b->blist;
     uint32_t* bcount0 = b->bcount;
@@ -283,6 +287,7 @@ int record_segment(sph_batch* b, int len) {
     b->aux = aux0;
     b->nbr = nbr0;
     b->nbr_count = cnt0;
+    b->list_cap = cap0;
     b->blist = blist0;
     b->bcount = bcount0;
     b->bflag = bflag0;
@@ -334,7 +339,9 @@ int sphb_rollout_forward(sph_batch* b, const float* v0_xyz, const float* viscosi
     const int K = checkpoint_every > steps ? steps : checkpoint_every;
     if (b->rollout && (b->rollout->T != steps || b->rollout->K != K)) sphb_rollout_release(b);
     if (!b->rollout) {
-        int rc = alloc_brollout(b, steps, K, &b->rollout);
+        const int rc = with_list_capacity((uint64_t)b->N * K, b->list_cap, [&](uint32_t list_cap) {
+            return alloc_brollout(b, steps, K, list_cap, &b->rollout);
+        });
         if (rc != SPH_OK) return rc;
     }
     BRollout* r = b->rollout;

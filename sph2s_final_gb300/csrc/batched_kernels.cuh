@@ -147,12 +147,13 @@ __global__ void __launch_bounds__(BS) b_gather_cells_kernel(
     }
 }
 
-template <int BS>
+template <int BS, class LISTS>
 __global__ void __launch_bounds__(BS) b_density_kernel(
     const uint2* __restrict__ tiles, uint32_t num_tiles, const SceneRec* __restrict__ recs,
     const float4* __restrict__ pos, const uint2* __restrict__ cells, uint32_t n,
     float* __restrict__ rho, float2* __restrict__ aux, uint4* __restrict__ nbr4,
-    uint32_t* __restrict__ nbr_count, float4* __restrict__ xa, float4* __restrict__ svel) {
+    uint32_t* __restrict__ nbr_count, LISTS lists, float4* __restrict__ xa,
+    float4* __restrict__ svel) {
     grid_wait();
     for (uint32_t t = blockIdx.x; t < num_tiles; t += gridDim.x) {
         const uint2 tile = tiles[t];
@@ -160,8 +161,8 @@ __global__ void __launch_bounds__(BS) b_density_kernel(
         const uint32_t i = after_wait(tile.y + threadIdx.x);
         if (i >= R.p_off + R.p_n) continue;
         const SimParams P = R.P;
-        density_one<false>(i, pos, cells + R.c_off, n, P, rho, aux, nbr4, nbr_count, nullptr, xa,
-                           svel);
+        density_one<false>(i, pos, cells + R.c_off, n, P, rho, aux, nbr4, nbr_count, lists, nullptr,
+                           xa, svel);
     }
 }
 

@@ -28,7 +28,8 @@ struct sph_batch {
     float* rho = nullptr;
     float2* aux = nullptr;
     float4* xa = nullptr;  // force-pass records (x, p/rho^2), written by the density pass
-    uint4* nbr = nullptr;
+    uint4* nbr = nullptr;  // neighbour lists, list_cap per particle
+    uint32_t list_cap = sph::kMaxNbr;
     uint32_t* nbr_count = nullptr;
     uint32_t* keys[2] = {nullptr, nullptr};
     uint32_t* vals[2] = {nullptr, nullptr};

@@ -18,8 +18,8 @@
 // stored and loaded with streaming (evict-first) cache hints, so it displaces
 // less of the force records the force pass gathers from L2 (2M step
 // 0.837 -> 0.830 ms).
-// nbr_count[i] may exceed kMaxNbr; the force pass then
-// rescans the stencil for that particle.
+// A count beyond the list (above kMaxNbr) has the force pass rescan the stencil for
+// that particle.
 //
 // One thread per particle, particles in Morton order (a warp's particles
 // share most of their stencil cells, so candidate loads hit in L1).  Measured
@@ -39,12 +39,12 @@ constexpr int kDensityThreads = 256;
 // Density of particle i of the sorted array (n particles, indices in `cells`
 // refer to that array); the batched solver calls this with per-scene P and
 // cell table.
-template <bool DEBUG>
+template <bool DEBUG, class LISTS>
 __device__ __forceinline__ void density_one(uint32_t i, const float4* __restrict__ pos,
                                             const uint2* __restrict__ cells, uint32_t n,
                                             const SimParams& P, float* __restrict__ rho,
                                             float2* __restrict__ aux, uint4* __restrict__ nbr4,
-                                            uint32_t* __restrict__ nbr_count,
+                                            uint32_t* __restrict__ nbr_count, LISTS lists,
                                             uint32_t* __restrict__ dbg_count,
                                             float4* __restrict__ xa, float4* __restrict__ svel) {
     uint32_t k = 0, zero = 0;
@@ -68,7 +68,7 @@ __device__ __forceinline__ void density_one(uint32_t i, const float4* __restrict
                         const float a = P.h2 - r2;
                         sum = fmaf(a * a, a, sum);
                         if (r2 != 0.0f) {
-                            if (k < (uint32_t)kMaxNbr) __stcs(out, j);  // evict-first
+                            if (lists.holds(k)) __stcs(out, j);  // evict-first
                             out += (k & 3u) == 3u ? next_group : 1u;
                             ++k;
                         } else {
@@ -85,20 +85,20 @@ __device__ __forceinline__ void density_one(uint32_t i, const float4* __restrict
     aux[i] = make_float2(p * inv * inv, inv);
     xa[i] = make_float4(xi.x, xi.y, xi.z, p * inv * inv);
     reinterpret_cast<float*>(svel + i)[3] = inv;
-    nbr_count[i] = k;
+    nbr_count[i] = lists.count(k);
     if (DEBUG) dbg_count[i] = k + zero;
 }
 
-template <bool DEBUG>
+template <bool DEBUG, class LISTS>
 __global__ void __launch_bounds__(kDensityThreads) density_kernel(
     const float4* __restrict__ pos, const uint2* __restrict__ cells, uint32_t n, SimParams P,
     float* __restrict__ rho, float2* __restrict__ aux, uint4* __restrict__ nbr4,
-    uint32_t* __restrict__ nbr_count, uint32_t* __restrict__ dbg_count, float4* __restrict__ xa,
-    float4* __restrict__ svel) {
+    uint32_t* __restrict__ nbr_count, LISTS lists, uint32_t* __restrict__ dbg_count,
+    float4* __restrict__ xa, float4* __restrict__ svel) {
     grid_wait();
     const uint32_t i = after_wait(blockIdx.x * blockDim.x + threadIdx.x);
     if (i >= n) return;
-    density_one<DEBUG>(i, pos, cells, n, P, rho, aux, nbr4, nbr_count, dbg_count, xa, svel);
+    density_one<DEBUG>(i, pos, cells, n, P, rho, aux, nbr4, nbr_count, lists, dbg_count, xa, svel);
 }
 
 // Below this many particles the density pass takes nine lanes to one: 4,096
@@ -123,12 +123,12 @@ struct SplitScratch {  // of one warp
 // stencil's cell rows.  Lane 0 adds the terms in the scan's order, and the list is
 // written in it: the results are density_one's bit for bit.  The neighbours
 // of a lane that the scratch does not hold are found again.
-template <bool DEBUG>
+template <bool DEBUG, class LISTS>
 __global__ void __launch_bounds__(32 * kSplitWarps) density_split_kernel(
     const float4* __restrict__ pos, const uint2* __restrict__ cells, uint32_t n, SimParams P,
     float* __restrict__ rho, float2* __restrict__ aux, uint4* __restrict__ nbr4,
-    uint32_t* __restrict__ nbr_count, uint32_t* __restrict__ dbg_count, float4* __restrict__ xa,
-    float4* __restrict__ svel) {
+    uint32_t* __restrict__ nbr_count, LISTS lists, uint32_t* __restrict__ dbg_count,
+    float4* __restrict__ xa, float4* __restrict__ svel) {
     constexpr uint32_t kAll = 0xFFFFFFFFu, L = kSplitLanes;
     __shared__ SplitScratch scratch[kSplitWarps];
     SplitScratch& S = scratch[threadIdx.x >> 5];
@@ -188,7 +188,7 @@ __global__ void __launch_bounds__(32 * kSplitWarps) density_split_kernel(
             reinterpret_cast<uint32_t*>(nbr4) + 4 * ((size_t)(k >> 2) * n + i) + (k & 3u);
         const uint32_t next_group = 4u * n - 3u;
         auto put = [&](uint32_t j) {
-            if (k < (uint32_t)kMaxNbr) __stcs(out, j);
+            if (lists.holds(k)) __stcs(out, j);
             out += (k & 3u) == 3u ? next_group : 1u;
             ++k;
         };
@@ -228,7 +228,7 @@ __global__ void __launch_bounds__(32 * kSplitWarps) density_split_kernel(
     aux[i] = make_float2(p * inv * inv, inv);
     xa[i] = make_float4(xi.x, xi.y, xi.z, p * inv * inv);
     reinterpret_cast<float*>(svel + i)[3] = inv;
-    nbr_count[i] = total;
+    nbr_count[i] = lists.count(total);
     if (DEBUG) dbg_count[i] = all;
 }
 

@@ -9,6 +9,7 @@
 namespace sph {
 
 thread_local std::string g_last_error;
+thread_local cudaError_t g_last_cuda = cudaSuccess;
 const double kPi = 3.14159265358979323846;  // M_PI, SPH2S_FINAL_SINGLE_SCALE/Solver.h:11
 
 void set_last_error(const std::string& msg) { g_last_error = msg; }
@@ -24,9 +25,12 @@ int check_cuda(cudaError_t e, const char* what, const char* file, int line) {
     std::snprintf(buf, sizeof(buf), "CUDA error %d (%s) in %s at %s:%d", (int)e,
                   cudaGetErrorString(e), what, file, line);
     g_last_error = buf;
+    g_last_cuda = e;
     cudaGetLastError();  // clear the sticky-free error so later calls can proceed
     return SPH_E_CUDA;
 }
+
+bool out_of_memory() { return g_last_cuda == cudaErrorMemoryAllocation; }
 
 int check_device_pointer(const void* p, const char* who) {
     cudaPointerAttributes a;

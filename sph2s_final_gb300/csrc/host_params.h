@@ -75,6 +75,37 @@ inline int boundary_depth_bits(const GridParams& p, float h, int key_bits) {
     return std::max(0, std::min(8, 32 - key_bits));
 }
 
+// Calls make(entries), which allocates neighbour lists of that many entries for
+// `lists` particles (or particle-steps of a tape), with at most `most`: kMaxNbr, or
+// fewer where the memory does not hold them (the results are the same: a particle
+// whose list is too short rescans).  A scene of hundreds of millions of particles, or
+// a long tape, fits with 64 or less and would not with 96: 384 of the ~600 bytes that
+// a handle takes per particle, and of the ~440 of a tape per particle and step.  Lists
+// beyond a quarter of the free memory start at 64, which leaves a program's other
+// handles and buffers their room.
+template <class F>
+int with_list_capacity(uint64_t lists, uint32_t most, F&& make) {
+    constexpr uint32_t entries[] = {(uint32_t)kMaxNbr, 64, 48, 32, 16};
+    constexpr uint64_t kAsk = 1u << 22;  // 1.6 GB of lists: from here on the memory is asked for
+    if (lists >= kAsk) {
+        size_t available = 0, total = 0;
+        const int rc = check_cuda(cudaMemGetInfo(&available, &total), "memory", __FILE__, __LINE__);
+        if (rc != SPH_OK) return rc;
+        if (lists * (4u * kMaxNbr) > available / 4) most = most < 64 ? most : 64;
+    }
+    int rc = make(most);
+    for (uint32_t e : entries)
+        if (e < most && rc == SPH_E_CUDA && out_of_memory()) rc = make(e);
+    return rc;
+}
+
+// The entries that a test may ask for (sph_debug_list_capacity).
+inline int check_list_capacity(uint32_t entries, const char* who) {
+    if (entries < 4 || entries > (uint32_t)kMaxNbr || entries % 4)
+        return fail(SPH_E_INVALID, std::string(who) + ": entries must be 4, 8, ... 96");
+    return SPH_OK;
+}
+
 inline int make_sim_params(const sph_config& c, SimParams* out) {
     int rc = validate_grid(c.grid, "sph_config");
     if (rc != SPH_OK) return rc;

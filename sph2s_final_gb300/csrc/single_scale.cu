@@ -110,22 +110,25 @@ void enqueue_density(sph_solver* s, uint32_t* xall) {
                                                       s->bcand, s->blist, s->bcount, s->n, s->nb,
                                                       s->P, s->bacc);
     cudaEventRecord(s->join, s->side);
-    const auto kernel = xall ? density_kernel<true> : density_kernel<false>;
-    if (s->n < kDensitySplitMost) {
-        launch_after(xall ? density_split_kernel<true> : density_split_kernel<false>,
-                     blocks_for(s->n, kSplitWarps * kSplitPer), 32 * kSplitWarps, s->stream, s->spos,
-                     s->cells, s->n, s->P, s->rho, s->aux, s->nbr, s->nbr_count, xall, s->xa,
-                     s->svel);
-        return;
-    }
-    const uint32_t blocks = blocks_for(s->n, kDensityThreads);
-    if (s->n < kDensityAfterMost)
-        launch_after(kernel, blocks, kDensityThreads, s->stream, s->spos, s->cells, s->n, s->P,
-                     s->rho, s->aux, s->nbr, s->nbr_count, xall, s->xa, s->svel);
-    else
-        kernel<<<blocks, kDensityThreads, 0, s->stream>>>(s->spos, s->cells, s->n, s->P, s->rho,
-                                                          s->aux, s->nbr, s->nbr_count, xall,
-                                                          s->xa, s->svel);
+    with_lists(s->list_cap, [&](auto lists) {
+        using L = decltype(lists);
+        if (s->n < kDensitySplitMost) {
+            launch_after(xall ? density_split_kernel<true, L> : density_split_kernel<false, L>,
+                         blocks_for(s->n, kSplitWarps * kSplitPer), 32 * kSplitWarps, s->stream,
+                         s->spos, s->cells, s->n, s->P, s->rho, s->aux, s->nbr, s->nbr_count, lists,
+                         xall, s->xa, s->svel);
+            return;
+        }
+        const auto kernel = xall ? density_kernel<true, L> : density_kernel<false, L>;
+        const uint32_t blocks = blocks_for(s->n, kDensityThreads);
+        if (s->n < kDensityAfterMost)
+            launch_after(kernel, blocks, kDensityThreads, s->stream, s->spos, s->cells, s->n, s->P,
+                         s->rho, s->aux, s->nbr, s->nbr_count, lists, xall, s->xa, s->svel);
+        else
+            kernel<<<blocks, kDensityThreads, 0, s->stream>>>(s->spos, s->cells, s->n, s->P, s->rho,
+                                                              s->aux, s->nbr, s->nbr_count, lists,
+                                                              xall, s->xa, s->svel);
+    });
 }
 
 void enqueue_force(sph_solver* s, float dt) {
@@ -190,8 +193,10 @@ int check_device_error(sph_solver* s) {
     return SPH_OK;
 }
 
-int create_solver(const sph_config* config, const HostInit& init, uint32_t n_fluid,
-                  uint32_t n_boundary, uint64_t step, sph_solver** out) {
+namespace {
+
+int create_with_lists(const sph_config* config, const HostInit& init, uint32_t n_fluid,
+                      uint32_t n_boundary, uint64_t step, uint32_t list_cap, sph_solver** out) {
     *out = nullptr;
     SimParams P;
     int rc = make_sim_params(*config, &P);
@@ -205,6 +210,7 @@ int create_solver(const sph_config* config, const HostInit& init, uint32_t n_flu
     s->ncells = sph_grid_num_cells(&config->grid);
     s->key_bits = 3 * P.g.mbits;
     s->step = step;
+    s->list_cap = list_cap;
 #define TRY(x)                      \
     do {                            \
         int _r = (x);               \
@@ -226,7 +232,7 @@ int create_solver(const sph_config* config, const HostInit& init, uint32_t n_flu
     TRY(dalloc(&s->rho, n_fluid));
     TRY(dalloc(&s->aux, n_fluid));
     TRY(dalloc(&s->xa, n_fluid));
-    TRY(dalloc(&s->nbr, (size_t)n_fluid * (kMaxNbr / 4)));
+    TRY(dalloc(&s->nbr, (size_t)n_fluid * (list_cap / 4)));
     TRY(dalloc(&s->nbr_count, n_fluid));
     TRY(dalloc(&s->bnear, s->ncells));
     TRY(dalloc(&s->bacc, n_fluid));
@@ -344,6 +350,15 @@ int create_solver(const sph_config* config, const HostInit& init, uint32_t n_flu
 #undef TRY
     *out = s;
     return SPH_OK;
+}
+
+}  // namespace
+
+int create_solver(const sph_config* config, const HostInit& init, uint32_t n_fluid,
+                  uint32_t n_boundary, uint64_t step, sph_solver** out) {
+    return with_list_capacity(n_fluid, kMaxNbr, [&](uint32_t list_cap) {
+        return create_with_lists(config, init, n_fluid, n_boundary, step, list_cap, out);
+    });
 }
 
 }  // namespace sph_ss
@@ -584,8 +599,10 @@ int sph_debug_step_fields(sph_solver* s, uint32_t* keys, uint32_t* ids, uint32_t
     SPH_CUDA(cudaMalloc(&dnf, 4 * (size_t)n));
     SPH_CUDA(cudaMalloc(&dnb, 4 * (size_t)n));
     const int out = enqueue_neighborhood(s);  // buffer index holding the sorted keys
-    density_kernel<true><<<blocks_for(n, kDensityThreads), kDensityThreads, 0, s->stream>>>(
-        s->spos, s->cells, n, s->P, drho, daux, s->nbr, s->nbr_count, dnf, s->xa, s->svel);
+    with_lists(s->list_cap, [&](auto lists) {
+        density_kernel<true><<<blocks_for(n, kDensityThreads), kDensityThreads, 0, s->stream>>>(
+            s->spos, s->cells, n, s->P, drho, daux, s->nbr, s->nbr_count, lists, dnf, s->xa, s->svel);
+    });
     force_kernel<1><<<blocks_for(n), 256, 0, s->stream>>>(
         s->spos, s->xa, s->svel, s->cells, s->nbr, s->nbr_count, s->bpos, s->bcells, s->bnear, n,
         s->nb, s->P, 0.0f, nullptr, nullptr, dacc, dnb);
@@ -673,6 +690,24 @@ int sph_profile_phases(sph_solver* s, float dt, int32_t steps, float* ms) {
 int sph_debug_force_lookback_timeout(sph_solver* s, int32_t on) {
     if (!s) return fail(SPH_E_INVALID, "NULL handle");
     s->force_timeout = on ? 1 : 0;
+    return SPH_OK;
+}
+
+int sph_debug_list_capacity(sph_solver* s, uint32_t entries) {
+    if (!s) return fail(SPH_E_INVALID, "NULL handle");
+    const int rc = check_list_capacity(entries, "sph_debug_list_capacity");
+    if (rc != SPH_OK) return rc;
+    SPH_CUDA(cudaStreamSynchronize(s->stream));
+    sph_rollout_release(s);
+    if (s->graph) {
+        cudaGraphExecDestroy(s->graph);
+        s->graph = nullptr;
+    }
+    uint4* lists = nullptr;
+    SPH_CUDA(cudaMalloc(&lists, 4 * (size_t)entries * std::max(s->n, 1u)));
+    cudaFree(s->nbr);
+    s->nbr = lists;
+    s->list_cap = entries;
     return SPH_OK;
 }
 

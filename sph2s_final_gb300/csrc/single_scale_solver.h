@@ -24,7 +24,8 @@ struct sph_solver {
     float* rho = nullptr;
     float2* aux = nullptr;
     float4* xa = nullptr;           // force-pass records (x, p/rho^2), written by the density pass
-    uint4* nbr = nullptr;           // neighbour lists, kMaxNbr per particle, [group][particle]
+    uint4* nbr = nullptr;           // neighbour lists, list_cap per particle, [group][particle]
+    uint32_t list_cap = sph::kMaxNbr;
     uint32_t* nbr_count = nullptr;  // neighbours per particle (force set, r > 0)
     uint8_t* bnear = nullptr;       // per cell: boundary particles within stencil reach
     uint32_t* bstart = nullptr;     // per cell + 1: start of its static boundary candidates ...

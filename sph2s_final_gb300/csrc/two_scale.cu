@@ -40,7 +40,7 @@ struct Pop {
     int32_t* istt = nullptr;
     uint32_t *igrp = nullptr, *keep = nullptr, *off = nullptr, *split = nullptr, *soff = nullptr;
     uint2* cells = nullptr;
-    uint4* list = nullptr;           // same-population force neighbours, kMaxNbr per particle
+    uint4* list = nullptr;           // same-population force neighbours, list_cap per particle
     uint32_t* list_count = nullptr;
     uint4* clist = nullptr;          // complementary force neighbours, ComplCap per particle
     uint32_t* clist_count = nullptr;
@@ -112,6 +112,7 @@ struct sph_solver2 {
     uint32_t* err = nullptr;
     uint32_t group_base = 0;
     uint32_t stats[6] = {0, 0, 0, 0, 0, 0};
+    uint32_t list_cap = kMaxNbr;
     uint32_t next_id[2] = {0, 0};  // persistent id of the next particle created (LOW, HIGH)
     uint64_t step = 0;             // steps advanced since creation
     float* colour[2] = {nullptr, nullptr};  // colour output of the last step
@@ -135,7 +136,7 @@ int free_solver2(sph_solver2* s) {
     if (s->pjoin) cudaEventDestroy(s->pjoin);
     if (s->lowst) cudaStreamDestroy(s->lowst);
     for (void* p : s->owned) cudaFree(p);
-    for (void* p : {(void*)s->btab.start, (void*)s->btab.cand})
+    for (void* p : {(void*)s->btab.start, (void*)s->btab.cand, (void*)s->pop[0].list, (void*)s->pop[1].list})
         if (p) cudaFree(p);
     if (s->fork) cudaEventDestroy(s->fork);
     if (s->join) cudaEventDestroy(s->join);
@@ -194,7 +195,8 @@ int make_ts_params(const sph_config2& c, TSParams* out) {
     return SPH_OK;
 }
 
-int alloc_pop(Pop& p, uint32_t cap, const sph_grid& g, uint32_t compl_cap, std::vector<void*>& o) {
+int alloc_pop(Pop& p, uint32_t cap, const sph_grid& g, uint32_t list_cap, uint32_t compl_cap,
+              std::vector<void*>& o) {
     p.cap = cap;
     p.ncells = sph_grid_num_cells(&g);
     p.key_bits = 3 * morton_bits_for(g);
@@ -209,11 +211,11 @@ int alloc_pop(Pop& p, uint32_t cap, const sph_grid& g, uint32_t compl_cap, std::
         (rc = dalloc(&p.keep, cap, o)) || (rc = dalloc(&p.off, cap, o)) ||
         (rc = dalloc(&p.split, cap, o)) || (rc = dalloc(&p.soff, cap, o)) ||
         (rc = dalloc(&p.cells, p.ncells, o)) ||
-        (rc = dalloc(&p.list, (size_t)cap * (kMaxNbr / 4), o)) ||
         (rc = dalloc(&p.list_count, cap, o)) ||
         (rc = dalloc(&p.clist, (size_t)cap * (compl_cap / 4), o)) ||
         (rc = dalloc(&p.clist_count, cap, o)) || (rc = dalloc(&p.bacc, cap, o)))
         return rc;
+    SPH_CUDA(cudaMalloc(&p.list, 4 * (size_t)list_cap * (cap ? cap : 1)));
     return SPH_OK;
 }
 
@@ -326,47 +328,49 @@ void ts_front(sph_solver2* s, float dt, bool debug, int dbg_pop, uint32_t* dnb_s
     }
     cudaEventRecord(s->pfork, st);
     cudaStreamWaitEvent(lo, s->pfork, 0);
-    if (lanes) {
-        cudaStreamWaitEvent(s->nearst, s->pfork, 0);
-        const uint32_t blocks = std::min(blocks_for(L.n, 32 * kTsWarps / kTsLanes),
-                                         (uint32_t)(4 * s->sms));
-        ts_density_lanes_kernel<0, kTsLanes, 32, 56><<<blocks, 32 * kTsWarps, 0, s->nearst>>>(
-            s->near_list, s->near_count, L.spos, L.cells, L.n, H.spos, H.cells, H.n, s->P, L.rho,
-            L.aux, L.list, L.list_count, L.clist, L.clist_count);
-        cudaEventRecord(s->njoin, s->nearst);
-    }
-    if (H.n) {
-        if (small)
-            ts_density_lanes_kernel<1, kTsSmallHigh, 48, 24>
-                <<<blocks_for(H.n, 32 * kTsWarps / kTsSmallHigh), 32 * kTsWarps, 0, st>>>(
-                    nullptr, nullptr, H.spos, H.cells, H.n, L.spos, L.cells, L.n, s->P, H.rho, H.aux,
-                    H.list, H.list_count, H.clist, H.clist_count, H.sgrp, gb, s->gsum,
-                    L.n ? s->occ + s->occ_low : nullptr);
-        else if (debug && dbg_pop == 1)
-            ts_density_kernel<1, true><<<blocks_for(H.n), 256, 0, st>>>(
-                H.spos, H.cells, H.n, L.spos, L.cells, L.n, s->P, H.rho, H.aux, dnb_same, dnb_compl,
-                H.sgrp, gb, s->gsum, H.list, H.list_count, H.clist, H.clist_count);
-        else
-            ts_density_kernel<1, false><<<blocks_for(H.n), 256, 0, st>>>(
-                H.spos, H.cells, H.n, L.spos, L.cells, L.n, s->P, H.rho, H.aux, nullptr, nullptr,
-                H.sgrp, gb, s->gsum, H.list, H.list_count, H.clist, H.clist_count, nullptr,
-                lanes ? s->occ + s->occ_low : nullptr);
-    }
-    if (L.n) {
-        if (small)
-            ts_density_lanes_kernel<0, kTsSmallLow, 32, 40>
-                <<<blocks_for(L.n, 32 * kTsWarps / kTsSmallLow), 32 * kTsWarps, 0, lo>>>(
-                    nullptr, nullptr, L.spos, L.cells, L.n, H.spos, H.cells, H.n, s->P, L.rho, L.aux,
-                    L.list, L.list_count, L.clist, L.clist_count);
-        else if (debug && dbg_pop == 0)
-            ts_density_kernel<0, true><<<blocks_for(L.n), 256, 0, lo>>>(
-                L.spos, L.cells, L.n, H.spos, H.cells, H.n, s->P, L.rho, L.aux, dnb_same, dnb_compl,
-                L.sgrp, gb, s->gsum, L.list, L.list_count, L.clist, L.clist_count);
-        else
-            ts_density_kernel<0, false><<<blocks_for(L.n), 256, 0, lo>>>(
-                L.spos, L.cells, L.n, H.spos, H.cells, H.n, s->P, L.rho, L.aux, nullptr, nullptr,
-                L.sgrp, gb, s->gsum, L.list, L.list_count, L.clist, L.clist_count, skip);
-    }
+    with_lists(s->list_cap, [&](auto lists) {
+        if (lanes) {
+            cudaStreamWaitEvent(s->nearst, s->pfork, 0);
+            const uint32_t blocks = std::min(blocks_for(L.n, 32 * kTsWarps / kTsLanes),
+                                             (uint32_t)(4 * s->sms));
+            ts_density_lanes_kernel<0, kTsLanes, 32, 56><<<blocks, 32 * kTsWarps, 0, s->nearst>>>(
+                s->near_list, s->near_count, L.spos, L.cells, L.n, H.spos, H.cells, H.n, s->P, L.rho,
+                L.aux, L.list, lists, L.list_count, L.clist, L.clist_count);
+            cudaEventRecord(s->njoin, s->nearst);
+        }
+        if (H.n) {
+            if (small)
+                ts_density_lanes_kernel<1, kTsSmallHigh, 48, 24>
+                    <<<blocks_for(H.n, 32 * kTsWarps / kTsSmallHigh), 32 * kTsWarps, 0, st>>>(
+                        nullptr, nullptr, H.spos, H.cells, H.n, L.spos, L.cells, L.n, s->P, H.rho, H.aux,
+                        H.list, lists, H.list_count, H.clist, H.clist_count, H.sgrp, gb, s->gsum,
+                        L.n ? s->occ + s->occ_low : nullptr);
+            else if (debug && dbg_pop == 1)
+                ts_density_kernel<1, true><<<blocks_for(H.n), 256, 0, st>>>(
+                    H.spos, H.cells, H.n, L.spos, L.cells, L.n, s->P, H.rho, H.aux, dnb_same, dnb_compl,
+                    H.sgrp, gb, s->gsum, H.list, lists, H.list_count, H.clist, H.clist_count);
+            else
+                ts_density_kernel<1, false><<<blocks_for(H.n), 256, 0, st>>>(
+                    H.spos, H.cells, H.n, L.spos, L.cells, L.n, s->P, H.rho, H.aux, nullptr, nullptr,
+                    H.sgrp, gb, s->gsum, H.list, lists, H.list_count, H.clist, H.clist_count, nullptr,
+                    lanes ? s->occ + s->occ_low : nullptr);
+        }
+        if (L.n) {
+            if (small)
+                ts_density_lanes_kernel<0, kTsSmallLow, 32, 40>
+                    <<<blocks_for(L.n, 32 * kTsWarps / kTsSmallLow), 32 * kTsWarps, 0, lo>>>(
+                        nullptr, nullptr, L.spos, L.cells, L.n, H.spos, H.cells, H.n, s->P, L.rho, L.aux,
+                        L.list, lists, L.list_count, L.clist, L.clist_count);
+            else if (debug && dbg_pop == 0)
+                ts_density_kernel<0, true><<<blocks_for(L.n), 256, 0, lo>>>(
+                    L.spos, L.cells, L.n, H.spos, H.cells, H.n, s->P, L.rho, L.aux, dnb_same, dnb_compl,
+                    L.sgrp, gb, s->gsum, L.list, lists, L.list_count, L.clist, L.clist_count);
+            else
+                ts_density_kernel<0, false><<<blocks_for(L.n), 256, 0, lo>>>(
+                    L.spos, L.cells, L.n, H.spos, H.cells, H.n, s->P, L.rho, L.aux, nullptr, nullptr,
+                    L.sgrp, gb, s->gsum, L.list, lists, L.list_count, L.clist, L.clist_count, skip);
+        }
+    });
     cudaEventRecord(s->pjoin, lo);
     cudaStreamWaitEvent(st, s->pjoin, 0);
     if (lanes) cudaStreamWaitEvent(st, s->njoin, 0);
@@ -577,13 +581,10 @@ int upload_pop(sph_solver2* s, int r, const HostPop& h) {
 // Allocates a handle for capacities capL / capH, uploads both populations,
 // sets the group and id counters and presorts the boundary (float4, ordered
 // by depth outside the LOW grid's box with the depth in w) on the LOW grid.
-int create_solver2(const sph_config2* config, const TSParams& P, uint64_t capL, uint64_t capH,
-                   const HostPop* pops, const float4* hb, uint32_t n_boundary,
-                   uint32_t group_base, const uint32_t next_id[2], uint64_t step,
-                   sph_solver2** out) {
-    // both populations share one sort, whose look-back counts hold 30 bits
-    if (capL + capH > kMaxParticles || n_boundary > kMaxParticles)
-        return fail(SPH_E_CAPACITY, "two-scale: more than 2^30 particles");
+int create_with_lists(const sph_config2* config, const TSParams& P, uint64_t capL, uint64_t capH,
+                      const HostPop* pops, const float4* hb, uint32_t n_boundary,
+                      uint32_t group_base, const uint32_t next_id[2], uint64_t step,
+                      uint32_t list_cap, sph_solver2** out) {
     sph_solver2* s = new sph_solver2();
     s->cfg = *config;
     s->P = P;
@@ -592,6 +593,7 @@ int create_solver2(const sph_config2* config, const TSParams& P, uint64_t capL, 
     s->next_id[1] = next_id[1];
     s->group_base = group_base;
     s->step = step;
+    s->list_cap = list_cap;
     s->cap_groups = (uint32_t)(capH / 8 * 4 + 64);
 #define TRY(x)                                 \
     do {                                       \
@@ -629,8 +631,8 @@ int create_solver2(const sph_config2* config, const TSParams& P, uint64_t capL, 
     s->BP.bnd_coef = P.bnd_coef;
     s->BP.two_over_h = P.two_over_h0;
     s->BP.bmargin = P.bmargin;
-    TRY(alloc_pop(s->pop[0], (uint32_t)capL, config->grid[0], ComplCap<0>::value, s->owned));
-    TRY(alloc_pop(s->pop[1], (uint32_t)capH, config->grid[1], ComplCap<1>::value, s->owned));
+    TRY(alloc_pop(s->pop[0], (uint32_t)capL, config->grid[0], list_cap, ComplCap<0>::value, s->owned));
+    TRY(alloc_pop(s->pop[1], (uint32_t)capH, config->grid[1], list_cap, ComplCap<1>::value, s->owned));
     // one sort holds both populations (ts_neighborhoods), or the boundary at creation
     const uint32_t nmax = (uint32_t)std::max<uint64_t>(capL + capH, n_boundary);
     for (int b = 0; b < 2; ++b) {
@@ -721,6 +723,19 @@ int create_solver2(const sph_config2* config, const TSParams& P, uint64_t capL, 
 #undef TRY
     *out = s;
     return SPH_OK;
+}
+
+int create_solver2(const sph_config2* config, const TSParams& P, uint64_t capL, uint64_t capH,
+                   const HostPop* pops, const float4* hb, uint32_t n_boundary,
+                   uint32_t group_base, const uint32_t next_id[2], uint64_t step,
+                   sph_solver2** out) {
+    // both populations share one sort, whose look-back counts hold 30 bits
+    if (capL + capH > kMaxParticles || n_boundary > kMaxParticles)
+        return fail(SPH_E_CAPACITY, "two-scale: more than 2^30 particles");
+    return with_list_capacity(capL + capH, kMaxNbr, [&](uint32_t list_cap) {
+        return create_with_lists(config, P, capL, capH, pops, hb, n_boundary, group_base, next_id,
+                                 step, list_cap, out);
+    });
 }
 
 uint64_t ts_state_bytes(uint64_t n_low, uint64_t n_high, uint64_t nb) {
@@ -918,6 +933,31 @@ int sph2_debug_step_fields(sph_solver2* s, int32_t population, uint32_t* ids_sor
     cudaFree(db);
     SPH_CUDA(e);
     return check_err2(s);
+}
+
+int sph2_debug_list_capacity(sph_solver2* s, uint32_t entries) {
+    if (!s) return fail(SPH_E_INVALID, "NULL handle");
+    const int rc = check_list_capacity(entries, "sph2_debug_list_capacity");
+    if (rc != SPH_OK) return rc;
+    SPH_CUDA(cudaStreamSynchronize(s->stream));
+    if (s->graph) {
+        cudaGraphExecDestroy(s->graph);
+        s->graph = nullptr;
+    }
+    uint4* lists[2] = {nullptr, nullptr};
+    for (int r = 0; r < 2; ++r) {
+        const cudaError_t e = cudaMalloc(&lists[r], 4 * (size_t)entries * std::max(s->pop[r].cap, 1u));
+        if (e != cudaSuccess) {
+            cudaFree(lists[0]);
+            SPH_CUDA(e);
+        }
+    }
+    for (int r = 0; r < 2; ++r) {
+        cudaFree(s->pop[r].list);
+        s->pop[r].list = lists[r];
+    }
+    s->list_cap = entries;
+    return SPH_OK;
 }
 
 int sph2_destroy(sph_solver2* s) { return free_solver2(s); }

@@ -251,13 +251,13 @@ static __global__ void __launch_bounds__(256) ts_near_kernel(
 // blocks of LOW cells that hold LOW particles (ts_gather_kernel); looking at up
 // to eight of them instead of 27 LOW cells leaves the pass where it was
 // (622,592 HIGH particles: 204 -> 199 us).
-template <int R, bool DEBUG>
+template <int R, bool DEBUG, class LISTS>
 __global__ void __launch_bounds__(256) ts_density_kernel(
     const float4* __restrict__ spos_r, const uint2* __restrict__ cells_r, uint32_t n_r,
     const float4* __restrict__ spos_c, const uint2* __restrict__ cells_c, uint32_t n_c,
     TSParams P, float* __restrict__ rho, float2* __restrict__ aux, uint32_t* __restrict__ nbr_same,
     uint32_t* __restrict__ nbr_compl, const uint32_t* __restrict__ sgrp_r, uint32_t group_base,
-    unsigned long long* __restrict__ gsurf, uint4* __restrict__ list4,
+    unsigned long long* __restrict__ gsurf, uint4* __restrict__ list4, LISTS lists,
     uint32_t* __restrict__ list_count, uint4* __restrict__ clist4,
     uint32_t* __restrict__ clist_count, const uint8_t* __restrict__ skip = nullptr,
     const uint8_t* __restrict__ low_blocks = nullptr) {
@@ -289,7 +289,7 @@ __global__ void __launch_bounds__(256) ts_density_kernel(
                             s = fmaf(P.coupled ? 1.0f : xj.w, a * a * a, s);
                             if (DEBUG) ++ns;
                             if (r2 != 0.0f) {
-                                if (k < (uint32_t)kMaxNbr) __stcs(out, j);  // lists: evict-first
+                                if (lists.holds(k)) __stcs(out, j);  // lists: evict-first
                                 out += (k & 3u) == 3u ? next_group : 1u;
                                 ++k;
                             }
@@ -334,7 +334,7 @@ __global__ void __launch_bounds__(256) ts_density_kernel(
     }
     clist_count[i] = kcl;
     const float rh = ts_density_out<R>(i, s, sc, P, rho, aux);
-    list_count[i] = k;
+    list_count[i] = lists.count(k);
     if (DEBUG) {
         nbr_same[i] = ns;
         nbr_compl[i] = nc;
@@ -380,13 +380,13 @@ __device__ __forceinline__ void ts_list_put(uint4* __restrict__ list4, uint32_t 
 
 // R the population, SAME and COMPL the hits a lane has room for; without a list
 // (near NULL) every particle.
-template <int R, uint32_t LANES, uint32_t SAME, uint32_t COMPL>
+template <int R, uint32_t LANES, uint32_t SAME, uint32_t COMPL, class LISTS>
 __global__ void __launch_bounds__(32 * kTsWarps) ts_density_lanes_kernel(
     const uint32_t* __restrict__ near, const uint32_t* __restrict__ near_count,
     const float4* __restrict__ spos_r, const uint2* __restrict__ cells_r, uint32_t n_r,
     const float4* __restrict__ spos_c, const uint2* __restrict__ cells_c, uint32_t n_c,
     TSParams P, float* __restrict__ rho, float2* __restrict__ aux, uint4* __restrict__ list4,
-    uint32_t* __restrict__ list_count, uint4* __restrict__ clist4,
+    LISTS lists, uint32_t* __restrict__ list_count, uint4* __restrict__ clist4,
     uint32_t* __restrict__ clist_count, const uint32_t* __restrict__ sgrp_r = nullptr,
     uint32_t group_base = 0, unsigned long long* __restrict__ gsurf = nullptr,
     const uint8_t* __restrict__ low_blocks = nullptr) {
@@ -454,11 +454,11 @@ __global__ void __launch_bounds__(32 * kTsWarps) ts_density_lanes_kernel(
         uint32_t same, compl_;
         uint32_t at = ts_lanes_start<LANES>(k, same), cat = ts_lanes_start<LANES>(kc, compl_);
         if (k <= SAME) {
-            for (uint32_t e = 0; e < k && at < (uint32_t)kMaxNbr; ++e, ++at)
+            for (uint32_t e = 0; e < k && lists.holds(at); ++e, ++at)
                 ts_list_put(list4, at, i, n_r, hs[e * 32]);
         } else {
             scan(P.g[R], cells_r, spos_r, n_r, P.h[R], P.T[R], [&](uint32_t j, const float4&, float r2) {
-                if (r2 != 0.0f && at < (uint32_t)kMaxNbr) ts_list_put(list4, at++, i, n_r, j);
+                if (r2 != 0.0f && lists.holds(at)) ts_list_put(list4, at++, i, n_r, j);
             });
         }
         if (kc <= COMPL) {
@@ -476,7 +476,7 @@ __global__ void __launch_bounds__(32 * kTsWarps) ts_density_lanes_kernel(
         }
         if (on && sub == 0) {
             const float rh = ts_density_out<R>(i, s, sc, P, rho, aux);
-            list_count[i] = same;
+            list_count[i] = lists.count(same);
             clist_count[i] = compl_;
             if (R == 1) ts_surface(i, rh, P, sgrp_r, group_base, gsurf);
         }

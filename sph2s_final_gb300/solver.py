@@ -251,6 +251,10 @@ class Solver:
         "coherent" = only the particles that changed cell); same results."""
         check(lib().sph_debug_sort_mode(self._h, self.SORT_MODES[mode]))
 
+    def debug_list_capacity(self, entries: int) -> None:
+        """Test hook: entries of the neighbour lists (4, 8, ... 96); same results."""
+        check(lib().sph_debug_list_capacity(self._h, int(entries)))
+
     def positions_async(self, out: np.ndarray, order: str = "sorted") -> None:
         """Enqueues a readback of the positions into `out` (float32 (n, 3), best
         pinned); valid after sync().  The copy overlaps the next steps."""

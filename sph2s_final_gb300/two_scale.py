@@ -123,6 +123,10 @@ class Solver2:
                                            uptr(r["nbr_compl"]), uptr(r["nbr_boundary"])))
         return r
 
+    def debug_list_capacity(self, entries: int) -> None:
+        """Test hook: entries of the same-population neighbour lists (4, 8, ... 96)."""
+        check(lib().sph2_debug_list_capacity(self._h, int(entries)))
+
     def set_color_output(self, on: bool = True) -> None:
         """Colour / energy output of the force pass (dColorValues), off by default."""
         check(lib().sph2_set_color_output(self._h, 1 if on else 0))
