@@ -336,6 +336,13 @@ int sph2_get_states_device(sph_solver2* s, int32_t population, int32_t* d_state)
 int sph2_debug_step_fields(sph_solver2* s, int32_t population, uint32_t* ids_sorted, float* rho,
                            float* acc, uint32_t* nbr_same, uint32_t* nbr_compl,
                            uint32_t* nbr_boundary);
+/* Parity instrumentation: what the last sph2_advance step's own kernels found
+ * for one population, in that step's sorted order: persistent ids, densities,
+ * and the lengths of the particles' lists of neighbours at a distance above 0
+ * (same population; complementary), or a number beyond a list's capacity.
+ * *count: particles of that step.  NULL arrays are left out. */
+int sph2_debug_last_step(sph_solver2* s, int32_t population, uint32_t* ids_sorted, float* rho,
+                         uint32_t* nbr_same, uint32_t* nbr_compl, uint32_t* count);
 /* sph_debug_list_capacity for the same-population lists. */
 int sph2_debug_list_capacity(sph_solver2* s, uint32_t entries);
 int sph2_destroy(sph_solver2* s);

@@ -135,6 +135,7 @@ SIGNATURES = {
     "sph2_next_ids": (C.c_int, [_vp, _u, _u]),
     "sph2_get_state": (C.c_int, [_vp, C.c_int32, _f, _f, _f, C.POINTER(C.c_int32), _u, _u]),
     "sph2_debug_step_fields": (C.c_int, [_vp, C.c_int32, _u, _f, _f, _u, _u, _u]),
+    "sph2_debug_last_step": (C.c_int, [_vp, C.c_int32, _u, _f, _u, _u, _u]),
     "sph2_destroy": (C.c_int, [_vp]),
     "sph2_set_color_output": (C.c_int, [_vp, C.c_int32]),
     "sph2_get_colors": (C.c_int, [_vp, C.c_int32, _f, _u, _u]),

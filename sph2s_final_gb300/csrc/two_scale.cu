@@ -118,6 +118,7 @@ struct sph_solver2 {
     float* colour[2] = {nullptr, nullptr};  // colour output of the last step
     bool colour_on = false;
     uint32_t colour_n[2] = {0, 0};          // particles of that step per population
+    uint32_t stepped_n[2] = {0, 0};         // the same, with or without colours
     std::vector<void*> owned;
 };
 
@@ -531,8 +532,8 @@ int ts_step(sph_solver2* s, float dt) {
     s->stats[3] = H.n - c[kCtlSurvH];
     s->stats[4] = c[kCtlFadedL];
     s->stats[5] = c[kCtlFadedH];
-    s->colour_n[0] = L.n;
-    s->colour_n[1] = H.n;
+    s->colour_n[0] = s->stepped_n[0] = L.n;
+    s->colour_n[1] = s->stepped_n[1] = H.n;
     H.n = c[kCtlNextH];
     L.n = c[kCtlNextL];
     s->group_base = c[kCtlGroupBase];
@@ -933,6 +934,26 @@ int sph2_debug_step_fields(sph_solver2* s, int32_t population, uint32_t* ids_sor
     cudaFree(db);
     SPH_CUDA(e);
     return check_err2(s);
+}
+
+int sph2_debug_last_step(sph_solver2* s, int32_t population, uint32_t* ids_sorted, float* rho,
+                         uint32_t* nbr_same, uint32_t* nbr_compl, uint32_t* count) {
+    if (!s || population < 0 || population > 1)
+        return fail(SPH_E_INVALID, "sph2_debug_last_step: bad handle or population");
+    const Pop& p = s->pop[population];
+    const size_t n = s->stepped_n[population];
+    if (count) *count = (uint32_t)n;
+    if (!n) return SPH_OK;
+    SPH_CUDA(cudaStreamSynchronize(s->stream));
+    if (ids_sorted) {
+        std::vector<float4> sv(n);
+        SPH_CUDA(cudaMemcpy(sv.data(), p.svel, 16 * n, cudaMemcpyDeviceToHost));
+        for (size_t k = 0; k < n; ++k) std::memcpy(&ids_sorted[k], &sv[k].w, 4);
+    }
+    if (rho) SPH_CUDA(cudaMemcpy(rho, p.rho, 4 * n, cudaMemcpyDeviceToHost));
+    if (nbr_same) SPH_CUDA(cudaMemcpy(nbr_same, p.list_count, 4 * n, cudaMemcpyDeviceToHost));
+    if (nbr_compl) SPH_CUDA(cudaMemcpy(nbr_compl, p.clist_count, 4 * n, cudaMemcpyDeviceToHost));
+    return SPH_OK;
 }
 
 int sph2_debug_list_capacity(sph_solver2* s, uint32_t entries) {

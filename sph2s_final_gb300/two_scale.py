@@ -123,6 +123,16 @@ class Solver2:
                                            uptr(r["nbr_compl"]), uptr(r["nbr_boundary"])))
         return r
 
+    def debug_last_step(self, population: int) -> dict:
+        """What the last step's own kernels found, in that step's sorted order."""
+        n = C.c_uint32()
+        check(lib().sph2_debug_last_step(self._h, population, None, None, None, None, C.byref(n)))
+        r = {"ids": np.empty(n.value, np.uint32), "rho": np.empty(n.value, np.float32),
+             "nbr_same": np.empty(n.value, np.uint32), "nbr_compl": np.empty(n.value, np.uint32)}
+        check(lib().sph2_debug_last_step(self._h, population, uptr(r["ids"]), fptr(r["rho"]),
+                                         uptr(r["nbr_same"]), uptr(r["nbr_compl"]), C.byref(n)))
+        return r
+
     def debug_list_capacity(self, entries: int) -> None:
         """Test hook: entries of the same-population neighbour lists (4, 8, ... 96)."""
         check(lib().sph2_debug_list_capacity(self._h, int(entries)))
