@@ -431,9 +431,14 @@ int sphb_create(const sph_scene_desc* scenes, uint32_t num_scenes, sph_batch** o
     if (!scenes || !out || num_scenes == 0)
         return fail(SPH_E_INVALID, "sphb_create: need at least one scene and an output handle");
     *out = nullptr;
-    uint64_t n = 0;
-    for (uint32_t s = 0; s < num_scenes; ++s) n += scenes[s].n_fluid;
-    return with_list_capacity(n, kMaxNbr, [&](uint32_t list_cap) {
+    uint64_t n = 0, crowded = 0;
+    for (uint32_t s = 0; s < num_scenes; ++s) {
+        const sph_config& c = scenes[s].config;
+        n += scenes[s].n_fluid;
+        if (list_entries(c.effective_radius, c.fluid_particle_mass, c.rest_density) < (uint32_t)kMaxNbr)
+            crowded += scenes[s].n_fluid;
+    }
+    return with_list_capacity(n, 2 * crowded > n ? kCrowdedNbr : kMaxNbr, [&](uint32_t list_cap) {
         return create_with_lists(scenes, num_scenes, list_cap, out);
     });
 }

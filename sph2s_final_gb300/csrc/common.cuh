@@ -21,24 +21,34 @@ constexpr uint32_t kEmptyCell = 0xFFFFFFFFu;  // EMPTY_CELL_ID, SPH2S_FINAL_SING
 // against 103.  Slots past a particle's neighbours are never touched.
 constexpr int kMaxNbr = 96;
 
+// Slots where the support holds more than kMaxNbr particles (list_entries).
+constexpr int kCrowdedNbr = 64;
+
 // The density passes write the lists through one of these: the slots a list has, and
 // the count to leave for k neighbours, of which the passes after them see whether it is
 // above kMaxNbr.  Where memory is short a handle's lists have fewer slots
 // (with_list_capacity), in a variant of its own: with the number as an argument every
 // density pass took 1 to 2 % longer (a step of 2,097,152 particles 756 -> 768 us).
-struct FullLists {
-    __device__ __forceinline__ bool holds(uint32_t k) const { return k < (uint32_t)kMaxNbr; }
-    __device__ __forceinline__ uint32_t count(uint32_t k) const { return k; }
+template <int SLOTS>
+struct FixedLists {
+    __device__ __forceinline__ bool holds(uint32_t k) const { return k < (uint32_t)SLOTS; }
+    __device__ __forceinline__ bool fits(uint32_t k) const { return k <= (uint32_t)SLOTS; }
+    __device__ __forceinline__ uint32_t count(uint32_t k) const {
+        return SLOTS == kMaxNbr || fits(k) ? k : ~0u;
+    }
 };
 struct ShortLists {
     uint32_t slots;
     __device__ __forceinline__ bool holds(uint32_t k) const { return k < slots; }
-    __device__ __forceinline__ uint32_t count(uint32_t k) const { return k <= slots ? k : ~0u; }
+    __device__ __forceinline__ bool fits(uint32_t k) const { return k <= slots; }
+    __device__ __forceinline__ uint32_t count(uint32_t k) const { return fits(k) ? k : ~0u; }
 };
 template <class F>
 inline void with_lists(uint32_t slots, F&& launch) {
     if (slots == (uint32_t)kMaxNbr)
-        launch(FullLists{});
+        launch(FixedLists<kMaxNbr>{});
+    else if (slots == (uint32_t)kCrowdedNbr)
+        launch(FixedLists<kCrowdedNbr>{});
     else
         launch(ShortLists{slots});
 }

@@ -182,13 +182,13 @@ __global__ void __launch_bounds__(32 * kSplitWarps) density_split_kernel(
     const uint32_t total = __shfl_sync(kAll, at, end);
     all = __shfl_sync(kAll, all, end);
     at -= listed;
-    if (on) {
+    if (on && lists.fits(total)) {  // a longer list is not read
         uint32_t k = at;
         uint32_t* out =
             reinterpret_cast<uint32_t*>(nbr4) + 4 * ((size_t)(k >> 2) * n + i) + (k & 3u);
         const uint32_t next_group = 4u * n - 3u;
         auto put = [&](uint32_t j) {
-            if (lists.holds(k)) __stcs(out, j);
+            __stcs(out, j);
             out += (k & 3u) == 3u ? next_group : 1u;
             ++k;
         };

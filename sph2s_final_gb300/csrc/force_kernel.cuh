@@ -207,13 +207,12 @@ static __global__ void __launch_bounds__(256) boundary_force_kernel(
 constexpr uint32_t kForceManyParticles = 1u << 17;
 
 // The pair sums of a particle whose list overflowed: from the stencil, in the
-// same order.  Out of line, so that its registers are not the pass's.
-static __device__ __noinline__ ForceAcc force_rescan(float4 xi, float4 vi, float tcoef,
-                                                     const float4* __restrict__ xa,
-                                                     const float4* __restrict__ va,
-                                                     const uint2* __restrict__ cells, uint32_t n,
-                                                     const SimParams* params) {
-    const SimParams& P = *params;
+// same order.
+__device__ __forceinline__ ForceAcc force_stencil(const float4& xi, const float4& vi, float tcoef,
+                                                  const float4* __restrict__ xa,
+                                                  const float4* __restrict__ va,
+                                                  const uint2* __restrict__ cells, uint32_t n,
+                                                  const SimParams& P) {
     ForceAcc A = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
     const Stencil s = stencil(P.g, xi.x, xi.y, xi.z, P.h);
     for (int cz = s.z0; cz <= s.z1; ++cz)
@@ -237,6 +236,15 @@ static __device__ __noinline__ ForceAcc force_rescan(float4 xi, float4 vi, float
     return A;
 }
 
+// Out of line, so that its registers are not the pass's.
+static __device__ __noinline__ ForceAcc force_rescan(float4 xi, float4 vi, float tcoef,
+                                                     const float4* __restrict__ xa,
+                                                     const float4* __restrict__ va,
+                                                     const uint2* __restrict__ cells, uint32_t n,
+                                                     const SimParams* params) {
+    return force_stencil(xi, vi, tcoef, xa, va, cells, n, *params);
+}
+
 // Pressure (spiky gradient), viscosity (Laplacian), tension (Poly6), boundary
 // force and gravity; MODE 0 integrates (symplectic Euler) into pos_out/vel_out,
 // MODE 1 writes the acceleration and the boundary neighbour count instead,
@@ -255,8 +263,10 @@ static __device__ __noinline__ ForceAcc force_rescan(float4 xi, float4 vi, float
 // 705 to 674 us.  From kForceManyParticles on, one at a time at 48 registers and
 // 5 blocks: three solvers of 155,184 side by side 298 us for four steps (four
 // together: 307), a step of 2,097,152 773 us (four together 796, 40 registers
-// 783).  All the same bits.
-template <int MODE, bool BSEP = false, int AHEAD = 4>
+// 783).  CROWDED, where most lists overflow (list_entries): the rescan in line, one
+// gather at a time, 40 registers and 6 blocks (1,000,000 particles with 110
+// neighbours: force 1,076 -> 889 us).  All the same bits.
+template <int MODE, bool BSEP = false, int AHEAD = 4, bool CROWDED = false>
 __device__ __forceinline__ void force_one(
     uint32_t i, const float4* __restrict__ pos, const float4* __restrict__ xa,
     const float4* __restrict__ va, const uint2* __restrict__ cells, const uint4* __restrict__ nbr4,
@@ -300,7 +310,8 @@ __device__ __forceinline__ void force_one(
             g = gn;
         }
     } else {
-        A = force_rescan(xi, vi, tcoef, xa, va, cells, n, params);
+        A = CROWDED ? force_stencil(xi, vi, tcoef, xa, va, cells, n, P)
+                    : force_rescan(xi, vi, tcoef, xa, va, cells, n, params);
     }
     float bx = 0.f, by = 0.f, bz = 0.f;
     uint32_t bcnt = 0;
@@ -333,8 +344,8 @@ __device__ __forceinline__ void force_one(
     }
 }
 
-template <int MODE, bool BSEP = false, int AHEAD = 4>
-__global__ void __launch_bounds__(256, AHEAD > 1 ? 4 : 5) force_kernel(
+template <int MODE, bool BSEP = false, int AHEAD = 4, bool CROWDED = false>
+__global__ void __launch_bounds__(256, CROWDED ? 6 : AHEAD > 1 ? 4 : 5) force_kernel(
     const float4* __restrict__ pos, const float4* __restrict__ xa, const float4* __restrict__ va,
     const uint2* __restrict__ cells, const uint4* __restrict__ nbr4,
     const uint32_t* __restrict__ nbr_count, const float4* __restrict__ bpos,
@@ -344,7 +355,7 @@ __global__ void __launch_bounds__(256, AHEAD > 1 ? 4 : 5) force_kernel(
     const float4* __restrict__ bacc = nullptr, const uint8_t* __restrict__ nflag = nullptr) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    force_one<MODE, BSEP, AHEAD>(i, pos, xa, va, cells, nbr4, nbr_count, bpos, bcells, bnear, n, nb,
+    force_one<MODE, BSEP, AHEAD, CROWDED>(i, pos, xa, va, cells, nbr4, nbr_count, bpos, bcells, bnear, n, nb,
                                  P, &P, dt, pos_out, vel_out, acc_out, nbr_b, bacc, nflag);
 }
 

@@ -75,6 +75,17 @@ inline int boundary_depth_bits(const GridParams& p, float h, int key_bits) {
     return std::max(0, std::min(8, 32 - key_bits));
 }
 
+// Entries of the neighbour lists where a support of radius h holds rho0 / m particles
+// per volume.  Above kMaxNbr of them most lists overflow: they are then written for
+// nothing and the force pass rescans all the same, so they have kCrowdedNbr entries,
+// which the particles at a surface still fit.  Us per step with 96 and with 64 entries,
+// 1,000,000 particles: h = 3 spacings (113 in the support) 1,930 and 1,510, h = 2.9
+// (102) after 400 steps 1,542 and 1,440; h = 2.8 (92) 1,321 and 1,364.
+inline uint32_t list_entries(float h, float m, float rho0) {
+    const double held = 4.18879020478639 * (double)h * h * h * rho0 / m;  // 4 pi / 3
+    return held > (double)kMaxNbr ? kCrowdedNbr : kMaxNbr;
+}
+
 // Calls make(entries), which allocates neighbour lists of that many entries for
 // `lists` particles (or particle-steps of a tape), with at most `most`: kMaxNbr, or
 // fewer where the memory does not hold them (the results are the same: a particle

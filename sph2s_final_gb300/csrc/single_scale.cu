@@ -95,7 +95,10 @@ int enqueue_neighborhood(sph_solver* s) {
 // Below this many particles the density pass's blocks are set up while the pass
 // before it drains (launch_after: 262,144 particles 158.3 -> 156.9 us per step).
 // At 2,097,152 they then hold every SM before the boundary pass gets a block, and
-// the force pass waits for that one: 788 -> 792 us; 1,000,000: 420 either way.
+// the force pass waits for that one: 788 -> 792 us; 1,000,000: 420 either way.  A
+// quarter as many where the support holds more than a list (list_entries), whose
+// boundary pass is longer: 195,112 particles with 113 neighbours 432 -> 416 us, but
+// 512,000 881 -> 922.
 constexpr uint32_t kDensityAfterMost = 1u << 20;
 
 // The density pass, and beside it on the second branch (fork/join events,
@@ -121,7 +124,8 @@ void enqueue_density(sph_solver* s, uint32_t* xall) {
         }
         const auto kernel = xall ? density_kernel<true, L> : density_kernel<false, L>;
         const uint32_t blocks = blocks_for(s->n, kDensityThreads);
-        if (s->n < kDensityAfterMost)
+        const bool full = s->list_cap == (uint32_t)kMaxNbr;
+        if (s->n < (full ? kDensityAfterMost : kDensityAfterMost / 4))
             launch_after(kernel, blocks, kDensityThreads, s->stream, s->spos, s->cells, s->n, s->P,
                          s->rho, s->aux, s->nbr, s->nbr_count, lists, xall, s->xa, s->svel);
         else
@@ -133,7 +137,9 @@ void enqueue_density(sph_solver* s, uint32_t* xall) {
 
 void enqueue_force(sph_solver* s, float dt) {
     cudaStreamWaitEvent(s->stream, s->join, 0);
-    const auto kernel = s->n < kForceManyParticles ? force_kernel<0, true, 4> : force_kernel<0, true, 1>;
+    const auto kernel = s->list_cap != (uint32_t)kMaxNbr ? force_kernel<0, true, 1, true>
+                        : s->n < kForceManyParticles     ? force_kernel<0, true, 4>
+                                                         : force_kernel<0, true, 1>;
     kernel<<<blocks_for(s->n), 256, 0, s->stream>>>(
         s->spos, s->xa, s->svel, s->cells, s->nbr, s->nbr_count, s->bpos, s->bcells, s->bnear,
         s->n, s->nb, s->P, dt, s->pos, s->vel, nullptr, nullptr, s->bacc, s->bflag);
@@ -356,7 +362,9 @@ int create_with_lists(const sph_config* config, const HostInit& init, uint32_t n
 
 int create_solver(const sph_config* config, const HostInit& init, uint32_t n_fluid,
                   uint32_t n_boundary, uint64_t step, sph_solver** out) {
-    return with_list_capacity(n_fluid, kMaxNbr, [&](uint32_t list_cap) {
+    const uint32_t most = list_entries(config->effective_radius, config->fluid_particle_mass,
+                                       config->rest_density);
+    return with_list_capacity(n_fluid, most, [&](uint32_t list_cap) {
         return create_with_lists(config, init, n_fluid, n_boundary, step, list_cap, out);
     });
 }
