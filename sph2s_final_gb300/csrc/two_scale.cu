@@ -273,6 +273,11 @@ void ts_neighborhoods(sph_solver2* s) {
 // 177, 88,587 189 and 213.
 constexpr uint32_t kTsSmall = 49152;
 constexpr int kTsSmallLow = 16, kTsSmallHigh = 8, kTsForceLow = 16, kTsForceHigh = 2;
+// From this many particles on the near LOW particles' density is one lane's again: the
+// chip is full, and eight lanes to a particle are more work.  Us per step with eight
+// lanes and one, a slab of 0.3 refined: 885,000 particles 1,147 and 1,216; 1,260,000
+// 1,596 and 1,541; 1,715,000 2,190 and 1,994.
+constexpr uint32_t kTsLanesMost = 1u << 20;
 
 // Everything up to and including the force/integrate pass; DEBUG variants
 // also write accelerations and neighbour counts of population `dbg_pop`.
@@ -322,6 +327,7 @@ void ts_front(sph_solver2* s, float dt, bool debug, int dbg_pop, uint32_t* dnb_s
     // each, on a third stream (not in the debug passes)
     const bool small = !debug && L.n + H.n < kTsSmall;
     const bool lanes = !debug && !small && L.n && H.n;
+    const bool dlanes = lanes && L.n + H.n < kTsLanesMost;  // the density passes' own
     const uint8_t* skip = lanes ? s->near_flag : nullptr;
     if (lanes) {
         ts_near_kernel<<<blocks_for(L.n), 256, 0, st>>>(L.spos, L.n, s->P.g[0], s->P.h[0], s->occ,
@@ -330,7 +336,7 @@ void ts_front(sph_solver2* s, float dt, bool debug, int dbg_pop, uint32_t* dnb_s
     cudaEventRecord(s->pfork, st);
     cudaStreamWaitEvent(lo, s->pfork, 0);
     with_lists(s->list_cap, [&](auto lists) {
-        if (lanes) {
+        if (dlanes) {
             cudaStreamWaitEvent(s->nearst, s->pfork, 0);
             const uint32_t blocks = std::min(blocks_for(L.n, 32 * kTsWarps / kTsLanes),
                                              (uint32_t)(4 * s->sms));
@@ -369,12 +375,13 @@ void ts_front(sph_solver2* s, float dt, bool debug, int dbg_pop, uint32_t* dnb_s
             else
                 ts_density_kernel<0, false><<<blocks_for(L.n), 256, 0, lo>>>(
                     L.spos, L.cells, L.n, H.spos, H.cells, H.n, s->P, L.rho, L.aux, nullptr, nullptr,
-                    L.sgrp, gb, s->gsum, L.list, lists, L.list_count, L.clist, L.clist_count, skip);
+                    L.sgrp, gb, s->gsum, L.list, lists, L.list_count, L.clist, L.clist_count,
+                    dlanes ? skip : nullptr);
         }
     });
     cudaEventRecord(s->pjoin, lo);
     cudaStreamWaitEvent(st, s->pjoin, 0);
-    if (lanes) cudaStreamWaitEvent(st, s->njoin, 0);
+    if (dlanes) cudaStreamWaitEvent(st, s->njoin, 0);
     // merge decisions (slab: start-of-step centroids; surface: this step's densities)
     if (gb && (s->P.axis >= 0 || s->P.surface))
         ts_group_decide_kernel<<<blocks_for(gb), 256, 0, st>>>(s->gsum, s->gready, gb, s->P.lo43,
@@ -733,7 +740,11 @@ int create_solver2(const sph_config2* config, const TSParams& P, uint64_t capL, 
     // both populations share one sort, whose look-back counts hold 30 bits
     if (capL + capH > kMaxParticles || n_boundary > kMaxParticles)
         return fail(SPH_E_CAPACITY, "two-scale: more than 2^30 particles");
-    return with_list_capacity(capL + capH, kMaxNbr, [&](uint32_t list_cap) {
+    uint32_t most = kCrowdedNbr;
+    for (int r = 0; r < 2; ++r)
+        most = std::max(most, list_entries(config->effective_radius[r],
+                                           config->fluid_particle_mass[r], config->rest_density));
+    return with_list_capacity(capL + capH, most, [&](uint32_t list_cap) {
         return create_with_lists(config, P, capL, capH, pops, hb, n_boundary, group_base, next_id,
                                  step, list_cap, out);
     });

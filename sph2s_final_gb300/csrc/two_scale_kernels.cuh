@@ -453,20 +453,21 @@ __global__ void __launch_bounds__(32 * kTsWarps) ts_density_lanes_kernel(
         __syncwarp();
         uint32_t same, compl_;
         uint32_t at = ts_lanes_start<LANES>(k, same), cat = ts_lanes_start<LANES>(kc, compl_);
-        if (k <= SAME) {
-            for (uint32_t e = 0; e < k && lists.holds(at); ++e, ++at)
-                ts_list_put(list4, at, i, n_r, hs[e * 32]);
+        if (!lists.fits(same)) {
+            // a list that does not fit is not read
+        } else if (k <= SAME) {
+            for (uint32_t e = 0; e < k; ++e) ts_list_put(list4, at++, i, n_r, hs[e * 32]);
         } else {
             scan(P.g[R], cells_r, spos_r, n_r, P.h[R], P.T[R], [&](uint32_t j, const float4&, float r2) {
-                if (r2 != 0.0f && lists.holds(at)) ts_list_put(list4, at++, i, n_r, j);
+                if (r2 != 0.0f) ts_list_put(list4, at++, i, n_r, j);
             });
         }
-        if (kc <= COMPL) {
-            for (uint32_t e = 0; e < kc && cat < ComplCap<R>::value; ++e, ++cat)
-                ts_list_put(clist4, cat, i, n_r, hc[e * 32]);
+        if (compl_ > ComplCap<R>::value) {
+        } else if (kc <= COMPL) {
+            for (uint32_t e = 0; e < kc; ++e) ts_list_put(clist4, cat++, i, n_r, hc[e * 32]);
         } else {
             scan(P.g[C], cells_c, spos_c, n_c, P.h[0], P.T[0], [&](uint32_t j, const float4&, float r2) {
-                if (r2 != 0.0f && cat < ComplCap<R>::value) ts_list_put(clist4, cat++, i, n_r, j);
+                if (r2 != 0.0f) ts_list_put(clist4, cat++, i, n_r, j);
             });
         }
 #pragma unroll
@@ -525,7 +526,11 @@ struct TSOut {
 // taking every LANES-th group of its lists (a coarse one has ~270 fine
 // neighbours, whose gathers are a chain of latencies), their sums added in a
 // fixed order: the LOW pass 55 / 61 us (10,368 / 184,000 particles) before,
-// 15 / 14 us for the near ones beside 19 / 39 us for the others now;
+// 15 / 14 us for the near ones beside 19 / 39 us for the others now.  Where a list
+// overflows they rescan together, each taking every LANES-th candidate of a cell.  Us
+// per step with one lane to a particle, with one of eight rescanning alone, and now:
+// 884,736 particles, a support of 2.5 spacings 3,560, 2,630 and 2,440; 373,000 and 3
+// spacings 2,960, 3,770 and 1,900.
 // LANES = 1: one thread per particle, those flagged in skip left out.
 template <int R, bool DEBUG, int LANES = 1>
 __global__ void __launch_bounds__(256) ts_force_kernel(
@@ -620,7 +625,7 @@ __global__ void __launch_bounds__(256) ts_force_kernel(
                 }
                 g = gn;
             }
-        } else if (sub == 0) {
+        } else {
             const Stencil st = stencil(P.g[R], xi.x, xi.y, xi.z, P.h[R]);
             for (int cz = st.z0; cz <= st.z1; ++cz)
                 for (int cy = st.y0; cy <= st.y1; ++cy) {
@@ -628,7 +633,7 @@ __global__ void __launch_bounds__(256) ts_force_kernel(
                     for (int cx = st.x0; cx <= st.x1; ++cx) {
                         const uint2 r = __ldg(&cells_r[row + cx]);
                         const uint32_t e = min(r.y, n_r);
-                        for (uint32_t j = r.x; j < e; ++j) {
+                        for (uint32_t j = r.x < e ? r.x + sub : e; j < e; j += LANES) {
                             const float4 xj = __ldg(&spos_r[j]);
                             float dx, dy, dz;
                             const float r2 = dist2(xi.x, xi.y, xi.z, xj.x, xj.y, xj.z, dx, dy, dz);
@@ -691,7 +696,7 @@ __global__ void __launch_bounds__(256) ts_force_kernel(
                     }
                 }
             }
-        } else if (sub == 0) {
+        } else {
             const Stencil st = stencil(P.g[C], xi.x, xi.y, xi.z, P.h[0]);
             for (int cz = st.z0; cz <= st.z1; ++cz)
                 for (int cy = st.y0; cy <= st.y1; ++cy) {
@@ -699,7 +704,7 @@ __global__ void __launch_bounds__(256) ts_force_kernel(
                     for (int cx = st.x0; cx <= st.x1; ++cx) {
                         const uint2 r = __ldg(&cells_c[row + cx]);
                         const uint32_t e = min(r.y, n_c);
-                        for (uint32_t j = r.x; j < e; ++j) {
+                        for (uint32_t j = r.x < e ? r.x + sub : e; j < e; j += LANES) {
                             const float4 xj = __ldg(&spos_c[j]);
                             float dx, dy, dz;
                             const float r2 = dist2(xi.x, xi.y, xi.z, xj.x, xj.y, xj.z, dx, dy, dz);
