@@ -130,6 +130,13 @@ void enqueue_force(sph_batch* b, float dt) {
     }
 }
 
+// Blocks of the step's first kernel: one per tile of particles, or as many as clearing
+// the cell table takes.  By the tiles alone, two scenes of 600 particles in 128^3 cells
+// (33 MB) cleared it with 6 blocks: 158 us per step, 52 when a memset did it, now 37.
+uint32_t hash_grid(const sph_batch* b) {
+    return pgrid(b, std::max(b->ntiles[1], (uint32_t)(((uint64_t)b->NC + 1023) / 1024)));
+}
+
 // hash -> stable sort of (scene, cell key, index) -> reorder + cell ranges.
 // From 524,288 fluid particles the sort is the coherent one (coherent_sort.cuh:
 // the same permutation, radix-sorting only the particles that changed cell).
@@ -143,7 +150,7 @@ int enqueue_neighborhood(sph_batch* b) {
     near.count = b->bcount;
     near.flag = b->bflag;
     if (b->coherent) {
-        b_hash_hist_kernel<256><<<pgrid(b, b->ntiles[1]), 256, 0, st>>>(
+        b_hash_hist_kernel<256><<<hash_grid(b), 256, 0, st>>>(
             b->tiles[1], b->ntiles[1], b->recs, b->pos, b->shift, 0, b->keys[0], b->sort.hist,
             clear);
         coherent_sort_keys(b->co, b->keys[0], 8 * b->passes, b->keys[1], b->vals[1], b->err, 0,
@@ -151,7 +158,7 @@ int enqueue_neighborhood(sph_batch* b) {
     } else {
         clear.words = b->sort.tile_ctr;
         clear.nwords = sort_step_words(b->N, b->passes);
-        b_hash_hist_kernel<256><<<pgrid(b, b->ntiles[1]), 256, 0, st>>>(
+        b_hash_hist_kernel<256><<<hash_grid(b), 256, 0, st>>>(
             b->tiles[1], b->ntiles[1], b->recs, b->pos, b->shift, b->passes, b->keys[0],
             b->sort.hist, clear);
         o = sort_step_run(b->keys, b->vals, b->N, b->passes, b->sort, b->err, 0, st);
