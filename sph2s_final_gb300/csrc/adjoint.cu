@@ -143,9 +143,13 @@ int record_segment(sph_solver* s, int len) {
     uint32_t* blist0 = s->blist;
     uint32_t* bcount0 = s->bcount;
     uint8_t* bflag0 = s->bflag;
+    const int out = sort_output(s);
+    uint32_t* vals0 = s->vals[out];
     for (int k = 0; k < len; ++k) {
+        s->vals[out] = r->perm[k];
         s->spos = r->xh[k];
         s->svel = r->vh[k];
+        s->cells_prev = s->cells;
         s->cells = r->cells[k];
         s->rho = r->rho[k];
         s->aux = r->aux[k];
@@ -154,15 +158,15 @@ int record_segment(sph_solver* s, int len) {
         s->blist = r->nlist[k];
         s->bcount = r->ncount[k];
         s->bflag = r->nflag[k];
-        const int out = enqueue_neighborhood(s);
-        cudaMemcpyAsync(r->perm[k], s->vals[out], 4 * (size_t)s->n, cudaMemcpyDeviceToDevice,
-                        s->stream);
+        enqueue_neighborhood(s);
         enqueue_density(s);
         enqueue_force(s, r->dt);
     }
+    s->vals[out] = vals0;
     s->spos = spos0;
     s->svel = svel0;
     s->cells = cells0;
+    s->cells_prev = nullptr;
     s->rho = rho0;
     s->aux = aux0;
     s->nbr = nbr0;

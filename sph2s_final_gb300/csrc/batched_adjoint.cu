@@ -263,7 +263,10 @@ int record_segment(sph_batch* b, int len) {
     uint2* blist0 = b->blist;
     uint32_t* bcount0 = b->bcount;
     uint8_t* bflag0 = b->bflag;
+    const int out = b->coherent ? 1 : b->passes & 1;  // where the step's sort leaves its output
+    uint32_t* vals0 = b->vals[out];
     for (int k = 0; k < len; ++k) {
+        b->vals[out] = r->perm[k];
         b->spos = r->xh[k];
         b->svel = r->vh[k];
         b->cells = r->cells[k];
@@ -274,12 +277,11 @@ int record_segment(sph_batch* b, int len) {
         b->blist = r->nlist[k];
         b->bcount = r->ncount[k];
         b->bflag = r->nflag[k];
-        const int out = enqueue_neighborhood(b);
-        cudaMemcpyAsync(r->perm[k], b->vals[out], 4 * (size_t)b->N, cudaMemcpyDeviceToDevice,
-                        b->stream);
+        enqueue_neighborhood(b);
         enqueue_density(b);
         enqueue_force(b, r->dt);
     }
+    b->vals[out] = vals0;
     b->spos = spos0;
     b->svel = svel0;
     b->cells = cells0;

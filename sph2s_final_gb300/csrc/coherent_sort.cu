@@ -441,10 +441,10 @@ void coherent_reset(const CoherentSort& c, cudaStream_t st) {
 }
 
 void coherent_sort_cells(const CoherentSort& c, const float4* pos, const float4* vel,
-                         const GridParams& g, uint2* cells, int key_bits, uint32_t* keys,
-                         uint32_t* keys_out, uint32_t* perm_out, float4* pos_out, float4* vel_out,
+                         const GridParams& g, const uint2* cells_prev, uint2* cells, int key_bits,
+                         uint32_t* keys, uint32_t* keys_out, uint32_t* perm_out, float4* pos_out, float4* vel_out,
                          uint32_t* err, int force_timeout, cudaStream_t st, NearList near) {
-    coherent_run(c, pos, &g, cells, keys, key_bits, keys_out, perm_out, pos, vel, pos_out, vel_out,
+    coherent_run(c, pos, &g, cells_prev, keys, key_bits, keys_out, perm_out, pos, vel, pos_out, vel_out,
                  err, force_timeout, st, near.count);
     if (c.n == 0) return;
     cudaMemsetAsync(cells, 0xFF, sizeof(uint2) * (size_t)g.dx * g.dy * g.dz, st);

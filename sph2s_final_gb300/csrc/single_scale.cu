@@ -65,14 +65,12 @@ namespace sph_ss {
 int enqueue_neighborhood(sph_solver* s) {
     cudaStream_t st = s->stream;
     int out = 1;
-    const bool coherent = s->sort_mode == kSortCoherent ||
-                          (s->sort_mode == kSortAuto && s->n >= kCoherentMinParticles);
     NearList near;  // the near-boundary particles, for the boundary force pass
     near.bnear = s->bnear;
     near.list = s->blist;
     near.count = s->bcount;
     near.flag = s->bflag;
-    if (!coherent || s->force_timeout) {
+    if (!sorts_coherently(s)) {
         const int passes = sort_passes(s->key_bits);
         const uint32_t hb = std::min(std::max(blocks_for(s->n), blocks_for(s->ncells, 1024)), 152u * 8u);
         const StepClear clear = {s->cells, s->ncells, s->sort.tile_ctr, sort_step_words(s->n, passes),
@@ -81,9 +79,9 @@ int enqueue_neighborhood(sph_solver* s) {
                                              clear);
         out = sort_step_run(s->keys, s->vals, s->n, passes, s->sort, s->err, s->force_timeout, st);
     } else {  // sort, reorder and cell table in one sequence
-        coherent_sort_cells(s->co, s->pos, s->vel, s->P.g, s->cells, s->key_bits, s->keys[0],
-                            s->keys[1], s->vals[1], s->spos, s->svel, s->err, s->force_timeout, st,
-                            near);
+        coherent_sort_cells(s->co, s->pos, s->vel, s->P.g, s->cells_prev ? s->cells_prev : s->cells,
+                            s->cells, s->key_bits, s->keys[0], s->keys[1], s->vals[1], s->spos,
+                            s->svel, s->err, s->force_timeout, st, near);
         return out;
     }
     launch_after(gather_cells_kernel<true>, blocks_for(s->n), 256, st, s->keys[out], s->vals[out],

@@ -40,6 +40,7 @@ struct sph_solver {
     uint32_t* keys[2] = {nullptr, nullptr};
     uint32_t* vals[2] = {nullptr, nullptr};
     uint2* cells = nullptr;
+    const uint2* cells_prev = nullptr;  // the last step's, where not in `cells` (a rollout records)
     uint2* bcells = nullptr;
     float4* bpos = nullptr;
     float4* pos0 = nullptr;  // positions at creation, creation order (rollout restarts)
@@ -75,6 +76,15 @@ namespace sph_ss {
 // launches, 1.17M particles of a batch 585 and 569.
 constexpr int kSortAuto = 0, kSortFull = 1, kSortCoherent = 2;
 constexpr uint32_t kCoherentMinParticles = 1u << 19;
+// Whether the step sorts coherently (from scratch too while a test forces timeouts).
+inline bool sorts_coherently(const sph_solver* s) {
+    return !s->force_timeout && (s->sort_mode == kSortCoherent ||
+                                 (s->sort_mode == kSortAuto && s->n >= kCoherentMinParticles));
+}
+// The index of the key/value buffers that the step's sort leaves its output in.
+inline int sort_output(const sph_solver* s) {
+    return sorts_coherently(s) ? 1 : sph::sort_passes(s->key_bits) & 1;
+}
 // hash -> sort (coherent or from scratch, sort_mode) -> reorder + cell ranges;
 // returns the index of the key/value buffers that hold the sorted keys and
 // the permutation.
