@@ -541,16 +541,22 @@ int sphb_get_scene(sph_batch* b, uint32_t scene, float* xyz, float* vel, float* 
         if (b->pack) cudaFree(b->pack);
         b->pack = nullptr;
         b->pack_floats = 0;
-        SPH_CUDA(cudaMalloc(&b->pack, 4 * floats));
-        b->pack_floats = floats;
+        if (cudaMalloc(&b->pack, 4 * floats) == cudaSuccess)
+            b->pack_floats = floats;
+        else
+            cudaGetLastError();
     }
-    // the wanted arrays one after another in b->pack
+    // the wanted arrays one after another in b->pack, or, where the memory does not hold
+    // it, in the neighbour lists (64 bytes a particle at least), which a step writes anew
+    if (!b->pack && (size_t)b->list_cap * b->N < floats)
+        return fail(SPH_E_CUDA, "sphb_get_scene: out of device memory");
+    float* const pack = b->pack ? b->pack : reinterpret_cast<float*>(b->nbr);
     float* const host[3] = {xyz, vel, rho};
     float* dev[3] = {nullptr, nullptr, nullptr};
     size_t bytes[3] = {0, 0, 0}, at = 0;
     for (int a = 0; a < 3; ++a)
         if (host[a]) {
-            dev[a] = b->pack + at;
+            dev[a] = pack + at;
             bytes[a] = 4 * n * (a < 2 ? 3 : 1);
             at += bytes[a] / 4;
         }
@@ -562,7 +568,7 @@ int sphb_get_scene(sph_batch* b, uint32_t scene, float* xyz, float* vel, float* 
     const size_t total = 4 * floats, chunks = (total + kChunk - 1) / kChunk;
     auto fetch = [&](size_t c) {
         const size_t len = std::min(kChunk, total - c * kChunk);
-        const cudaError_t e = cudaMemcpyAsync(b->pinned[c & 1], (char*)b->pack + c * kChunk, len,
+        const cudaError_t e = cudaMemcpyAsync(b->pinned[c & 1], (char*)pack + c * kChunk, len,
                                               cudaMemcpyDeviceToHost, b->stream);
         return e == cudaSuccess ? cudaEventRecord(b->copied[c & 1], b->stream) : e;
     };
