@@ -169,10 +169,10 @@ int set_integrator(sph_solver* s, int32_t integrator) {
     if (integrator != SPH_INTEGRATOR_SYMPLECTIC_EULER && integrator != SPH_INTEGRATOR_XSPH)
         return fail(SPH_E_INVALID, "sph_set_integrator: unknown integrator");
     SPH_CUDA(cudaStreamSynchronize(s->stream));
-    if (integrator == SPH_INTEGRATOR_XSPH && !s->xvel) {
+    if (integrator == SPH_INTEGRATOR_XSPH) {  // each by itself: the second may have failed before
         const size_t n = s->n ? s->n : 1;
-        SPH_CUDA(cudaMalloc(&s->xvel, 16 * n));
-        SPH_CUDA(cudaMalloc(&s->xall, 4 * n));
+        if (!s->xvel) SPH_CUDA(cudaMalloc(&s->xvel, 16 * n));
+        if (!s->xall) SPH_CUDA(cudaMalloc(&s->xall, 4 * n));
     }
     if (s->graph) {
         cudaGraphExecDestroy(s->graph);
