@@ -14,6 +14,7 @@
 #include <vector>
 #include "batched_solver.h"
 #include "errors.h"
+#include "graph_capture.h"
 #include "host_params.h"
 #include "scan.cuh"
 #include "single_scale_kernels.cuh"
@@ -478,12 +479,7 @@ int sphb_advance(sph_batch* b, float dt, int32_t steps) {
             b->graph = nullptr;
         }
         cudaGraph_t g;
-        SPH_CUDA(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
-        enqueue_step(b, dt);
-        cudaError_t le = cudaGetLastError();
-        cudaError_t ce = cudaStreamEndCapture(b->stream, &g);
-        SPH_CUDA(le);
-        SPH_CUDA(ce);
+        SPH_CUDA(capture_graph(b->stream, [&] { enqueue_step(b, dt); }, &g));
         cudaError_t ie = cudaGraphInstantiate(&b->graph, g, 0);
         cudaGraphDestroy(g);
         SPH_CUDA(ie);

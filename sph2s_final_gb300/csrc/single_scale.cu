@@ -9,6 +9,7 @@
 #include <cstring>
 #include <vector>
 #include "errors.h"
+#include "graph_capture.h"
 #include "host_params.h"
 #include "boundary_tables.cuh"
 
@@ -421,12 +422,7 @@ int sph_advance(sph_solver* s, float dt, int32_t steps) {
             s->graph = nullptr;
         }
         cudaGraph_t g;
-        SPH_CUDA(cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal));
-        enqueue_step(s, dt);
-        cudaError_t le = cudaGetLastError();
-        cudaError_t ce = cudaStreamEndCapture(s->stream, &g);
-        SPH_CUDA(le);
-        SPH_CUDA(ce);
+        SPH_CUDA(capture_graph(s->stream, [&] { enqueue_step(s, dt); }, &g));
         cudaError_t ie = cudaGraphInstantiate(&s->graph, g, 0);
         cudaGraphDestroy(g);
         SPH_CUDA(ie);

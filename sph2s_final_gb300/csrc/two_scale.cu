@@ -13,6 +13,7 @@
 #include <string>
 #include <vector>
 #include "errors.h"
+#include "graph_capture.h"
 #include "state_format.h"
 #include "host_params.h"
 #include "radix_sort.cuh"
@@ -504,12 +505,7 @@ int ts_launch(sph_solver2* s, float dt) {
     }
     if (!s->graph || !(key == s->graph_key)) {
         cudaGraph_t g = nullptr;
-        SPH_CUDA(cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal));
-        ts_enqueue(s, dt);
-        const cudaError_t le = cudaGetLastError();
-        const cudaError_t ce = cudaStreamEndCapture(s->stream, &g);
-        SPH_CUDA(le);
-        SPH_CUDA(ce);
+        SPH_CUDA(capture_graph(s->stream, [&] { ts_enqueue(s, dt); }, &g));
         if (s->graph) {
             cudaGraphExecUpdateResultInfo info;
             if (cudaGraphExecUpdate(s->graph, g, &info) != cudaSuccess) {
