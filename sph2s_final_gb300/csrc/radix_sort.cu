@@ -214,7 +214,6 @@ SortScratch sort_scratch_from(void* base, uint32_t max_n) {
     p += align256(kSortMaxPasses * 4);
     s.status = (uint32_t*)p;
     p += align256((size_t)kSortMaxPasses * tiles * 256 * 4);
-    s.max_tiles = tiles;
     s.zero_bytes = (size_t)(p - (char*)base);
     return s;
 }

@@ -42,7 +42,6 @@ struct SortScratch {
     uint32_t* hist;      // [kSortMaxPasses][256] histograms
     uint32_t* tile_ctr;  // [kSortMaxPasses]
     uint32_t* status;    // [passes][tiles][256] look-back words
-    uint32_t max_tiles;
     size_t zero_bytes;   // bytes from hist through status
 };
 
