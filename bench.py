@@ -413,8 +413,8 @@ def measure_batched(steps: int, warmup: int = 3, peaks=None, ratio=None):
 
 def measure_adjoint(steps: int = 200, every: int = 20, reps: int = 3, peaks=None, ratio=None):
     """65,536-particle differentiable rollout (T steps, checkpoints every K):
-    forward (with checkpoints) and backward (segment recompute + adjoint
-    kernels) wall time per rollout, synchronous calls, best of `reps`."""
+    forward (with checkpoints, its last segment recorded) and backward (the
+    other segments recomputed + adjoint kernels) wall time per rollout, synchronous calls, best of `reps`."""
     import torch
 
     from sph2s_final_gb300 import scenes
@@ -452,17 +452,25 @@ def measure_adjoint(steps: int = 200, every: int = 20, reps: int = 3, peaks=None
     if peaks is not None:
         n = sc.fluid.num_particles
         algo, flops = step_work([sc], xs, ratio)
-        # backward per step: the segment's forward recomputed with its tape written
-        # (310 B per particle), then the adjoint integrate / force / density passes,
-        # which read the tape and the same records as their forward passes
-        bw_algo = 2 * algo + 2 * 310 * n
+        # backward per step: the forward steps of every segment but the last recomputed
+        # with their tape written (the last one's was written by the forward pass), then
+        # the adjoint integrate / force / density passes, which read the tape and the same
+        # records as their forward passes.  Tape per particle: permutation, position,
+        # velocity, density, EOS pair, list length, near flag and the list's used entries
+        cand = stencil_candidates(sc.config.grid, float(sc.config.effective_radius), xs[0], xs[0])
+        nbr = float(cand.sum()) * (ratio or 0.155) - n
+        tape = (4 + 16 + 16 + 4 + 8 + 4 + 1) * n + 4 * nbr
+        segments = -(-steps // every)
+        again = (segments - 1) / segments
+        bw_algo = (1 + again) * (algo + tape)
         out["roofline_forward"] = pass_roofline("rollout_forward", 1e3 * f / steps, algo, flops,
                                                 *peaks, "c3")
         out["roofline_backward"] = pass_roofline("rollout_backward", 1e3 * b / steps, bw_algo,
-                                                 3 * flops, *peaks, "c3")
-        out["roofline_backward"]["note"] = ("per step, estimated: recompute (one forward step + "
-                                            "310 B/particle of tape) + adjoint passes (one more "
-                                            "step's bytes + the tape read; twice the forward flops)")
+                                                 (2 + again) * flops, *peaks, "c3")
+        out["roofline_backward"]["note"] = (
+            f"per step, estimated: {segments - 1} of {segments} segments recomputed (a forward "
+            f"step + {tape / n:.0f} B/particle of tape written) + adjoint passes (one more step's "
+            "bytes + the tape read; twice the forward flops)")
     return out
 
 

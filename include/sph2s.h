@@ -200,7 +200,7 @@ int sph_debug_force_lookback_timeout(sph_solver* s, int32_t on);
 
 /* Test hook selecting how each step sorts its (cell key, index) pairs; both
  * ways give the same permutation.  0 (default): automatic -- coherent from
- * 131,072 particles on, from scratch below (where the radix sort alone is
+ * 524,288 particles on, from scratch below (where the radix sort alone is
  * faster); 1: from scratch (sph_sort_pairs' onesweep sort); 2: coherent
  * (sph_sort_keys_coherent's scheme: only the particles that changed cell
  * since the last step are radix-sorted, the rest merged around them). */

@@ -5,12 +5,14 @@
 // viscosity, T steps; the state is checkpointed every K steps.
 // Loss: L = mean_n (G_n - target_n)^2, G the Poly6 splat of the final
 // positions on the cell centres of a node grid.
-// Backward: segment by segment, latest first: the segment is recomputed from
-// its checkpoint while the step's own buffers are redirected into a tape
-// (sort permutation, sorted positions and velocities, densities, neighbour
-// lists), then the hand-written adjoint kernels run backwards through it,
-// holding the neighbour structure of every step constant.  Memory is one
-// segment of tape (~440 bytes per particle per step) plus T/K checkpoints.
+// Backward: segment by segment, latest first: the hand-written adjoint kernels run
+// backwards through a tape of the segment's steps (sort permutation, sorted
+// positions and velocities, densities, neighbour lists, near-boundary particles),
+// holding the neighbour structure of every step constant.  The tape of the last
+// segment is recorded by the forward pass, the other segments are recomputed from
+// their checkpoints; in both the step's own buffers are redirected into the tape.
+// Memory is one segment of tape (~440 bytes per particle per step, 384 of them the
+// lists, or less where that does not fit) plus T/K checkpoints.
 #include <cmath>
 #include <cstring>
 #include <vector>

@@ -3,8 +3,9 @@
 //
 // The single-scale rollout (adjoint.cu) restated over the batch's packed
 // arrays: one forward with checkpoints every K steps, one Poly6-splat loss per
-// scene on its own node grid, and one reverse pass that recomputes each
-// segment into a tape and runs the adjoint kernels backwards.  Every kernel
+// scene on its own node grid, and one reverse pass that runs the adjoint kernels
+// backwards through the tape of each segment: the last one's is recorded by the
+// forward pass, the others' are recomputed.  Every kernel
 // walks the batch's 256-particle tiles, so a block's scene constants (grid
 // tables, P, viscosity) are uniform and the per-particle code is the
 // single-scale adjoint's (adj_force_one, adj_density_one, splat_node,

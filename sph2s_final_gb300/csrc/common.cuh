@@ -17,7 +17,7 @@ constexpr uint32_t kEmptyCell = 0xFFFFFFFFu;  // EMPTY_CELL_ID, SPH2S_FINAL_SING
 // 40-60 us, which then sets the force pass's duration at any size below ~1M.  With
 // 64 slots a dam break reaches that after 100 steps (up to 84 neighbours, a few
 // dozen particles where the block hits its corners): a step of 110,592 particles
-// took 144 us against 102 now, of 262,144 208 against 162, of 16 scenes 154
+// took 144 us against 102 now, of 262,144 208 against 164, of 16 scenes 154
 // against 103.  Slots past a particle's neighbours are never touched.
 constexpr int kMaxNbr = 96;
 

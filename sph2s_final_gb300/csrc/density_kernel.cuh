@@ -106,7 +106,7 @@ __global__ void __launch_bounds__(kDensityThreads) density_kernel(
 // candidates.  Us per step alone, and of three solvers in turn, one lane and nine:
 // 4,096 particles 64 and 39, 25 and 17; 8,000 68 and 44, 27 and 20; 13,824 70 and
 // 52, 28 and 25; 21,952 72 and 62, but 29 and 34: nine lanes are more work, which
-// pays while the chip has room.
+// pays while the chip has room.  (The first hundred steps of a dam break.)
 constexpr uint32_t kDensitySplitMost = 16384;
 constexpr uint32_t kSplitLanes = 9, kSplitPer = 32 / kSplitLanes, kSplitWarps = 4;
 // Neighbours that a lane keeps; one with more scans its share again, for the list

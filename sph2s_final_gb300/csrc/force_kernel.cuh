@@ -125,8 +125,9 @@ __device__ __forceinline__ void scan_boundary(const float4& xi, const float4* __
 // from the stencil scan.  A superset of the boundary particles within h in both
 // cases; f applies the r < h test itself.  AHEAD candidates' indices, then their
 // positions, are loaded together: one after the other, ~70 candidates are a chain
-// of 140 loads, the longest of a small scene's step (4,096 particles 42.5 us per
-// step; four together 35.2, eight 33.4).
+// of 140 loads, the longest of a small scene's step (4,096 particles 42.8 us per
+// step 400 steps into a dam break, 49.7 at its start; four together 36.1 and 42.2,
+// eight 34.5 and 41.0).
 template <int AHEAD = 4, class F>
 __device__ __forceinline__ void visit_boundary(const float4& xi, int hx, int hy, int hz,
                                                uint32_t home, const float4* __restrict__ bpos,
@@ -261,7 +262,10 @@ static __device__ __noinline__ ForceAcc force_rescan(float4 xi, float4 vi, float
 // 705 to 674 us.  From kForceManyParticles on, one at a time at 48 registers and
 // 5 blocks: three solvers of 155,184 side by side 298 us for four steps (four
 // together: 307), a step of 2,097,152 773 us (four together 796, 40 registers
-// 783).  CROWDED, where most lists overflow (list_entries): the rescan in line, one
+// 783).  XSPH takes four at every size, since one makes less than 1 % of its step
+// (65,536 to 2,097,152 particles; 32,768 87 us, 91 with one), and so does the batched
+// pass (32 scenes of 1.17M particles 558 us per step, 590 with two, over 600 with one).
+// CROWDED, where most lists overflow (list_entries): the rescan in line, one
 // gather at a time, 40 registers and 6 blocks (1,000,000 particles with 110
 // neighbours: force 1,076 -> 889 us).  All the same bits.
 template <int MODE, bool BSEP = false, int AHEAD = 4, bool CROWDED = false>

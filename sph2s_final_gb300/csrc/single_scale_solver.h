@@ -70,10 +70,12 @@ struct sph_solver {
 namespace sph_ss {
 // The step's sort: automatic (coherent from kCoherentMinParticles on, where it
 // is faster on GB300), from scratch, or coherent.  Us per step from scratch and
-// coherent: 110,592 particles 92.7 and 97.3, 262,144 152 and 156, 512,000 240 and
-// 244, 1,000,000 410 and 415, 1,481,544 587 and 583, 2,097,152 798 and 787; with
-// several solvers on the GPU at once, where the memory it saves counts more than its
-// launches, 1.17M particles of a batch 585 and 569.
+// coherent, one solver waited for every 20 steps: 262,144 particles 152 and 157,
+// 512,000 245 and 246, 636,056 284 and 285, 1,000,000 410 and 410, 1,560,896 611 and
+// 605, 2,097,152 798 and 787.  Of three solvers in turn, where the memory it saves counts
+// more than its launches: 262,144 107 and 107, 512,000 201 and 194, 636,056 242 and 237,
+// 1,000,000 377 and 366, 1,560,896 580 and 552.  The line lies where the second gains
+// more than the first loses.
 constexpr int kSortAuto = 0, kSortFull = 1, kSortCoherent = 2;
 constexpr uint32_t kCoherentMinParticles = 1u << 19;
 // Whether the step sorts coherently (from scratch too while a test forces timeouts).

@@ -273,6 +273,12 @@ void ts_neighborhoods(sph_solver2* s) {
 // 7,290 particles 128 and 83, 19,565 140 and 105, 38,397 154 and 132, 65,416 173 and
 // 177, 88,587 189 and 213.
 constexpr uint32_t kTsSmall = 49152;
+// Lanes of the LOW and HIGH density and force passes.  Us per step of 5,184, 18,792 and
+// 46,080 particles at the start and (4,767, 17,126, 41,701) 300 steps on: as here 85,
+// 145, 217 (88, 118, 154); LOW density 8 lanes 108, 171, 235 (102, 131, 177), 32 84, 137,
+// 214 (79, 110, 153); HIGH density 4 86, 136, 202 (88, 110, 151), 16 86, 150, 232 (88,
+// 120, 168); LOW force 8 87, 150, 223 (88, 119, 158), 32 85, 144, 222 (89, 120, 158);
+// HIGH force 1 96, 148, 217 (94, 125, 165), 4 84, 145, 221 (78, 109, 157).
 constexpr int kTsSmallLow = 16, kTsSmallHigh = 8, kTsForceLow = 16, kTsForceHigh = 2;
 // From this many particles on the near LOW particles' density is one lane's again: the
 // chip is full, and eight lanes to a particle are more work.  Us per step with eight
