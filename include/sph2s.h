@@ -90,7 +90,10 @@ int sph_particle_box_canvas(const sph_grid* grid, int32_t border, float* xyz, ui
 
 /* Solver::Solver(fluid, boundary, config) + Bind().  Copies the fluid and
  * boundary positions (and optional initial velocities, NULL = zero) to the
- * device, sorts the static boundary once on the fluid grid.  The handle has
+ * device, sorts the static boundary once on the fluid grid.  Takes about 560
+ * bytes of device memory per fluid particle, 384 of them neighbour lists of 96
+ * entries; where those do not fit, lists of 64 down to 16 entries, with the same
+ * results (more particles then look their neighbours up a second time).  The handle has
  * its own stream and keeps the configuration in kernel parameters, so several
  * handles can coexist (the reference binds one __constant__ config). */
 int sph_create(const sph_config* config, const float* fluid_xyz, uint32_t n_fluid,
@@ -395,7 +398,8 @@ void* sphb_stream(sph_batch* b);
 int sphb_counts(sph_batch* b, uint32_t* num_scenes, uint32_t* total_fluid,
                 uint32_t* total_boundary);
 /* Positions, velocities (3 floats per particle) and densities of one scene,
- * sorted order or by the scene-local creation index; each pointer optional. */
+ * sorted order or by the scene-local creation index; each pointer optional.
+ * Several threads may read one batch at a time. */
 int sphb_get_scene(sph_batch* b, uint32_t scene, float* xyz, float* vel, float* rho,
                    int32_t order);
 /* Times block sizes 128/256/512 for the density and force passes and 4/8/12

@@ -90,7 +90,7 @@ inline uint32_t list_entries(float h, float m, float rho0) {
 // `lists` particles (or particle-steps of a tape), with at most `most`: kMaxNbr, or
 // fewer where the memory does not hold them (the results are the same: a particle
 // whose list is too short rescans).  A scene of hundreds of millions of particles, or
-// a long tape, fits with 64 or less and would not with 96: 384 of the ~600 bytes that
+// a long tape, fits with 64 or less and would not with 96: 384 of the ~560 bytes that
 // a handle takes per particle, and of the ~440 of a tape per particle and step.  Lists
 // beyond a quarter of the free memory start at 64, which leaves a program's other
 // handles and buffers their room.
