@@ -192,3 +192,28 @@ def test_tape_when_memory_is_short(cloud, short):
             s.rollout_forward(v, MU, 1e-5, 2, 2)
         for a, w in zip(run(s), want):
             np.testing.assert_array_equal(np.asarray(a), np.asarray(w))
+
+
+def test_lists_beyond_a_quarter_of_the_memory():
+    """4,200,000 particles' lists: 1,538 MiB with 96 entries, 1,025 with 64, which they
+    have where less than four times the former is free."""
+    n = 4200000
+    g = Grid.make_grid((0, 0, 0), (1, 1, 1), 0.02)
+    cfg = SolverConfiguration.direct(0.02, 1e-3, 1000.0, 30.0, MU, 88.1472, 0.8, g)
+    x = scenes.jitter(scenes.lattice_block(1 / 170, (162, 162, 162))[:n], 1 / 170, 0.01, 2)
+
+    def make():
+        before = free_bytes()
+        s = Solver(ParticleData(x), None, cfg)
+        return s, before - free_bytes()
+
+    s, much = make()
+    with s:
+        s.advance(1e-6, 2)
+        want = s.positions()
+    with Short(6000 * MiB):
+        s, less = make()
+        with s:
+            s.advance(1e-6, 2)
+            np.testing.assert_array_equal(s.positions(), want)
+    assert abs((much - less) - 4 * 32 * n) <= 16 * MiB
